@@ -103,6 +103,11 @@ struct hobak_batch_t {
   bool clusterOrderStale = false;    // new iteration counts since the classes were last ordered
   std::vector<int> sceneCluster;  // per scene: 0 by the tuning, > 0 a cluster size, -1 the tile path
   bool anyTileScene = true;
+  // the tile path's PCG in one launch (pcg_grid.cu), where the tiles fit
+  GridPlan grid{};
+  bool gridDirty = true;
+  int2* gridList = nullptr;  // device: the plan's CTA table
+  int longestRow = 0;        // blocks of the longest matrix row
   cudaStream_t classStream[kClusterClasses] = {};  // classes run beside the tile path (fork/join)
   cudaEvent_t evFork = nullptr, evJoin[kClusterClasses] = {};
   int lastStatus = HOBAK_OK;
@@ -314,6 +319,7 @@ int alloc_precision(hobak_batch_t* B) {
                             carve<double>(base, oVec[3]), d.y};
   }
   B->precMixed = mixed;
+  B->gridDirty = true;
   return HOBAK_OK;
 }
 
@@ -568,6 +574,8 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   const size_t oNewton = A.reserve(sizeof(int)), oNewtonRuns = A.reserve(sizeof(unsigned long long));
   const size_t oPart = A.reserve(sizeof(double) * kPartials * (size_t)ntilesCap);
   const size_t oPsi = A.reserve(sizeof(double) * nt);
+  const size_t oGridP = A.reserve(96 * (size_t)ntilesCap), oGridF = A.reserve(sizeof(int) * ntilesCap);
+  const size_t oGridL = A.reserve(sizeof(int2) * ntilesCap);
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, A.used);
   if (e != cudaSuccess)
@@ -639,6 +647,10 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   d.r64 = carve<double>(base, oR64);
   d.partial = carve<double>(base, oPart);
   d.psi = carve<double>(base, oPsi);
+  d.gridPartials = carve<double>(base, oGridP);
+  d.gridFlags = carve<int>(base, oGridF);
+  d.gridTilesCap = ntilesCap;
+  B->gridList = carve<int2>(base, oGridL);
   d.anyAniso = anyAniso;
   d.anyArap = anyArap;
   d.anySvdFree = anySvdFree;
@@ -678,6 +690,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   CUDA_TRY(up(d.tileV0, tileV0.data(), sizeof(int) * ntiles));
   CUDA_TRY(up(d.tileV1, tileV1.data(), sizeof(int) * ntiles));
   B->hostRowptr = rowptr;
+  for (int u = 0; u < nv; u++) B->longestRow = std::max(B->longestRow, rowptr[u + 1] - rowptr[u]);
   B->restHost = rest;
   B->hostCols = cols;
   return alloc_precision(B);
@@ -733,6 +746,7 @@ long long solve_launches(const hobak_batch_t* B) {
   // the cluster classes once; per sweep of the tile path: k_set_active,
   // inner init (+ the loop's arming kernel in a graph), the refinement
   if (!B->anyTileScene) return cl;
+  if (B->grid.ctas) return cl + sweeps * (2 + (mixed ? 2 : 0));  // inner init, the PCG launch, the refinement
   return cl + sweeps * (2 + (B->opts.use_graph ? 1 : 0) + (mixed ? 2 : 0));
 }
 
@@ -864,6 +878,39 @@ int prepare_cluster_classes(hobak_batch_t* B) {
   }
   if (changed) drop_graphs(B);
   B->clusterDirty = false;
+  B->gridDirty = true;
+  return HOBAK_OK;
+}
+
+// Whether the tile-path scenes' PCG runs in one cooperative launch, and its
+// CTA table.  Runs outside graph capture (it uploads); drops the graphs when
+// the plan changed.
+int prepare_grid_plan(hobak_batch_t* B) {
+  if (!B->gridDirty) return HOBAK_OK;
+  if (const int ce = configure_grid_pcg())
+    return fail(HOBAK_ERR_CUDA, std::string("PCG set-up: ") + cudaGetErrorString((cudaError_t)ce));
+  int dev = 0, sms = 0;
+  CUDA_TRY(cudaGetDevice(&dev));
+  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int n = (int)B->scenes.size();
+  std::vector<int> tiles(n);
+  for (int s = 0; s < n; s++) tiles[s] = B->sceneParams[s].pcgCluster ? 0 : B->sceneParams[s].ntiles;
+  GridPlan g = plan_grid_pcg(tiles.data(), n, B->d.tileV, B->longestRow,
+                             B->opts.precision == HOBAK_PRECISION_MIXED, sms);
+  if (g.ctas) {
+    std::vector<int2> list;
+    for (int s = 0; s < n; s++)
+      for (int t = 0; t < tiles[s]; t += g.tpc) list.push_back(make_int2(s, t));
+    CUDA_TRY(cudaStreamSynchronize(B->stream));
+    CUDA_TRY(cudaMemcpy(B->gridList, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice));
+    g.list = B->gridList;
+  }
+  if (g.ctas != B->grid.ctas || g.tpc != B->grid.tpc || g.rows != B->grid.rows || g.smem != B->grid.smem ||
+      g.scratch != B->grid.scratch)
+    drop_graphs(B);
+  B->grid = g;
+  B->d.gridOn = g.ctas ? 1 : 0;
+  B->gridDirty = false;
   return HOBAK_OK;
 }
 
@@ -998,10 +1045,16 @@ int enqueue_solve_t(hobak_batch_t* B, cudaStream_t s, bool capture, const PcgVec
     CUDA_TRY(cudaEventRecord(B->evJoin[c], B->classStream[c]));
   }
   for (int k = 0; k < sweeps && B->anyTileScene; k++) {
-    launch_set_active(d, s);
-    launch_inner_init<T>(d, v, s);
-    int rc = capture ? capture_pcg_loop<T>(B, s, v) : eager_pcg_loop<T>(B, s, v);
-    if (rc) return rc;
+    if (B->grid.ctas) {
+      launch_inner_init<T>(d, v, s);
+      const int ce = launch_grid_pcg<T>(d, v, B->grid, s);
+      if (ce) return fail(HOBAK_ERR_CUDA, std::string("PCG launch: ") + cudaGetErrorString((cudaError_t)ce));
+    } else {
+      launch_set_active(d, s);
+      launch_inner_init<T>(d, v, s);
+      int rc = capture ? capture_pcg_loop<T>(B, s, v) : eager_pcg_loop<T>(B, s, v);
+      if (rc) return rc;
+    }
     if (mixed) launch_refine(d, s);
   }
   for (int c = 0; c < kClusterClasses; c++)
@@ -1375,6 +1428,7 @@ int run_steps(hobak_batch_t* B, int nsteps) {
   const bool timed = B->timing;
   if (int rc = prepare_cluster_classes(B)) return rc;
   if (int rc = reorder_cluster_classes(B)) return rc;
+  if (int rc = prepare_grid_plan(B)) return rc;
   // cleared once per call: an overflow in any step or Newton iteration is reported
   if (B->d.collOn) CUDA_TRY(cudaMemsetAsync(B->d.coll.overflow, 0, sizeof(int), s));
   for (int k = 0; k < nsteps; k++) {
@@ -1466,6 +1520,7 @@ int apply_tile_size(hobak_batch_t* B, int TV) {
   d.ntiles = ntiles;
   d.tileV = TV;
   B->ntiles = ntiles;
+  B->gridDirty = true;
   drop_graphs(B);
   return HOBAK_OK;
 }
@@ -1618,7 +1673,8 @@ int hobak_batch_wait(hobak_batch b, hobak_step_stats* stats) {
   int status = HOBAK_OK;
   for (int s = 0; s < n; s++) {
     const SolveState& st = b->lastSolve[s];
-    if (st.converged < 0) status = HOBAK_ERR_NAN;
+    if (st.converged == kSolveTimedOut) status = HOBAK_ERR_CUDA;
+    else if (st.converged < 0 && status != HOBAK_ERR_CUDA) status = HOBAK_ERR_NAN;
     else if (st.converged == 0 && status == HOBAK_OK) status = HOBAK_WARN_NOT_CONVERGED;
     if (stats) {
       stats[s].iterations = st.totalIters;
@@ -1627,6 +1683,7 @@ int hobak_batch_wait(hobak_batch b, hobak_step_stats* stats) {
       stats[s].refinements = st.sweep > 0 ? st.sweep - 1 : 0;
     }
   }
+  if (status == HOBAK_ERR_CUDA) return fail(status, "a wait inside the PCG launch ran out");
   if (status == HOBAK_ERR_NAN) return fail(status, "non-finite residual in PCG");
   if (b->d.collOn) {
     int over = 0;
@@ -2039,7 +2096,8 @@ int hobak_batch_launch_count(hobak_batch b, long long* launches) {
 
 int hobak_batch_time_kernels(hobak_batch b, int reps, double* ms) {
   if (!b || !ms || reps <= 0) return fail(HOBAK_ERR_INVALID, "bad arguments");
-  const DeviceBatch& d = b->d;
+  DeviceBatch d = b->d;
+  d.gridOn = 0;  // the two kernels of an iteration, whichever way the step runs it
   cudaStream_t s = b->stream;
   const int n = (int)b->scenes.size();
   cudaEvent_t e0 = b->ev[0], e1 = b->ev[1];
@@ -2076,7 +2134,7 @@ int hobak_batch_time_kernels(hobak_batch b, int reps, double* ms) {
       else launch_inner_init<double>(d, d.v64, s);
       CUDA_TRY(cudaStreamSynchronize(s));
       if (int rc = keep_running()) return rc;
-      CUDA_TRY(cudaMemcpyAsync(d.nLoopTiles, &d.ntiles, sizeof(int), cudaMemcpyHostToDevice, s));
+      CUDA_TRY(cudaMemcpyAsync(d.nLoopTiles, &b->d.ntiles, sizeof(int), cudaMemcpyHostToDevice, s));
     }
     CUDA_TRY(cudaEventRecord(e0, s));
     for (int r = 0; r < reps; r++) {

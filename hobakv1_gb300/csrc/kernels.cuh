@@ -37,6 +37,17 @@ struct ClusterClass {
   const int* scenes;  // device list of their scene ids
 };
 
+// The tile path's PCG in one cooperative launch (pcg_grid.cu): ctas == 0 where
+// the batch's tiles do not fit the GPU at once.
+struct GridPlan {
+  int ctas, tpc;     // CTAs, tiles per CTA (one scene per CTA)
+  int rows;          // blocks of every matrix row kept in shared memory
+  int scratch;       // doubles of its exchange area
+  size_t smem;       // dynamic shared memory of a CTA
+  const int2* list;  // device: per CTA its scene and its first tile in the scene
+};
+constexpr int kSolveTimedOut = -2;  // SolveState::converged: a wait of the one-launch PCG ran out
+
 // Device pointers of one packed batch.  Plain struct passed by value.
 // LHS storage: 32-vertex slices of 3x3 blocks (SELL-32).  The row of vertex
 // u (blocks k = rowptr[u] + j, j < rowptr[u + 1] - rowptr[u]) lives in the
@@ -145,6 +156,12 @@ struct DeviceBatch {
   PcgVecs<double> v64;  // FP64 path (r = r64, d = y)
   PcgVecs<float> v32;   // mixed path
   double* partial;      // [ntiles][kPartials]
+  // one-launch PCG (pcg_grid.cu): [2][gridTilesCap][3] 16-byte words {partial,
+  // iteration} and a flag per tile
+  double* gridPartials;
+  int* gridFlags;
+  int gridTilesCap;
+  int gridOn;  // the tile-path scenes take that path
   double* psi;          // [T] energy density scratch
   int anyAniso;          // some scene has an anisotropic energy (k_element_aniso)
   int anyArap, anySvdFree;  // some scene has ARAP / another isotropic energy (mixed element kernels)
@@ -249,6 +266,12 @@ void launch_element_eval(int nt, const int4* tets, const double* rest, const dou
 template <typename T>
 int launch_cluster_pcg(const DeviceBatch& b, const PcgVecs<T>& v, const ClusterClass* classes, int k,
                        cudaStream_t s);
+GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, int longestRow, bool mixed, int sms);
+int configure_grid_pcg();
+// Every iteration of the inner solves that launch_inner_init has started, for
+// all scenes of the plan.  Returns a cudaError_t value (0 on success).
+template <typename T>
+int launch_grid_pcg(const DeviceBatch& b, const PcgVecs<T>& v, const GridPlan& g, cudaStream_t s);
 // Rebuilds the cluster kernels' gather table from the scenes' cluster sizes.
 void launch_cluster_gather(const DeviceBatch& b, cudaStream_t s);
 // Dynamic shared-memory opt-in of the cluster kernels (once, outside capture).

@@ -1,0 +1,273 @@
+// Device helpers shared by the PCG kernels of the tile path (solver.cu) and
+// its one-launch form (pcg_grid.cu): reductions in a fixed order, contact
+// rows and the scalar recurrences.
+#pragma once
+#include <cfloat>
+
+#include "kernels.cuh"
+
+namespace hobak {
+
+// Fixed-order sum over the CTA; result valid in thread 0.  NT multiple of 32.
+// The whole tree runs in R (FP32 for the inner solve of the mixed path) and
+// only the CTA's total is widened to FP64: a conversion per warp costs a
+// 16-cycle issue on GB300's 2-lane FP64 pipe even when one lane uses it.
+template <int NT, typename R>
+__device__ __forceinline__ double block_sum(R v, double* sh) {
+  R* shr = reinterpret_cast<R*>(sh);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int w = threadIdx.x / 32, l = threadIdx.x % 32;
+  if (l == 0) shr[w] = v;
+  __syncthreads();
+  double s = 0;
+  if (threadIdx.x == 0) {
+    R t = R(0);
+#pragma unroll
+    for (int i = 0; i < NT / 32; i++) t += shr[i];
+    s = double(t);
+  }
+  __syncthreads();
+  return s;
+}
+
+// Three sums in one pass (one pair of barriers), each in the order of
+// block_sum; results valid in thread 0.  `sh` holds 3 * NT / 32 doubles.
+template <int NT, typename R>
+__device__ __forceinline__ void block_sum3(R a, R b, R c, double* sh, double (&out)[3]) {
+  R* shr = reinterpret_cast<R*>(sh);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  }
+  const int w = threadIdx.x / 32, l = threadIdx.x % 32;
+  if (l == 0) {
+    shr[w] = a;
+    shr[NT / 32 + w] = b;
+    shr[2 * (NT / 32) + w] = c;
+  }
+  __syncthreads();
+  out[0] = out[1] = out[2] = 0.0;
+  if (threadIdx.x == 0) {
+    R ta = R(0), tb = R(0), tc = R(0);
+#pragma unroll
+    for (int i = 0; i < NT / 32; i++) {
+      ta += shr[i];
+      tb += shr[NT / 32 + i];
+      tc += shr[2 * (NT / 32) + i];
+    }
+    out[0] = double(ta);
+    out[1] = double(tb);
+    out[2] = double(tc);
+  }
+  __syncthreads();
+}
+
+// After thread 0 wrote the CTA's partial(s): true in the CTA that finishes
+// the scene's reduction (ticket == ntiles - 1).  Only thread 0 published
+// anything the last CTA reads, so only it fences before taking its ticket.
+// The ticket is reset for reuse.
+__device__ __forceinline__ bool last_tile(unsigned* ticket, int ntiles, int* flag) {
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned t = atomicAdd(ticket, 1u);
+    *flag = (t == (unsigned)(ntiles - 1));
+    if (*flag) *ticket = 0u;
+  }
+  __syncthreads();
+  const bool last = *flag != 0;
+  if (last) __threadfence();
+  return last;
+}
+
+// Sum partial[(tile0 + i) * kPartials + comp] over i < n in a fixed order.
+template <int NT>
+__device__ __forceinline__ double sum_partials(const double* partial, int tile0, int n, int comp, double* sh) {
+  double s = 0;
+  for (int i = threadIdx.x; i < n; i += NT) s += __ldcg(&partial[(size_t)(tile0 + i) * kPartials + comp]);
+  return block_sum<NT>(s, sh);
+}
+
+// Order of the PCG's three dot products, the same on every path so that all
+// give the same bits.  FP64 costs 19 cycles of the SM's pipe per warp
+// instruction however few lanes it has, and 64 cycles of latency, so sums
+// use few instructions in short chains on several warps.
+//   tile    FP32: a tree per warp, the warps in order (block_sum3).  FP64: lane
+//           l adds the tile's vertices l, l + 32, ..., then a warp tree.
+//   group   kGroupVerts / TV consecutive tiles of the scene, added pairwise
+//   scene   lane l adds groups l, l + 32, ..., then a warp tree
+constexpr int kGroupVerts = 512;
+
+__device__ __forceinline__ double warp_tree(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// FP64 tile sum by one warp; vals: the tile's TV values.
+template <int TV>
+__device__ __forceinline__ double tile_sum64(const double* vals) {
+  double s = vals[threadIdx.x % 32];
+#pragma unroll
+  for (int i = 32; i < TV; i += 32) s += vals[i + threadIdx.x % 32];
+  return warp_tree(s);
+}
+
+// The sum of a group's tiles, get(i) its i-th (0 past the scene's last tile).
+template <int TV, typename Get>
+__device__ __forceinline__ double group_sum(Get get) {
+  double a = (get(0) + get(1)) + (get(2) + get(3));
+  if (kGroupVerts / TV == 4) return a;
+  return a + ((get(4) + get(5)) + (get(6) + get(7)));
+}
+
+// A scene's sum by one warp: group(g) for its n groups.
+template <typename Group>
+__device__ __forceinline__ double scene_sum(int n, Group group) {
+  double s = 0.0;
+  for (int g = threadIdx.x % 32; g < n; g += 32) s += group(g);
+  return warp_tree(s);
+}
+
+// The three scene sums from global tile partials, by the last CTA of the
+// scene; sh: 3 doubles.  Result valid in thread 0.
+template <int NT, int TV>
+__device__ __forceinline__ void scene_sums(const double* partial, int tile0, int n, double* sh, double (&out)[3]) {
+  constexpr int kG = kGroupVerts / TV;
+  for (int c = threadIdx.x / 32; c < 3; c += NT / 32) {
+    const double t = scene_sum((n + kG - 1) / kG, [&](int g) {
+      return group_sum<TV>([&](int i) {
+        return g * kG + i < n ? __ldcg(&partial[(size_t)(tile0 + g * kG + i) * kPartials + c]) : 0.0;
+      });
+    });
+    if (threadIdx.x % 32 == 0) sh[c] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 3; c++) out[c] = sh[c];
+}
+
+__device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+// A scene's iteration step (one thread), from
+// rho = |r|^2, gamma = (r, u) and delta = (w, u): after an update, stop when
+// |r|^2 < threshold (ConjugateGradient.h:75-78), on a non-finite value, or at
+// the iteration limit; otherwise beta and alpha for this iteration's update,
+// which the iteration count then includes.  Returns true when it stops.
+template <typename T>
+__device__ __forceinline__ bool pcg_decide(SolveState& st, double rho, double gamma, double delta) {
+  if (st.iters > 0) {
+    st.rr = rho;
+    bool stop = false;
+    if (rho < st.innerThreshold) {
+      stop = true;
+    } else if (!finite(rho) || !finite(gamma) || !finite(st.alpha)) {
+      stop = true;
+      st.converged = -1;
+      st.outerDone = 1;
+    } else if (st.totalIters >= st.maxit) {
+      stop = true;
+    }
+    if (stop) {
+      st.done = 1;
+      if (sizeof(T) == sizeof(double) && st.converged >= 0) {
+        // FP64 path: the recursive residual is the solver's verdict (Eigen)
+        st.rr64 = rho;
+        st.converged = rho < st.threshold ? 1 : 0;
+        st.outerDone = 1;
+      }
+      return true;
+    }
+  }
+  st.delta = delta;
+  // The reciprocals of the last gamma and alpha are formed off this path
+  // (pcg_reciprocals): one division is left on it, of the ~1,000 cycles each
+  // takes in a single thread.
+  if (st.iters == 0) {
+    st.beta = 0.0;
+    st.alpha = gamma / delta;
+  } else {
+    st.beta = gamma * st.gammaInv;
+    st.alpha = gamma / (delta - st.beta * gamma * st.alphaInv);
+  }
+  st.gammaOld = st.gamma;
+  st.gamma = gamma;
+  st.alphaF = float(st.alpha);
+  st.betaF = float(st.beta);
+  st.iters += 1;
+  st.totalIters += 1;
+  return false;
+}
+
+__device__ __forceinline__ void pcg_reciprocals(SolveState& st) {
+  st.gammaInv = 1.0 / st.gamma;
+  st.alphaInv = 1.0 / st.alpha;
+}
+
+// u of a vertex as the one-launch PCG shares it, four wide: in FP32 with the
+// iteration it belongs to in the fourth word, written at once, so that a
+// reader knows by the value itself whether it is the one it needs.
+__device__ __forceinline__ void publish_u(float* u4, int w, const float (&x)[3], int iteration) {
+  const unsigned long long lo = (unsigned long long)__float_as_uint(x[1]) << 32 | __float_as_uint(x[0]);
+  const unsigned long long hi = (unsigned long long)(unsigned)iteration << 32 | __float_as_uint(x[2]);
+  asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(u4 + 4 * (size_t)w),
+               "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ void publish_u(double* u4, int w, const double (&x)[3], int) {
+  __stcg(reinterpret_cast<double2*>(u4) + 2 * (size_t)w, make_double2(x[0], x[1]));
+  __stcg(u4 + 4 * (size_t)w + 2, x[2]);
+}
+
+// a . b of two 3-vectors, as the compiler contracts a0 b0 + a1 b1 + a2 b2
+template <typename T>
+__device__ __forceinline__ T dot3v(T a0, T a1, T a2, T b0, T b1, T b2) {
+  return a0 * b0 + a1 * b1 + a2 * b2;
+}
+
+// Contact: w H_coll x at a vertex (w = collision_lhs_scale), H_coll = sum over
+// its collision tets of (c c^T) (x) G (free rows only; x vanishes on pinned
+// rows, which keeps the columns masked too).  FP64 throughout: the contact
+// blocks are not part of the (possibly FP32) assembled LHS.  One incidence's
+// three rows; load(id, x) reads the vector at a vertex.  Explicit roundings:
+// every PCG path rounds alike.
+template <typename T, typename Load>
+__device__ __forceinline__ void collision_incidence(const DeviceCollisions& c, int k, Load load, double out[3]) {
+  const int e = c.incList[k], p = e >> 2, a = e & 3;
+  const int4 ct = c.pairTet[p];
+  const double* C = c.pairC + 4 * (size_t)p;
+  const double* G = c.pairG + 9 * (size_t)p;
+  const int id[4] = {ct.x, ct.y, ct.z, ct.w};
+  T x[4][3];
+#pragma unroll
+  for (int q = 0; q < 4; q++) load(id[q], x[q]);
+  double z[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) z[j] = fma(C[q], double(x[q][j]), z[j]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) out[i] = __dmul_rn(C[a], fma(G[i + 6], z[2], fma(G[i + 3], z[1], __dmul_rn(G[i], z[0]))));
+}
+
+// A vertex's rows, its incidences in order.
+template <typename T, typename Load>
+__device__ __forceinline__ void collision_rows(const DeviceBatch& b, int u, Load load, double out[3]) {
+  const DeviceCollisions& c = b.coll;
+  const int k0 = c.incCount[u], k1 = c.incCount[u + 1];
+  out[0] = out[1] = out[2] = 0.0;
+  if (k0 == k1) return;
+  for (int k = k0; k < k1; k++) {
+    double t[3];
+    collision_incidence<T>(c, k, load, t);
+#pragma unroll
+    for (int i = 0; i < 3; i++) out[i] = __dadd_rn(out[i], t[i]);
+  }
+  const double scale = collision_lhs_scale(b, b.vertexScene[u]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) out[i] = __dmul_rn(out[i], scale);
+}
+
+}  // namespace hobak

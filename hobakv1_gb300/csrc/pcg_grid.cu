@@ -1,0 +1,574 @@
+// The tile path's inner PCG in one cooperative launch.
+//
+// solver.cu runs an iteration as two grid-wide kernels (SpMV, update).  For a
+// batch whose tiles fit the GPU at once that spends most of an iteration on
+// the kernels' edges: launch, a cold walk tile -> row -> column -> u, the
+// matrix again from L2, two reductions' tails.  Here one launch runs every
+// iteration of the solve: a CTA per SM owns up to 512 vertices (whole tiles of
+// one scene) for the whole solve, one per thread.  A vertex's u, p, s, d, r
+// stay in registers; the first blocks of its matrix row and their columns in
+// shared memory (as many as fit, the same count for every row); the rest of
+// the row comes from L2.  Per iteration the CTAs of a scene meet twice:
+//   * after the SpMV the partial sums of the three dot products go out as
+//     16-byte words {value, iteration}, written and polled with
+//     single-copy-atomic 128-bit accesses, so a reader needs no flag and no
+//     fence; every CTA adds them in the same order and takes the same decision;
+//   * after the update the new u: in FP32 the same way, each vertex's u carries
+//     its iteration and a gather repeats until it fits; in FP64 (two words a
+//     vertex) a CTA releases a flag, and a CTA waits for the flags of the CTAs
+//     its rows' columns lie in (with contact: all of the scene's).
+// The partials' exchange also orders u's reuse: a CTA overwrites its u only
+// after every CTA of the scene has published the partials of the SpMV that
+// read it.  Partials alternate between two buffers for the same reason.
+// Row, tile and scene sums are formed as in solver.cu (pcg_common.cuh), so
+// both give the same bits and a scene's result does not depend on the batch.
+//
+// What bounds it: in FP64 the SM's FP64 pipe, 19 cycles per warp instruction
+// (16 warps x 135 products of 512 vertices' rows are 41,000 of an iteration's
+// 59,000 cycles); in FP32 latency (row sums 8,400 of 19,800 cycles, the two
+// meetings and the scalars most of the rest).  68,921 vertices, us an iteration:
+// FP64 45.8 -> 28.7 (365 iterations: step 19.4 -> 12.8 ms), FP32 17.0 -> 10.1
+// (383: 7.0 -> 4.4 ms); two cubes in contact, 31,250 vertices, FP64 56 -> 27;
+// 1,331 vertices FP64 23 -> 15.
+//
+// Every wait is bounded; a wait that runs out ends the CTA's part, and the
+// scene's solve is marked failed.  All CTAs are resident (cooperative launch,
+// at most one per SM), so no CTA waits for one that cannot run.
+#include <algorithm>
+#include <atomic>
+
+#include "pcg_common.cuh"
+
+namespace hobak {
+
+namespace {
+
+constexpr int kGridThreads = 512;      // vertices of a CTA, at most (128 registers each)
+constexpr int kGridSmemMax = 225 * 1024;
+constexpr int kSpinLimit = 1 << 21;    // polls of one wait (about a second), then the solve fails
+constexpr int kMaxCtas = 256;          // CTAs of a launch, at most (one per SM)
+
+__device__ __forceinline__ void st_word(ulonglong2* p, double value, unsigned long long tag) {
+  asm volatile(
+      "{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
+      "l"(__double_as_longlong(value)), "l"(tag)
+      : "memory");
+}
+__device__ __forceinline__ void ld_word(const ulonglong2* p, double& value, unsigned long long& tag) {
+  unsigned long long bits;
+  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+               : "=l"(bits), "=l"(tag)
+               : "l"(p)
+               : "memory");
+  value = __longlong_as_double((long long)bits);
+}
+__device__ __forceinline__ int ld_flag(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_flag(int* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// The u of a vertex for iteration `it`, from L2: other SMs write it.
+struct Gather32 {
+  unsigned long long lo, hi;
+  __device__ __forceinline__ void load(const float* u4, int w) {
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(u4 + 4 * (size_t)w)
+                 : "memory");
+  }
+  // repeats the load of vertex() until it fits; clears ok when it does not
+  template <typename Vertex>
+  __device__ __forceinline__ void get(const float* u4, Vertex vertex, int it, float (&x)[3], bool& ok) {
+    for (int n = 0; (int)(hi >> 32) != it && ok; n++) {
+      if (n > kSpinLimit) ok = false;
+      load(u4, vertex());
+    }
+    x[0] = __uint_as_float((unsigned)lo);
+    x[1] = __uint_as_float((unsigned)(lo >> 32));
+    x[2] = __uint_as_float((unsigned)hi);
+  }
+};
+struct Gather64 {  // the caller has waited for the owner's flag
+  double2 a;
+  double z;
+  __device__ __forceinline__ void load(const double* u4, int w) {
+    a = __ldcg(reinterpret_cast<const double2*>(u4) + 2 * (size_t)w);
+    z = __ldcg(u4 + 4 * (size_t)w + 2);
+  }
+  template <typename Vertex>
+  __device__ __forceinline__ void get(const double*, Vertex, int, double (&x)[3], bool&) {
+    x[0] = a.x, x[1] = a.y, x[2] = z;
+  }
+};
+template <typename T>
+struct GatherOf {
+  using type = Gather64;
+};
+template <>
+struct GatherOf<float> {
+  using type = Gather32;
+};
+
+// One block times x into the row sums, in solver.cu's order: FP32 one nested
+// chain per row; FP64 two chains per row, even and odd blocks.
+template <typename T>
+struct RowSums {
+  T a[sizeof(T) == 4 ? 3 : 6];
+  __device__ __forceinline__ RowSums() {
+#pragma unroll
+    for (T& v : a) v = T(0);
+  }
+  __device__ __forceinline__ void add(const T (&m)[9], const T (&x)[3], bool odd) {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int i = 0; i < 3; i++) a[i] = fma(m[3 * i], x[0], fma(m[3 * i + 1], x[1], fma(m[3 * i + 2], x[2], a[i])));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        T& c = odd ? a[3 + i] : a[i];
+        c = fma(m[3 * i], x[0], c);
+        c = fma(m[3 * i + 1], x[1], c);
+        c = fma(m[3 * i + 2], x[2], c);
+      }
+    }
+  }
+  __device__ __forceinline__ void total(T (&w)[3]) const {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      if constexpr (sizeof(T) == 4) w[i] = a[i];
+      else w[i] = a[i] + a[3 + i];
+  }
+};
+
+// ctas: per CTA its scene and the scene's tile it starts at.  tpc: tiles per
+// CTA.  rows: blocks of every row kept in shared memory (even in FP64).
+// scratch: doubles of the exchange area.
+template <int TV, typename T>
+__global__ void __launch_bounds__(kGridThreads, 1)
+    k_pcg_grid(DeviceBatch b, PcgVecs<T> v, const int2* __restrict__ ctas, int tpc, int rows, int scratch) {
+  constexpr bool kF32 = sizeof(T) == sizeof(float);
+  constexpr int kTail = 4;  // FP32: row blocks past the shared ones, fetched before u is there
+  constexpr int kQ = kF32 ? 6 : 2;
+  constexpr int kG = kGroupVerts / TV;
+  using Gather = typename GatherOf<T>::type;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ SolveState ss;
+  __shared__ T warpSum[3 * (kGridThreads / 32)];
+  __shared__ double sums[3], tileSum[3 * (kGridThreads / 64)];
+  __shared__ unsigned nbrBits[kMaxCtas / 32];
+  __shared__ int nbr[kMaxCtas];
+  __shared__ int nNbr, stop;
+  __shared__ T sAlpha, sBeta;
+
+  const int tid = threadIdx.x, NT = blockDim.x;
+  const int2 cta = ctas[blockIdx.x];
+  const int s = cta.x;
+  const SceneParams& sp = b.scenes[s];
+  SolveState& st = b.solve[s];
+  if (st.done) return;  // converged at its start, parked or failed (every CTA of the scene alike)
+  const int ntiles = sp.ntiles, v0 = sp.v0;
+  const int slot = cta.y + tid / TV;  // the thread's tile of the scene
+  const int u = slot < ntiles ? b.tileV0[sp.tile0 + slot] + tid % TV : v0;
+  const bool valid = slot < ntiles && u < b.tileV1[sp.tile0 + slot];
+  const int own = valid ? u : v0;  // a vertex that any gather may read
+
+  double* area = reinterpret_cast<double*>(smem);
+  T* mat = reinterpret_cast<T*>(area + scratch);
+  int* col = reinterpret_cast<int*>(mat + (size_t)9 * rows * NT);  // both [entry][thread]
+
+  if (tid == 0) {
+    ss = st;
+    nNbr = 0;
+    stop = 0;
+  }
+  if (tid < kMaxCtas / 32) nbrBits[tid] = 0u;
+  __syncthreads();
+
+  // ---- the row's blocks and columns; the vertex's vectors (p = s = d = 0) ----
+  const int nCta = (ntiles + tpc - 1) / tpc, ctaVerts = tpc * TV;
+  T* u4 = v.p;  // p and s live in registers here: their buffers hold the shared u
+  int len = 0;
+  size_t lb = 0, cb = 0;
+  T un[3], p[3], sv[3], d[3], r[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) un[i] = p[i] = sv[i] = d[i] = r[i] = T(0);
+  if (valid) {
+    const T* rsrc = kF32 ? v.r : reinterpret_cast<const T*>(b.r64);
+    len = b.rowptr[u + 1] - b.rowptr[u];
+    lb = lhs_slot(b, u, 0);
+    cb = col_slot(b, u, 0);
+    if (!kF32)
+      for (int j = 0; j < len; j++) {
+        const int c = (__ldg(&b.colS[cb + kSlice * j]) - v0) / ctaVerts;
+        if (!((nbrBits[c / 32] >> (c % 32)) & 1u)) atomicOr(&nbrBits[c / 32], 1u << (c % 32));
+      }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      un[i] = v.u[3 * u + i];
+      r[i] = rsrc[3 * u + i];
+    }
+  }
+  for (int j = 0; j < rows; j++) {  // zeros past the row's end
+    col[(size_t)j * NT + tid] = j < len ? __ldg(&b.colS[cb + kSlice * j]) : own;
+#pragma unroll
+    for (int e = 0; e < 9; e++)
+      mat[((size_t)9 * j + e) * NT + tid] = j < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * j + kSlice * e]) : T(0);
+  }
+  int tailCol[kTail];
+  if (kF32)
+#pragma unroll
+    for (int q = 0; q < kTail; q++) tailCol[q] = rows + q < len ? __ldg(&b.colS[cb + kSlice * (rows + q)]) : own;
+  __syncthreads();
+  if (!kF32)
+    for (int c = tid; c < nCta; c += NT)
+      if ((b.collOn || ((nbrBits[c / 32] >> (c % 32)) & 1u)) && c != cta.y / tpc) nbr[atomicAdd(&nNbr, 1)] = c;
+  // the CTA's contact incidences (CSR by vertex, its vertices are consecutive)
+  int inc0 = 0, inc1 = 0, my0 = 0, my1 = 0;
+  double collScale = 0.0;
+  if (b.collOn) {
+    const int last = min(ntiles, cta.y + tpc) - 1;
+    inc0 = b.coll.incCount[b.tileV0[sp.tile0 + cta.y]];
+    inc1 = b.coll.incCount[b.tileV1[sp.tile0 + last]];
+    if (valid && b.freeMask[u]) {
+      my0 = b.coll.incCount[u];
+      my1 = b.coll.incCount[u + 1];
+    }
+    if (inc1 > inc0) collScale = collision_lhs_scale(b, s);
+  }
+  const int lenMax = __reduce_max_sync(0xffffffffu, len);
+  __syncthreads();
+  int* flags = b.gridFlags + sp.tile0;  // a CTA's flag: that of its first tile
+  const bool whole = tpc == kG;         // partials: one per group, else one per tile
+  const int nGroups = (ntiles + kG - 1) / kG, nParts = whole ? nGroups : ntiles;
+  bool ok = true;  // this thread's waits
+  int failed = 0;  // some thread's wait ran out (the same in all threads)
+
+  for (int it = 1;; it++) {
+    if (it > 1 && tid == NT - 1) pcg_reciprocals(ss);
+    RowSums<T> acc;
+    if constexpr (kF32) {
+      // the row's tail needs no u: its loads go ahead of the gathers, and all
+      // of the tail's and the first blocks' gathers before their uses
+      T tail[kTail][9];
+      Gather gt[kTail];
+#pragma unroll
+      for (int q = 0; q < kTail; q++)
+#pragma unroll
+        for (int e = 0; e < 9; e++)
+          tail[q][e] = rows + q < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * (rows + q) + kSlice * e]) : T(0);
+      const int nsm = min(lenMax, rows);
+      for (int j = 0; j < nsm; j += kQ) {
+        Gather g[kQ];
+#pragma unroll
+        for (int q = 0; q < kQ; q++) g[q].load(u4, j + q < nsm ? col[(size_t)(j + q) * NT + tid] : own);
+        if (j + kQ >= nsm && lenMax > rows)
+#pragma unroll
+          for (int q = 0; q < kTail; q++) gt[q].load(u4, tailCol[q]);
+#pragma unroll
+        for (int q = 0; q < kQ; q++)
+          if (j + q < nsm) {
+            T x[3], m[9];
+            g[q].get(u4, [&] { return col[(size_t)(j + q) * NT + tid]; }, it, x, ok);
+#pragma unroll
+            for (int e = 0; e < 9; e++) m[e] = mat[((size_t)9 * (j + q) + e) * NT + tid];
+            acc.add(m, x, false);
+          }
+      }
+      if (lenMax > rows) {
+#pragma unroll
+        for (int q = 0; q < kTail; q++) {
+          T x[3];
+          gt[q].get(u4, [&] { return tailCol[q]; }, it, x, ok);
+          acc.add(tail[q], x, false);
+        }
+        for (int j = rows + kTail; j < len; j++) {  // rows longer than the mesh's usual
+          T m[9], x[3];
+          Gather g;
+          const int w = __ldg(&b.colS[cb + kSlice * j]);
+          g.load(u4, w);
+#pragma unroll
+          for (int e = 0; e < 9; e++) m[e] = __ldg(&v.lhs[lb + (size_t)kSlotVals * j + kSlice * e]);
+          g.get(u4, [&] { return w; }, it, x, ok);
+          acc.add(m, x, false);
+        }
+      }
+    } else {
+      for (int i = tid; i < nNbr; i += NT) {
+        const int* f = flags + nbr[i] * tpc;
+        int n = 0;
+        while (ld_flag(f) < it && ok)
+          if (++n > kSpinLimit) ok = false;
+      }
+      if ((failed = __syncthreads_or(!ok))) break;
+      // Two blocks per trip (the chains of even and odd blocks), the next
+      // trip's u ahead of this trip's products.  FP64-pipe bound: the bounds
+      // are the warp's, so that no product is issued for nobody.
+      Gather g[kQ];
+      auto gather = [&](int j) {
+#pragma unroll
+        for (int q = 0; q < kQ; q++) {
+          const int w = j + q < rows  ? col[(size_t)(j + q) * NT + tid]
+                        : j + q < len ? __ldg(&b.colS[cb + kSlice * (j + q)])
+                                      : own;
+          g[q].load(u4, w);
+        }
+      };
+      gather(0);
+      for (int j = 0; j < lenMax; j += kQ) {
+        T m[kQ][9], x[kQ][3];
+        if (j < rows) {
+#pragma unroll
+          for (int q = 0; q < kQ; q++)
+#pragma unroll
+            for (int e = 0; e < 9; e++) m[q][e] = mat[((size_t)9 * (j + q) + e) * NT + tid];
+        } else {
+#pragma unroll
+          for (int q = 0; q < kQ; q++)
+#pragma unroll
+            for (int e = 0; e < 9; e++)
+              m[q][e] = j + q < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * (j + q) + kSlice * e]) : T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < kQ; q++) g[q].get(u4, [] { return 0; }, it, x[q], ok);
+        if (j + kQ < lenMax) gather(j + kQ);
+        acc.add(m[0], x[0], false);
+        if (j + 1 < lenMax) acc.add(m[1], x[1], true);
+      }
+    }
+    T w[3];
+    acc.total(w);
+    if (inc1 > inc0) {
+      // contact: an incidence per thread, then every vertex adds its own in order
+      double cr[3] = {0.0, 0.0, 0.0};
+      for (int base = inc0; base < inc1; base += NT) {
+        if (base + tid < inc1) {
+          double t[3];
+          collision_incidence<T>(
+              b.coll, base + tid,
+              [&](int id, T (&x)[3]) {
+                Gather g;
+                g.load(u4, id);
+                g.get(u4, [&] { return id; }, it, x, ok);
+              },
+              t);
+#pragma unroll
+          for (int i = 0; i < 3; i++) area[3 * tid + i] = t[i];
+        }
+        __syncthreads();
+        for (int k = max(my0, base); k < min(my1, base + NT); k++)
+#pragma unroll
+          for (int i = 0; i < 3; i++) cr[i] = __dadd_rn(cr[i], area[3 * (k - base) + i]);
+        __syncthreads();
+      }
+      if (my1 > my0)
+#pragma unroll
+        for (int i = 0; i < 3; i++) w[i] += T(__dmul_rn(cr[i], collScale));
+    }
+    // ---- |r|^2, (r, u), (w, u): tile sums, exchanged ----
+    T t0 = T(0), t1 = T(0), t2 = T(0);
+    if (valid) {
+      t2 = dot3v(w[0], w[1], w[2], un[0], un[1], un[2]);
+      t1 = dot3v(r[0], r[1], r[2], un[0], un[1], un[2]);
+      t0 = dot3v(r[0], r[1], r[2], r[0], r[1], r[2]);
+    }
+    double mine = 0.0;   // tile or group sum this thread publishes
+    int pub = -1;        // its partial (index in the scene), component pubC
+    int pubC = 0;
+    if constexpr (kF32) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+        t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+        t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+      }
+      if (tid % 32 == 0) {
+        warpSum[3 * (tid / 32)] = t0;
+        warpSum[3 * (tid / 32) + 1] = t1;
+        warpSum[3 * (tid / 32) + 2] = t2;
+      }
+      if ((failed = __syncthreads_or(!ok))) break;
+      auto tile = [&](int t, int c) {  // block_sum3's order over the tile's warps
+        T a = T(0);
+#pragma unroll
+        for (int i = 0; i < TV / 32; i++) a += warpSum[3 * (t * (TV / 32) + i) + c];
+        return double(a);
+      };
+      if (whole && tid < 3) {
+        mine = group_sum<TV>([&](int t) { return tile(t, tid); });
+        pub = cta.y / kG;
+        pubC = tid;
+      } else if (!whole && tid < 3 * tpc && cta.y + tid / 3 < ntiles) {
+        mine = tile(tid / 3, tid % 3);
+        pub = cta.y + tid / 3;
+        pubC = tid % 3;
+      }
+    } else {
+      area[tid] = t0;
+      area[NT + tid] = t1;
+      area[2 * NT + tid] = t2;
+      __syncthreads();
+      // a warp per (component, tile); a group's four sums meet in shared memory
+      for (int k = tid / 32; k < 3 * tpc; k += NT / 32) {
+        const double t = tile_sum64<TV>(reinterpret_cast<double*>(area) + (k / tpc) * NT + (k % tpc) * TV);
+        if (tid % 32 == 0) tileSum[k] = t;
+      }
+      __syncthreads();
+      if (whole && tid < 3) {
+        mine = group_sum<TV>([&](int t) { return tileSum[tid * tpc + t]; });
+        pub = cta.y / kG;
+        pubC = tid;
+      } else if (!whole && tid < 3 * tpc && cta.y + tid % tpc < ntiles) {
+        mine = tileSum[tid];
+        pub = cta.y + tid % tpc;
+        pubC = tid / tpc;
+      }
+    }
+    ulonglong2* words = reinterpret_cast<ulonglong2*>(b.gridPartials) +
+                        3 * ((it & 1) * (size_t)b.gridTilesCap + sp.tile0);
+    if (pub >= 0) st_word(words + 3 * (size_t)pub + pubC, mine, (unsigned long long)it);
+    for (int i = tid; i < 3 * nParts; i += NT) {
+      double value;
+      unsigned long long tag;
+      for (int n = 0;; n++) {
+        ld_word(words + i, value, tag);
+        if (tag == (unsigned long long)it || !ok) break;
+        if (n > kSpinLimit) ok = false;
+      }
+      area[(i % 3) * nParts + i / 3] = value;
+    }
+    failed = __syncthreads_or(!ok);
+    for (int c = tid / 32; c < 3; c += NT / 32) {
+      const double* q = area + c * nParts;
+      const double t = whole ? scene_sum(nGroups, [&](int g) { return q[g]; }) : scene_sum(nGroups, [&](int g) {
+        return group_sum<TV>([&](int i) { return g * kG + i < ntiles ? q[g * kG + i] : 0.0; });
+      });
+      if (tid % 32 == 0) sums[c] = t;
+    }
+    T M[9];
+    if (valid)
+#pragma unroll
+      for (int e = 0; e < 9; e++) M[e] = v.minv[9 * (size_t)u + e];
+    __syncthreads();
+    if (tid == 0) {
+      stop = pcg_decide<T>(ss, sums[0], sums[1], sums[2]) ? 1 : 0;
+      if constexpr (kF32) {
+        sAlpha = ss.alphaF;
+        sBeta = ss.betaF;
+      } else {
+        sAlpha = ss.alpha;
+        sBeta = ss.beta;
+      }
+    }
+    __syncthreads();
+    if (stop || failed) break;
+    // ---- p = u + beta p, s = w + beta s, d += alpha p, r -= alpha s, u = Minv r ----
+    const T alpha = sAlpha, beta = sBeta;
+    if (valid) {
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        p[i] = un[i] + beta * p[i];
+        sv[i] = w[i] + beta * sv[i];
+        r[i] = r[i] - alpha * sv[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 3; i++) un[i] = M[3 * i] * r[0] + M[3 * i + 1] * r[1] + M[3 * i + 2] * r[2];
+      publish_u(u4, u, un, it + 1);
+    }
+    if (!kF32) {
+      __syncthreads();
+      if (tid == 0) st_flag(flags + cta.y, it + 1);  // after the barrier: covers the whole CTA's u
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) d[i] = d[i] + alpha * p[i];
+  }
+  if (valid)
+#pragma unroll
+    for (int i = 0; i < 3; i++) v.d[3 * u + i] = d[i];
+  // A CTA whose wait ran out publishes nothing more, so the scene's first CTA
+  // runs out too, unless this iteration was the last.
+  if (tid == 0 && cta.y == 0) {
+    if (failed) {
+      ss.converged = kSolveTimedOut;
+      ss.outerDone = 1;
+    }
+    ss.done = 1;
+    st = ss;
+  }
+}
+
+template <int TV, typename T>
+cudaError_t launch_tv(const DeviceBatch& b, const PcgVecs<T>& v, const GridPlan& g, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)g.ctas);
+  cfg.blockDim = dim3((unsigned)(g.tpc * TV));
+  cfg.dynamicSmemBytes = g.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_pcg_grid<TV, T>, b, v, g.list, g.tpc, g.rows, g.scratch);
+}
+
+}  // namespace
+
+// The line between the one launch and the loop: whether the tiles are resident
+// at once, one CTA of at most 512 threads (128 registers each) per SM; below it
+// the launch was the faster at every size measured (343 to 68,921 vertices,
+// 1.3 to 2.0 times an iteration).
+// Tiles per CTA so that the tiles of the given scenes (their tile counts) take
+// at most one CTA per SM, the fewest that does (an SM's FP64 pipe and L2 port
+// are what an iteration runs at); none: they do not fit, and solver.cu's loop
+// runs them.  rows: the blocks of each row that then fit in shared memory.
+GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, int longestRow, bool mixed, int sms) {
+  GridPlan g{};
+  int most = 0;
+  for (int s = 0; s < n; s++) most = std::max(most, tiles[s]);
+  if (most == 0) return g;
+  for (int tpc = 1; tpc * tileV <= kGridThreads; tpc++) {
+    long long ctas = 0;
+    for (int s = 0; s < n; s++) ctas += (tiles[s] + tpc - 1) / tpc;
+    if (ctas > std::min(sms, kMaxCtas)) continue;
+    const int threads = tpc * tileV;
+    g.ctas = (int)ctas;
+    g.tpc = tpc;
+    g.scratch = (3 * std::max(most, threads) + 1) / 2 * 2;
+    const size_t row = (size_t)threads * (9 * (mixed ? sizeof(float) : sizeof(double)) + sizeof(int));
+    int rows = (int)std::min<size_t>(longestRow, (kGridSmemMax - sizeof(double) * g.scratch) / row);
+    if (!mixed) rows = longestRow % 2 && rows == longestRow && (rows + 1) * row + sizeof(double) * g.scratch <= kGridSmemMax
+                           ? rows + 1
+                           : rows / 2 * 2;
+    g.rows = rows;
+    g.smem = sizeof(double) * g.scratch + row * rows;
+    return g;
+  }
+  return g;
+}
+
+// Dynamic shared-memory opt-in (once per process, outside capture).
+int configure_grid_pcg() {
+  static std::atomic<int> done{0};
+  if (done.load()) return 0;
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_pcg_grid<64, float>, attr, kGridSmemMax);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<128, float>, attr, kGridSmemMax);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<64, double>, attr, kGridSmemMax);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<128, double>, attr, kGridSmemMax);
+  if (e != cudaSuccess) return (int)e;
+  done.store(1);
+  return 0;
+}
+
+template <typename T>
+int launch_grid_pcg(const DeviceBatch& b, const PcgVecs<T>& v, const GridPlan& g, cudaStream_t s) {
+  return (int)(b.tileV == 64 ? launch_tv<64, T>(b, v, g, s) : launch_tv<128, T>(b, v, g, s));
+}
+template int launch_grid_pcg<double>(const DeviceBatch&, const PcgVecs<double>&, const GridPlan&, cudaStream_t);
+template int launch_grid_pcg<float>(const DeviceBatch&, const PcgVecs<float>&, const GridPlan&, cudaStream_t);
+
+}  // namespace hobak

@@ -35,9 +35,8 @@
 // order), so results are bitwise reproducible and a scene's result does not
 // depend on the batch around it.
 #include <algorithm>
-#include <cfloat>
 
-#include "kernels.cuh"
+#include "pcg_common.cuh"
 
 namespace hobak {
 
@@ -47,134 +46,6 @@ namespace {
 // per tile): vector kernels and the SpMV run one thread per vertex (TV
 // threads), the update and residual one thread per scalar row.  The batch's
 // tile size is an autotuned launch shape (DeviceBatch::tileV).
-
-// Fixed-order sum over the CTA; result valid in thread 0.  NT multiple of 32.
-// The whole tree runs in R (FP32 for the inner solve of the mixed path) and
-// only the CTA's total is widened to FP64: a conversion per warp costs a
-// 16-cycle issue on GB300's 2-lane FP64 pipe even when one lane uses it.
-template <int NT, typename R>
-__device__ __forceinline__ double block_sum(R v, double* sh) {
-  R* shr = reinterpret_cast<R*>(sh);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x / 32, l = threadIdx.x % 32;
-  if (l == 0) shr[w] = v;
-  __syncthreads();
-  double s = 0;
-  if (threadIdx.x == 0) {
-    R t = R(0);
-#pragma unroll
-    for (int i = 0; i < NT / 32; i++) t += shr[i];
-    s = double(t);
-  }
-  __syncthreads();
-  return s;
-}
-
-// Two sums in one pass (one pair of barriers); results valid in thread 0.
-// `sh` holds 2 * NT / 32 doubles.
-template <int NT, typename R>
-__device__ __forceinline__ void block_sum2(R a, R b, double* sh, double& sa, double& sb) {
-  R* shr = reinterpret_cast<R*>(sh);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-  }
-  const int w = threadIdx.x / 32, l = threadIdx.x % 32;
-  if (l == 0) {
-    shr[w] = a;
-    shr[NT / 32 + w] = b;
-  }
-  __syncthreads();
-  sa = 0.0;
-  sb = 0.0;
-  if (threadIdx.x == 0) {
-    R ta = R(0), tb = R(0);
-#pragma unroll
-    for (int i = 0; i < NT / 32; i++) {
-      ta += shr[i];
-      tb += shr[NT / 32 + i];
-    }
-    sa = double(ta);
-    sb = double(tb);
-  }
-  __syncthreads();
-}
-
-// Three sums in one pass (one pair of barriers), each in the order of
-// block_sum; results valid in thread 0.  `sh` holds 3 * NT / 32 doubles.
-template <int NT, typename R>
-__device__ __forceinline__ void block_sum3(R a, R b, R c, double* sh, double (&out)[3]) {
-  R* shr = reinterpret_cast<R*>(sh);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-  }
-  const int w = threadIdx.x / 32, l = threadIdx.x % 32;
-  if (l == 0) {
-    shr[w] = a;
-    shr[NT / 32 + w] = b;
-    shr[2 * (NT / 32) + w] = c;
-  }
-  __syncthreads();
-  out[0] = out[1] = out[2] = 0.0;
-  if (threadIdx.x == 0) {
-    R ta = R(0), tb = R(0), tc = R(0);
-#pragma unroll
-    for (int i = 0; i < NT / 32; i++) {
-      ta += shr[i];
-      tb += shr[NT / 32 + i];
-      tc += shr[2 * (NT / 32) + i];
-    }
-    out[0] = double(ta);
-    out[1] = double(tb);
-    out[2] = double(tc);
-  }
-  __syncthreads();
-}
-
-// After thread 0 wrote the CTA's partial(s): true in the CTA that finishes
-// the scene's reduction (ticket == ntiles - 1).  Only thread 0 published
-// anything the last CTA reads, so only it fences before taking its ticket.
-// The ticket is reset for reuse.
-__device__ __forceinline__ bool last_tile(unsigned* ticket, int ntiles, int* flag) {
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned t = atomicAdd(ticket, 1u);
-    *flag = (t == (unsigned)(ntiles - 1));
-    if (*flag) *ticket = 0u;
-  }
-  __syncthreads();
-  const bool last = *flag != 0;
-  if (last) __threadfence();
-  return last;
-}
-
-// Sum partial[(tile0 + i) * kPartials + comp] over i < n in a fixed order.
-template <int NT>
-__device__ __forceinline__ double sum_partials(const double* partial, int tile0, int n, int comp, double* sh) {
-  double s = 0;
-  for (int i = threadIdx.x; i < n; i += NT) s += __ldcg(&partial[(size_t)(tile0 + i) * kPartials + comp]);
-  return block_sum<NT>(s, sh);
-}
-
-// Partials 0..2 of a scene's tiles, each summed in tile order (one pass).
-template <int NT>
-__device__ __forceinline__ void sum_partials3(const double* partial, int tile0, int n, double* sh, double (&out)[3]) {
-  double a = 0, b = 0, c = 0;
-  for (int i = threadIdx.x; i < n; i += NT) {
-    const double* q = partial + (size_t)(tile0 + i) * kPartials;
-    a += __ldcg(q);
-    b += __ldcg(q + 1);
-    c += __ldcg(q + 2);
-  }
-  block_sum3<NT>(a, b, c, sh, out);
-}
-
-__device__ __forceinline__ bool finite(double x) { return x == x && fabs(x) <= DBL_MAX; }
 
 // Programmatic dependent launch (sm_90 and later).  The PCG loop kernels are
 // launched with programmatic stream serialisation: the next kernel's CTAs may
@@ -667,6 +538,13 @@ __global__ void __launch_bounds__(TV) k_inner_init(DeviceBatch b, PcgVecs<T> v) 
     }
     return;
   }
+  if (b.gridOn) {  // the one-launch PCG (pcg_grid.cu): no partials yet, the first u published
+    if (threadIdx.x < 6) {
+      const size_t word = 3 * ((threadIdx.x / 3) * (size_t)b.gridTilesCap + tile) + threadIdx.x % 3;
+      reinterpret_cast<ulonglong2*>(b.gridPartials)[word] = make_ulonglong2(0ull, 0ull);
+    }
+    if (threadIdx.x == 0) b.gridFlags[tile] = 1;
+  }
   const int u = b.tileV0[tile] + threadIdx.x;
   const double sc = (sizeof(T) != sizeof(double) && st.rScale > 0.0) ? st.rScale : 1.0;
   const double inv = 1.0 / sc;  // exact: sc is a power of two
@@ -678,17 +556,21 @@ __global__ void __launch_bounds__(TV) k_inner_init(DeviceBatch b, PcgVecs<T> v) 
       r3[i] = T(b.r64[3 * u + i] * inv);
       if (sizeof(T) != sizeof(double)) v.r[3 * u + i] = r3[i];
       v.d[3 * u + i] = T(0);
-      v.p[3 * u + i] = T(0);
-      v.s[3 * u + i] = T(0);
+      if (!b.gridOn) {
+        v.p[3 * u + i] = T(0);
+        v.s[3 * u + i] = T(0);
+      }
       rr += r3[i] * r3[i];
     }
     const T* M = v.minv + 9 * (size_t)u;
+    T u3[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-      const T ui = M[3 * i] * r3[0] + M[3 * i + 1] * r3[1] + M[3 * i + 2] * r3[2];
-      v.u[3 * u + i] = ui;
-      ru += r3[i] * ui;
+      u3[i] = M[3 * i] * r3[0] + M[3 * i + 1] * r3[1] + M[3 * i + 2] * r3[2];
+      v.u[3 * u + i] = u3[i];
+      ru += r3[i] * u3[i];
     }
+    if (b.gridOn) publish_u(v.p, u, u3, 1);
   }
   const double trr = block_sum<TV>(rr, sh);
   const double tru = block_sum<TV>(ru, sh);
@@ -719,33 +601,6 @@ __global__ void __launch_bounds__(TV) k_inner_init(DeviceBatch b, PcgVecs<T> v) 
   }
 }
 
-// Row i of vertex u of w H_coll x (w = collision_lhs_scale), H_coll = sum over the
-// vertex's collision tets of (c c^T) (x) G (free rows only; x vanishes on
-// pinned rows, which keeps the columns masked too).  FP64 throughout: the
-// contact blocks are not part of the (possibly FP32) assembled LHS.
-template <typename T>
-__device__ __forceinline__ double collision_row(const DeviceBatch& b, int u, int i, const T* __restrict__ x) {
-  const DeviceCollisions& c = b.coll;
-  const int k0 = c.incCount[u], k1 = c.incCount[u + 1];
-  if (k0 == k1) return 0.0;
-  const double scale = collision_lhs_scale(b, b.vertexScene[u]);
-  double acc = 0.0;
-  for (int k = k0; k < k1; k++) {
-    const int e = c.incList[k], p = e >> 2, a = e & 3;
-    const int4 ct = c.pairTet[p];
-    const double* C = c.pairC + 4 * (size_t)p;
-    const double* G = c.pairG + 9 * (size_t)p;
-    const int id[4] = {ct.x, ct.y, ct.z, ct.w};
-    double z[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) z[j] += C[q] * double(x[3 * id[q] + j]);
-    acc += C[a] * (G[i] * z[0] + G[i + 3] * z[1] + G[i + 6] * z[2]);
-  }
-  return scale * acc;
-}
-
 // Threads of an SpMV CTA: one per vertex in FP32 (the sliced LHS makes
 // every matrix and column load of a warp one line, and a vertex's three rows
 // share its column loads and u gathers); one per scalar row in FP64, whose
@@ -754,56 +609,15 @@ __device__ __forceinline__ double collision_row(const DeviceBatch& b, int u, int
 template <typename T>
 __host__ __device__ constexpr int spmv_threads(int TV) { return sizeof(T) == sizeof(float) ? TV : 3 * TV; }
 
-// The scene's iteration step in its last SpMV CTA (thread 0), from
-// rho = |r|^2, gamma = (r, u) and delta = (w, u): after an update, stop when
-// |r|^2 < threshold (ConjugateGradient.h:75-78), on a non-finite value, or at
-// the iteration limit; otherwise beta and alpha for this iteration's update,
-// which the iteration count then includes.
+// pcg_decide on the scene's state in global memory.  A negative threshold
+// marks the kernel timing of hobak_batch_time_kernels, which repeats the SpMV
+// on fixed vectors: the scalars stay as they are.
 template <typename T>
 __device__ __forceinline__ void spmv_decide(const DeviceBatch& b, SolveState& st, double rho, double gamma,
                                             double delta) {
-  // a negative threshold marks the kernel timing of hobak_batch_time_kernels,
-  // which repeats the SpMV on fixed vectors: the scalars stay as they are
   if (st.innerThreshold < 0.0) return;
-  if (st.iters > 0) {
-    st.rr = rho;
-    bool stop = false;
-    if (rho < st.innerThreshold) {
-      stop = true;
-    } else if (!finite(rho) || !finite(gamma) || !finite(st.alpha)) {
-      stop = true;
-      st.converged = -1;
-      st.outerDone = 1;
-    } else if (st.totalIters >= st.maxit) {
-      stop = true;
-    }
-    if (stop) {
-      st.done = 1;
-      atomicSub(b.active, 1);
-      if (sizeof(T) == sizeof(double) && st.converged >= 0) {
-        // FP64 path: the recursive residual is the solver's verdict (Eigen)
-        st.rr64 = rho;
-        st.converged = rho < st.threshold ? 1 : 0;
-        st.outerDone = 1;
-      }
-      return;
-    }
-  }
-  st.delta = delta;
-  if (st.iters == 0) {
-    st.beta = 0.0;
-    st.alpha = gamma / delta;
-  } else {
-    const double beta = gamma / st.gamma;  // st.gamma: the previous iteration's (r, u)
-    st.beta = beta;
-    st.alpha = gamma / (delta - beta * gamma / st.alpha);
-  }
-  st.gammaOld = st.gamma;
-  st.gamma = gamma;
-  st.alphaF = float(st.alpha);
-  st.betaF = float(st.beta);
-  st.iters += 1;
-  st.totalIters += 1;
+  if (pcg_decide<T>(st, rho, gamma, delta)) atomicSub(b.active, 1);
+  else pcg_reciprocals(st);
 }
 
 // FP64: w = A u, one thread per scalar row (9 DFMA per block over the row's
@@ -812,7 +626,7 @@ __device__ __forceinline__ void spmv_decide(const DeviceBatch& b, SolveState& st
 // (10 vertices) read three lines per load.
 template <int TV, typename T>
 __device__ __forceinline__ void spmv_tile_rows(const DeviceBatch& b, const PcgVecs<T>& v, int tile, double* sh,
-                                               int* flag) {
+                                               T* rows, int* flag) {
   // before the dependency wait: what the previous kernel does not write
   const int s = b.tileScene[tile];
   const int row = 3 * b.tileV0[tile] + threadIdx.x;
@@ -857,25 +671,48 @@ __device__ __forceinline__ void spmv_tile_rows(const DeviceBatch& b, const PcgVe
         }
       }
     }
-    T acc = acc0 + acc1;
-    if (b.collOn && b.freeMask[u]) acc += T(collision_row<T>(b, u, i, uu));
-    v.w[row] = acc;
-    const T ui = uu[row], ri = r[row];
-    dl = acc * ui;
-    gl = ri * ui;
-    rl = ri * ri;
+    rows[threadIdx.x] = acc0 + acc1;
   }
-  double t[3];
-  block_sum3<3 * TV>(rl, gl, dl, sh, t);
-  if (threadIdx.x == 0) {
-    b.partial[kPartials * tile] = t[0];
-    b.partial[kPartials * tile + 1] = t[1];
-    b.partial[kPartials * tile + 2] = t[2];
+  __syncthreads();
+  // per vertex from here on (the order of every PCG path): contact rows, w
+  // and the three dot products
+  const int vt = b.tileV0[tile] + threadIdx.x;
+  if (threadIdx.x < TV && vt < b.tileV1[tile]) {
+    const T* __restrict__ uu = v.u;
+    T a0 = rows[3 * threadIdx.x], a1 = rows[3 * threadIdx.x + 1], a2 = rows[3 * threadIdx.x + 2];
+    if (b.collOn && b.freeMask[vt]) {
+      double cr[3];
+      collision_rows<T>(b, vt, [&](int id, T* x) { x[0] = uu[3 * id], x[1] = uu[3 * id + 1], x[2] = uu[3 * id + 2]; },
+                        cr);
+      a0 += T(cr[0]);
+      a1 += T(cr[1]);
+      a2 += T(cr[2]);
+    }
+    v.w[3 * vt] = a0;
+    v.w[3 * vt + 1] = a1;
+    v.w[3 * vt + 2] = a2;
+    const T u0 = uu[3 * vt], u1 = uu[3 * vt + 1], u2 = uu[3 * vt + 2];
+    const T r0 = r[3 * vt], r1 = r[3 * vt + 1], r2 = r[3 * vt + 2];
+    dl = dot3v(a0, a1, a2, u0, u1, u2);
+    gl = dot3v(r0, r1, r2, u0, u1, u2);
+    rl = dot3v(r0, r1, r2, r0, r1, r2);
   }
+  __syncthreads();
+  if (threadIdx.x < TV) {  // 3 * TV values, component by component
+    rows[threadIdx.x] = rl;
+    rows[TV + threadIdx.x] = gl;
+    rows[2 * TV + threadIdx.x] = dl;
+  }
+  __syncthreads();
+  if (threadIdx.x < 96) {
+    const double t = tile_sum64<TV>(rows + TV * (threadIdx.x / 32));
+    if (threadIdx.x % 32 == 0) b.partial[kPartials * tile + threadIdx.x / 32] = t;
+  }
+  __syncthreads();  // last_tile's fence by thread 0 covers the three writers
   const SceneParams& sp = b.scenes[s];
   if (!last_tile(&st.ticketA, sp.ntiles, flag)) return;
   double tot[3];
-  sum_partials3<3 * TV>(b.partial, sp.tile0, sp.ntiles, sh, tot);
+  scene_sums<3 * TV, TV>(b.partial, sp.tile0, sp.ntiles, sh, tot);
   if (threadIdx.x == 0) spmv_decide<T>(b, st, tot[0], tot[1], tot[2]);
 }
 
@@ -943,18 +780,21 @@ __device__ __forceinline__ void spmv_tile(const DeviceBatch& b, const PcgVecs<T>
       }
     }
     if (b.collOn && b.freeMask[u]) {
-      a0 += T(collision_row<T>(b, u, 0, uu));
-      a1 += T(collision_row<T>(b, u, 1, uu));
-      a2 += T(collision_row<T>(b, u, 2, uu));
+      double cr[3];
+      collision_rows<T>(b, u, [&](int id, T* x) { x[0] = uu[3 * id], x[1] = uu[3 * id + 1], x[2] = uu[3 * id + 2]; },
+                        cr);
+      a0 += T(cr[0]);
+      a1 += T(cr[1]);
+      a2 += T(cr[2]);
     }
     v.w[3 * u] = a0;
     v.w[3 * u + 1] = a1;
     v.w[3 * u + 2] = a2;
     const T u0 = uu[3 * u], u1 = uu[3 * u + 1], u2 = uu[3 * u + 2];
     const T r0 = v.r[3 * u], r1 = v.r[3 * u + 1], r2 = v.r[3 * u + 2];
-    dl = a0 * u0 + a1 * u1 + a2 * u2;
-    gl = r0 * u0 + r1 * u1 + r2 * u2;
-    rl = r0 * r0 + r1 * r1 + r2 * r2;
+    dl = dot3v(a0, a1, a2, u0, u1, u2);
+    gl = dot3v(r0, r1, r2, u0, u1, u2);
+    rl = dot3v(r0, r1, r2, r0, r1, r2);
   }
   if (done) return;  // threads without rows (the CTA returns as one)
   double t[3];
@@ -967,7 +807,7 @@ __device__ __forceinline__ void spmv_tile(const DeviceBatch& b, const PcgVecs<T>
   const SceneParams& sp = b.scenes[s];
   if (!last_tile(&st.ticketA, sp.ntiles, flag)) return;
   double tot[3];
-  sum_partials3<TV>(b.partial, sp.tile0, sp.ntiles, sh, tot);
+  scene_sums<TV, TV>(b.partial, sp.tile0, sp.ntiles, sh, tot);
   if (threadIdx.x == 0) spmv_decide<T>(b, st, tot[0], tot[1], tot[2]);
 }
 
@@ -988,8 +828,12 @@ __global__ void __launch_bounds__(spmv_threads<T>(TV)) k_spmv(DeviceBatch b, Pcg
   pdl_trigger();
   const int tile = loop_tile(b);
   if (tile < 0) return;
-  if constexpr (sizeof(T) == sizeof(float)) spmv_tile<TV, T>(b, v, tile, sh, &flag);
-  else spmv_tile_rows<TV, T>(b, v, tile, sh, &flag);
+  if constexpr (sizeof(T) == sizeof(float)) {
+    spmv_tile<TV, T>(b, v, tile, sh, &flag);
+  } else {
+    __shared__ T rows[3 * TV];
+    spmv_tile_rows<TV, T>(b, v, tile, sh, rows, &flag);
+  }
 }
 
 // p = u + beta p; s = w + beta s; d += alpha p; r -= alpha s; u = Minv r
@@ -1150,7 +994,12 @@ __global__ void __launch_bounds__(3 * TV) k_residual(DeviceBatch b) {
       const float* B = A + (size_t)kSlotVals * (k - k0);
       acc += double(B[0]) * b.y[3 * w] + double(B[kSlice]) * b.y[3 * w + 1] + double(B[2 * kSlice]) * b.y[3 * w + 2];
     }
-    if (b.collOn && b.freeMask[u]) acc += collision_row<double>(b, u, i, b.y);
+    if (b.collOn && b.freeMask[u]) {
+      double cr[3];
+      collision_rows<double>(
+          b, u, [&](int id, double* x) { x[0] = b.y[3 * id], x[1] = b.y[3 * id + 1], x[2] = b.y[3 * id + 2]; }, cr);
+      acc += cr[i];
+    }
     const double ri = b.rhs[row] - acc;
     b.r64[row] = ri;
     rr = ri * ri;
