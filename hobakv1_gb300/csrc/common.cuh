@@ -82,7 +82,6 @@ struct SolveState {
   int maxit;
   // inner PCG
   double gamma, gammaOld, delta, alpha, beta, rr, innerThreshold;
-  double gammaInv, alphaInv;  // reciprocals of the last iteration's gamma and alpha
   float alphaF, betaF;  // FP32 copies for the mixed inner solve (no per-thread conversion)
   int iters, done;
   unsigned ticketA, ticketB;

@@ -91,13 +91,14 @@ __device__ __forceinline__ double sum_partials(const double* partial, int tile0,
 }
 
 // Order of the PCG's three dot products, the same on every path so that all
-// give the same bits.  FP64 costs 19 cycles of the SM's pipe per warp
-// instruction however few lanes it has, and 64 cycles of latency, so sums
-// use few instructions in short chains on several warps.
-//   tile    FP32: a tree per warp, the warps in order (block_sum3).  FP64: lane
-//           l adds the tile's vertices l, l + 32, ..., then a warp tree.
-//   group   kGroupVerts / TV consecutive tiles of the scene, added pairwise
-//   scene   lane l adds groups l, l + 32, ..., then a warp tree
+// give the same bits.  An FP64 add costs 19 cycles of the SM's pipe per warp
+// instruction however few of its lanes work, and 64 cycles of latency, so the
+// trees below fill their lanes, and sums run in short chains on several warps.
+//   FP32  tile: a tree per warp, the warps in order (block_sum3); group:
+//         kGroupVerts / TV consecutive tiles of the scene, added pairwise in
+//         FP64; scene: lane l adds groups l, l + 32, ..., then a warp tree
+//   FP64  tile: its 3 TV row products, a tree over every 32, the trees in
+//         order; scene: lane l of 3 TV adds tiles l, l + 3 TV, ..., then as a tile
 constexpr int kGroupVerts = 512;
 
 __device__ __forceinline__ double warp_tree(double v) {
@@ -106,13 +107,64 @@ __device__ __forceinline__ double warp_tree(double v) {
   return v;
 }
 
-// FP64 tile sum by one warp; vals: the tile's TV values.
-template <int TV>
-__device__ __forceinline__ double tile_sum64(const double* vals) {
-  double s = vals[threadIdx.x % 32];
+// Sums of groups g0 .. g0 + 7 (those below n) of 32 values each, get(g, l)
+// value l of group g, by the pairs of an xor-shuffle tree (16, 8, 4, 2, 1), to
+// out[g].  One warp, which halves its number of values per lane with every
+// exchange: 9 adds where eight shuffle trees issue 40.
+template <typename Get>
+__device__ __forceinline__ void tree32_warp(int g0, int n, Get get, double* out) {
+  const int lane = threadIdx.x % 32, l = lane & 15, hi = lane >> 4;
+  const bool b3 = lane & 8, b2 = lane & 4;
+  double a[4];  // lanes 0..15: group g0 + 2 j, lanes 16..31: g0 + 2 j + 1
 #pragma unroll
-  for (int i = 32; i < TV; i += 32) s += vals[i + threadIdx.x % 32];
-  return warp_tree(s);
+  for (int j = 0; j < 4; j++) {
+    const int g = g0 + 2 * j + hi;
+    a[j] = g < n ? get(g, l) + get(g, l + 16) : 0.0;
+  }
+  double c[2];
+#pragma unroll
+  for (int m = 0; m < 2; m++)
+    c[m] = (b3 ? a[2 * m + 1] : a[2 * m]) + __shfl_xor_sync(0xffffffffu, b3 ? a[2 * m] : a[2 * m + 1], 8);
+  double d = (b2 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, b2 ? c[0] : c[1], 4);
+  d += __shfl_xor_sync(0xffffffffu, d, 2);
+  d += __shfl_xor_sync(0xffffffffu, d, 1);
+  const int g = g0 + 4 * (b2 ? 1 : 0) + 2 * (b3 ? 1 : 0) + hi;
+  if ((lane & 3) == 0 && g < n) out[g] = d;
+}
+// ... of all n groups by the CTA's warps
+template <typename Get>
+__device__ __forceinline__ void tree32(int n, Get get, double* out) {
+  for (int g0 = 8 * (threadIdx.x / 32); g0 < n; g0 += 8 * (blockDim.x / 32)) tree32_warp(g0, n, get, out);
+}
+
+// Sum of n values in order.
+__device__ __forceinline__ double chain(const double* v, int n) {
+  double t = v[0];
+  for (int i = 1; i < n; i++) t += v[i];
+  return t;
+}
+
+// FP64: the trees of a scene's three sums over its n tiles' partials,
+// tile(c, i), to out[trees * c + ...]; trees = scene_trees(n): those with a tile
+// in their lanes (the others are zero).
+template <int TV>
+__device__ __forceinline__ int scene_trees(int n) {
+  return n < 3 * TV ? (n + 31) / 32 : 3 * TV / 32;
+}
+template <int TV, typename Tile>
+__device__ __forceinline__ void scene_tree32(int n, Tile tile, double* out) {
+  const int trees = scene_trees<TV>(n), per = (trees + 7) / 8;
+  for (int k = threadIdx.x / 32; k < 3 * per; k += blockDim.x / 32) {
+    const int c = k >= 2 * per ? 2 : k >= per ? 1 : 0;
+    tree32_warp(
+        8 * (k - c * per), trees,
+        [&](int g, int l) {
+          double s = 32 * g + l < n ? tile(c, 32 * g + l) : 0.0;
+          for (int i = 32 * g + l + 3 * TV; i < n; i += 3 * TV) s += tile(c, i);
+          return s;
+        },
+        out + trees * c);
+  }
 }
 
 // The sum of a group's tiles, get(i) its i-th (0 past the scene's last tile).
@@ -131,7 +183,7 @@ __device__ __forceinline__ double scene_sum(int n, Group group) {
   return warp_tree(s);
 }
 
-// The three scene sums from global tile partials, by the last CTA of the
+// FP32: the three scene sums from global tile partials, by the last CTA of the
 // scene; sh: 3 doubles.  Result valid in thread 0.
 template <int NT, int TV>
 __device__ __forceinline__ void scene_sums(const double* partial, int tile0, int n, double* sh, double (&out)[3]) {
@@ -151,13 +203,31 @@ __device__ __forceinline__ void scene_sums(const double* partial, int tile0, int
 
 __device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
+// a / b, correctly rounded, from y = 1 / b correctly rounded (0: not given): a
+// quotient off by little and two of Markstein's corrections ("Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990), a chain
+// of five FMAs (320 cycles in one thread) where the division takes ~630.  Out
+// of the range where the residual is exact, the division.
+__device__ __forceinline__ double divide(double a, double b, double y) {
+  const auto plain = [](double x) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    return e > 523 && e < 1523;
+  };
+  if (!(plain(a) && plain(b) && plain(y))) return a / b;
+  double q = a * y;
+  q = fma(fma(-q, b, a), y, q);
+  return fma(fma(-q, b, a), y, q);
+}
+
 // A scene's iteration step (one thread), from
 // rho = |r|^2, gamma = (r, u) and delta = (w, u): after an update, stop when
 // |r|^2 < threshold (ConjugateGradient.h:75-78), on a non-finite value, or at
 // the iteration limit; otherwise beta and alpha for this iteration's update,
 // which the iteration count then includes.  Returns true when it stops.
+// gammaInv, alphaInv: 1 / st.gamma and 1 / st.alpha where the caller has them.
 template <typename T>
-__device__ __forceinline__ bool pcg_decide(SolveState& st, double rho, double gamma, double delta) {
+__device__ __forceinline__ bool pcg_decide(SolveState& st, double rho, double gamma, double delta,
+                                           double gammaInv = 0.0, double alphaInv = 0.0) {
   if (st.iters > 0) {
     st.rr = rho;
     bool stop = false;
@@ -182,15 +252,13 @@ __device__ __forceinline__ bool pcg_decide(SolveState& st, double rho, double ga
     }
   }
   st.delta = delta;
-  // The reciprocals of the last gamma and alpha are formed off this path
-  // (pcg_reciprocals): one division is left on it, of the ~1,000 cycles each
-  // takes in a single thread.
   if (st.iters == 0) {
     st.beta = 0.0;
     st.alpha = gamma / delta;
   } else {
-    st.beta = gamma * st.gammaInv;
-    st.alpha = gamma / (delta - st.beta * gamma * st.alphaInv);
+    const double beta = divide(gamma, st.gamma, gammaInv);  // st.gamma: the previous iteration's (r, u)
+    st.beta = beta;
+    st.alpha = gamma / (delta - divide(beta * gamma, st.alpha, alphaInv));
   }
   st.gammaOld = st.gamma;
   st.gamma = gamma;
@@ -199,11 +267,6 @@ __device__ __forceinline__ bool pcg_decide(SolveState& st, double rho, double ga
   st.iters += 1;
   st.totalIters += 1;
   return false;
-}
-
-__device__ __forceinline__ void pcg_reciprocals(SolveState& st) {
-  st.gammaInv = 1.0 / st.gamma;
-  st.alphaInv = 1.0 / st.alpha;
 }
 
 // u of a vertex as the one-launch PCG shares it, four wide: in FP32 with the
@@ -230,12 +293,12 @@ __device__ __forceinline__ T dot3v(T a0, T a1, T a2, T b0, T b1, T b2) {
 // Contact: w H_coll x at a vertex (w = collision_lhs_scale), H_coll = sum over
 // its collision tets of (c c^T) (x) G (free rows only; x vanishes on pinned
 // rows, which keeps the columns masked too).  FP64 throughout: the contact
-// blocks are not part of the (possibly FP32) assembled LHS.  One incidence's
-// three rows; load(id, x) reads the vector at a vertex.  Explicit roundings:
-// every PCG path rounds alike.
+// blocks are not part of the (possibly FP32) assembled LHS.  One incidence:
+// t = G sum_q c_q x_q, and the weight c_a of the vertex's own row; load(id, x)
+// reads the vector at a vertex.
 template <typename T, typename Load>
-__device__ __forceinline__ void collision_incidence(const DeviceCollisions& c, int k, Load load, double out[3]) {
-  const int e = c.incList[k], p = e >> 2, a = e & 3;
+__device__ __forceinline__ double collision_incidence(const DeviceCollisions& c, int k, Load load, double (&t)[3]) {
+  const int e = c.incList[k], p = e >> 2;
   const int4 ct = c.pairTet[p];
   const double* C = c.pairC + 4 * (size_t)p;
   const double* G = c.pairG + 9 * (size_t)p;
@@ -247,23 +310,24 @@ __device__ __forceinline__ void collision_incidence(const DeviceCollisions& c, i
 #pragma unroll
   for (int q = 0; q < 4; q++)
 #pragma unroll
-    for (int j = 0; j < 3; j++) z[j] = fma(C[q], double(x[q][j]), z[j]);
+    for (int j = 0; j < 3; j++) z[j] += C[q] * double(x[q][j]);
 #pragma unroll
-  for (int i = 0; i < 3; i++) out[i] = __dmul_rn(C[a], fma(G[i + 6], z[2], fma(G[i + 3], z[1], __dmul_rn(G[i], z[0]))));
+  for (int i = 0; i < 3; i++) t[i] = G[i] * z[0] + G[i + 3] * z[1] + G[i + 6] * z[2];
+  return C[e & 3];
 }
 
 // A vertex's rows, its incidences in order.
 template <typename T, typename Load>
-__device__ __forceinline__ void collision_rows(const DeviceBatch& b, int u, Load load, double out[3]) {
+__device__ __forceinline__ void collision_rows(const DeviceBatch& b, int u, Load load, double (&out)[3]) {
   const DeviceCollisions& c = b.coll;
   const int k0 = c.incCount[u], k1 = c.incCount[u + 1];
   out[0] = out[1] = out[2] = 0.0;
   if (k0 == k1) return;
   for (int k = k0; k < k1; k++) {
     double t[3];
-    collision_incidence<T>(c, k, load, t);
+    const double w = collision_incidence<T>(c, k, load, t);
 #pragma unroll
-    for (int i = 0; i < 3; i++) out[i] = __dadd_rn(out[i], t[i]);
+    for (int i = 0; i < 3; i++) out[i] = fma(w, t[i], out[i]);
   }
   const double scale = collision_lhs_scale(b, b.vertexScene[u]);
 #pragma unroll

@@ -7,10 +7,10 @@
 // iteration of the solve: a CTA per SM owns up to 512 vertices (whole tiles of
 // one scene) for the whole solve, one per thread.  A vertex's u, p, s, d, r
 // stay in registers; the first blocks of its matrix row and their columns in
-// shared memory (as many as fit, the same count for every row); the rest of
-// the row comes from L2.  Per iteration the CTAs of a scene meet twice:
-//   * after the SpMV the partial sums of the three dot products go out as
-//     16-byte words {value, iteration}, written and polled with
+// shared memory (as many as fit, the same count for every row), in FP32 the
+// next four in registers; the rest of the row comes from L2.  Per iteration the CTAs of a scene meet twice:
+//   * the partial sums of the three dot products go out as 16-byte words
+//     {value, iteration}, |r|^2 and (r, u) before the SpMV, (w, u) after it, written and polled with
 //     single-copy-atomic 128-bit accesses, so a reader needs no flag and no
 //     fence; every CTA adds them in the same order and takes the same decision;
 //   * after the update the new u: in FP32 the same way, each vertex's u carries
@@ -25,11 +25,11 @@
 //
 // What bounds it: in FP64 the SM's FP64 pipe, 19 cycles per warp instruction
 // (16 warps x 135 products of 512 vertices' rows are 41,000 of an iteration's
-// 59,000 cycles); in FP32 latency (row sums 8,400 of 19,800 cycles, the two
-// meetings and the scalars most of the rest).  68,921 vertices, us an iteration:
-// FP64 45.8 -> 28.7 (365 iterations: step 19.4 -> 12.8 ms), FP32 17.0 -> 10.1
-// (383: 7.0 -> 4.4 ms); two cubes in contact, 31,250 vertices, FP64 56 -> 27;
-// 1,331 vertices FP64 23 -> 15.
+// 70,000 cycles); in FP32 latency and the gathers (row sums 9,000 of 19,000
+// cycles, the two meetings and the scalars most of the rest).  68,921 vertices,
+// us an iteration: FP64 45.8 -> 34 (365 iterations: step 19.4 -> 14.4 ms),
+// FP32 17.0 -> 9.2 (383: 7.0 -> 4.4 ms); two cubes in contact, 31,250
+// vertices, FP64 56 -> 26; 1,331 vertices FP64 23 -> 15.
 //
 // Every wait is bounded; a wait that runs out ends the CTA's part, and the
 // scene's solve is marked failed.  All CTAs are resident (cooperative launch,
@@ -44,7 +44,7 @@ namespace hobak {
 namespace {
 
 constexpr int kGridThreads = 512;      // vertices of a CTA, at most (128 registers each)
-constexpr int kGridSmemMax = 225 * 1024;
+constexpr int kGridSmemMax = 224 * 1024;
 constexpr int kSpinLimit = 1 << 21;    // polls of one wait (about a second), then the solve fails
 constexpr int kMaxCtas = 256;          // CTAs of a launch, at most (one per SM)
 
@@ -151,14 +151,15 @@ template <int TV, typename T>
 __global__ void __launch_bounds__(kGridThreads, 1)
     k_pcg_grid(DeviceBatch b, PcgVecs<T> v, const int2* __restrict__ ctas, int tpc, int rows, int scratch) {
   constexpr bool kF32 = sizeof(T) == sizeof(float);
-  constexpr int kTail = 4;  // FP32: row blocks past the shared ones, fetched before u is there
+  constexpr int kTail = 4;  // FP32: row blocks past the shared ones, in registers
   constexpr int kQ = kF32 ? 6 : 2;
   constexpr int kG = kGroupVerts / TV;
   using Gather = typename GatherOf<T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ SolveState ss;
-  __shared__ T warpSum[3 * (kGridThreads / 32)];
-  __shared__ double sums[3], tileSum[3 * (kGridThreads / 64)];
+  __shared__ T warpSum[3][kGridThreads / 32];
+  __shared__ double sums[3], recip[2];              // recip: of the last gamma and alpha
+  __shared__ double trees[9 * kGridThreads / 32];  // FP64: sums of 32 rows or tiles
   __shared__ unsigned nbrBits[kMaxCtas / 32];
   __shared__ int nbr[kMaxCtas];
   __shared__ int nNbr, stop;
@@ -219,9 +220,15 @@ __global__ void __launch_bounds__(kGridThreads, 1)
       mat[((size_t)9 * j + e) * NT + tid] = j < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * j + kSlice * e]) : T(0);
   }
   int tailCol[kTail];
-  if (kF32)
+  T tail[kF32 ? kTail : 1][9];  // FP32: the row's next blocks stay in registers
+  if constexpr (kF32)
 #pragma unroll
-    for (int q = 0; q < kTail; q++) tailCol[q] = rows + q < len ? __ldg(&b.colS[cb + kSlice * (rows + q)]) : own;
+    for (int q = 0; q < kTail; q++) {
+      tailCol[q] = rows + q < len ? __ldg(&b.colS[cb + kSlice * (rows + q)]) : own;
+#pragma unroll
+      for (int e = 0; e < 9; e++)
+        tail[q][e] = rows + q < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * (rows + q) + kSlice * e]) : T(0);
+    }
   __syncthreads();
   if (!kF32)
     for (int c = tid; c < nCta; c += NT)
@@ -242,24 +249,73 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   const int lenMax = __reduce_max_sync(0xffffffffu, len);
   __syncthreads();
   int* flags = b.gridFlags + sp.tile0;  // a CTA's flag: that of its first tile
-  const bool whole = tpc == kG;         // partials: one per group, else one per tile
+  const bool whole = kF32 && tpc == kG;  // partials: one per group, else one per tile
   const int nGroups = (ntiles + kG - 1) / kG, nParts = whole ? nGroups : ntiles;
+  constexpr int kTrees = 3 * TV / 32;  // FP64: trees of a tile's rows
+  auto words = [&](int it) {
+    return reinterpret_cast<ulonglong2*>(b.gridPartials) + 3 * ((it & 1) * (size_t)b.gridTilesCap + sp.tile0);
+  };
+  // FP32: warp sums (one value each in warpSum[c]) -> tile or group sums of
+  // component c0 .. c0 + n - 1, published for iteration it
+  auto publish32 = [&](int c0, int n, int it) {
+    auto tile = [&](int t, int c) {  // block_sum3's order over the tile's warps
+      T a = T(0);
+#pragma unroll
+      for (int i = 0; i < TV / 32; i++) a += warpSum[c][t * (TV / 32) + i];
+      return double(a);
+    };
+    if (whole && tid < n)
+      st_word(words(it) + 3 * (cta.y / kG) + c0 + tid, group_sum<TV>([&](int t) { return tile(t, c0 + tid); }), it);
+    else if (!whole && tid < n * tpc && cta.y + tid % tpc < ntiles)
+      st_word(words(it) + 3 * (cta.y + tid % tpc) + c0 + tid / tpc, tile(tid % tpc, c0 + tid / tpc), it);
+  };
+  // FP64: row products in area[c][tile][row] -> the same
+  auto publish64 = [&](int c0, int n, int it) {
+    double* t = trees + c0 * tpc * kTrees;
+    tree32(n * tpc * kTrees, [&](int g, int l) { return area[3 * c0 * NT + 32 * g + l]; }, t);
+    __syncthreads();
+    if (tid < n * tpc && cta.y + tid % tpc < ntiles)
+      st_word(words(it) + 3 * (cta.y + tid % tpc) + c0 + tid / tpc, chain(t + tid * kTrees, kTrees), it);
+  };
+  // |r|^2 and (r, u) of iteration it, known as soon as its u is: ahead of the SpMV
+  auto publish_ru = [&](int it) {
+    if constexpr (kF32) {
+      T t0 = T(0), t1 = T(0);
+      if (valid) {
+        t1 = dot3v(r[0], r[1], r[2], un[0], un[1], un[2]);
+        t0 = dot3v(r[0], r[1], r[2], r[0], r[1], r[2]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+        t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+      }
+      if (tid % 32 == 0) {
+        warpSum[0][tid / 32] = t0;
+        warpSum[1][tid / 32] = t1;
+      }
+      __syncthreads();
+      publish32(0, 2, it);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        area[3 * tid + i] = valid ? r[i] * r[i] : 0.0;
+        area[3 * NT + 3 * tid + i] = valid ? r[i] * un[i] : 0.0;
+      }
+      __syncthreads();
+      publish64(0, 2, it);
+    }
+  };
   bool ok = true;  // this thread's waits
   int failed = 0;  // some thread's wait ran out (the same in all threads)
 
+  publish_ru(1);
   for (int it = 1;; it++) {
-    if (it > 1 && tid == NT - 1) pcg_reciprocals(ss);
+    if (it > 1 && tid >= NT - 2) recip[NT - 1 - tid] = 1.0 / (tid == NT - 1 ? ss.gamma : ss.alpha);
     RowSums<T> acc;
     if constexpr (kF32) {
-      // the row's tail needs no u: its loads go ahead of the gathers, and all
-      // of the tail's and the first blocks' gathers before their uses
-      T tail[kTail][9];
+      // the tail's gathers go out with the last of the shared blocks'
       Gather gt[kTail];
-#pragma unroll
-      for (int q = 0; q < kTail; q++)
-#pragma unroll
-        for (int e = 0; e < 9; e++)
-          tail[q][e] = rows + q < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * (rows + q) + kSlice * e]) : T(0);
       const int nsm = min(lenMax, rows);
       for (int j = 0; j < nsm; j += kQ) {
         Gather g[kQ];
@@ -344,10 +400,11 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     if (inc1 > inc0) {
       // contact: an incidence per thread, then every vertex adds its own in order
       double cr[3] = {0.0, 0.0, 0.0};
-      for (int base = inc0; base < inc1; base += NT) {
-        if (base + tid < inc1) {
+      const int chunk = min(NT, scratch / 4);
+      for (int base = inc0; base < inc1; base += chunk) {
+        if (tid < chunk && base + tid < inc1) {
           double t[3];
-          collision_incidence<T>(
+          area[4 * tid + 3] = collision_incidence<T>(
               b.coll, base + tid,
               [&](int id, T (&x)[3]) {
                 Gather g;
@@ -356,105 +413,74 @@ __global__ void __launch_bounds__(kGridThreads, 1)
               },
               t);
 #pragma unroll
-          for (int i = 0; i < 3; i++) area[3 * tid + i] = t[i];
+          for (int i = 0; i < 3; i++) area[4 * tid + i] = t[i];
         }
         __syncthreads();
-        for (int k = max(my0, base); k < min(my1, base + NT); k++)
+        for (int k = max(my0, base); k < min(my1, base + chunk); k++)
 #pragma unroll
-          for (int i = 0; i < 3; i++) cr[i] = __dadd_rn(cr[i], area[3 * (k - base) + i]);
+          for (int i = 0; i < 3; i++) cr[i] = fma(area[4 * (k - base) + 3], area[4 * (k - base) + i], cr[i]);
         __syncthreads();
       }
       if (my1 > my0)
 #pragma unroll
         for (int i = 0; i < 3; i++) w[i] += T(__dmul_rn(cr[i], collScale));
     }
-    // ---- |r|^2, (r, u), (w, u): tile sums, exchanged ----
-    T t0 = T(0), t1 = T(0), t2 = T(0);
-    if (valid) {
-      t2 = dot3v(w[0], w[1], w[2], un[0], un[1], un[2]);
-      t1 = dot3v(r[0], r[1], r[2], un[0], un[1], un[2]);
-      t0 = dot3v(r[0], r[1], r[2], r[0], r[1], r[2]);
-    }
-    double mine = 0.0;   // tile or group sum this thread publishes
-    int pub = -1;        // its partial (index in the scene), component pubC
-    int pubC = 0;
+    // ---- (w, u): tile sums, exchanged ----
     if constexpr (kF32) {
+      T t2 = valid ? dot3v(w[0], w[1], w[2], un[0], un[1], un[2]) : T(0);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        t0 += __shfl_xor_sync(0xffffffffu, t0, o);
-        t1 += __shfl_xor_sync(0xffffffffu, t1, o);
-        t2 += __shfl_xor_sync(0xffffffffu, t2, o);
-      }
-      if (tid % 32 == 0) {
-        warpSum[3 * (tid / 32)] = t0;
-        warpSum[3 * (tid / 32) + 1] = t1;
-        warpSum[3 * (tid / 32) + 2] = t2;
-      }
+      for (int o = 16; o > 0; o >>= 1) t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+      if (tid % 32 == 0) warpSum[2][tid / 32] = t2;
       if ((failed = __syncthreads_or(!ok))) break;
-      auto tile = [&](int t, int c) {  // block_sum3's order over the tile's warps
-        T a = T(0);
-#pragma unroll
-        for (int i = 0; i < TV / 32; i++) a += warpSum[3 * (t * (TV / 32) + i) + c];
-        return double(a);
-      };
-      if (whole && tid < 3) {
-        mine = group_sum<TV>([&](int t) { return tile(t, tid); });
-        pub = cta.y / kG;
-        pubC = tid;
-      } else if (!whole && tid < 3 * tpc && cta.y + tid / 3 < ntiles) {
-        mine = tile(tid / 3, tid % 3);
-        pub = cta.y + tid / 3;
-        pubC = tid % 3;
-      }
+      publish32(2, 1, it);
     } else {
-      area[tid] = t0;
-      area[NT + tid] = t1;
-      area[2 * NT + tid] = t2;
+#pragma unroll
+      for (int i = 0; i < 3; i++) area[6 * NT + 3 * tid + i] = valid ? w[i] * un[i] : 0.0;
       __syncthreads();
-      // a warp per (component, tile); a group's four sums meet in shared memory
-      for (int k = tid / 32; k < 3 * tpc; k += NT / 32) {
-        const double t = tile_sum64<TV>(reinterpret_cast<double*>(area) + (k / tpc) * NT + (k % tpc) * TV);
-        if (tid % 32 == 0) tileSum[k] = t;
-      }
-      __syncthreads();
-      if (whole && tid < 3) {
-        mine = group_sum<TV>([&](int t) { return tileSum[tid * tpc + t]; });
-        pub = cta.y / kG;
-        pubC = tid;
-      } else if (!whole && tid < 3 * tpc && cta.y + tid % tpc < ntiles) {
-        mine = tileSum[tid];
-        pub = cta.y + tid % tpc;
-        pubC = tid / tpc;
-      }
+      publish64(2, 1, it);
     }
-    ulonglong2* words = reinterpret_cast<ulonglong2*>(b.gridPartials) +
-                        3 * ((it & 1) * (size_t)b.gridTilesCap + sp.tile0);
-    if (pub >= 0) st_word(words + 3 * (size_t)pub + pubC, mine, (unsigned long long)it);
-    for (int i = tid; i < 3 * nParts; i += NT) {
-      double value;
-      unsigned long long tag;
-      for (int n = 0;; n++) {
-        ld_word(words + i, value, tag);
-        if (tag == (unsigned long long)it || !ok) break;
-        if (n > kSpinLimit) ok = false;
+    const ulonglong2* in = words(it);
+    for (int i0 = tid; i0 < 3 * nParts; i0 += 4 * NT) {
+      double value[4];
+      unsigned long long tag[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (i0 + k * NT < 3 * nParts) ld_word(in + i0 + k * NT, value[k], tag[k]);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int i = i0 + k * NT;
+        if (i >= 3 * nParts) break;
+        for (int n = 0; tag[k] != (unsigned long long)it && ok; n++) {
+          if (n > kSpinLimit) ok = false;
+          ld_word(in + i, value[k], tag[k]);
+        }
+        area[(i % 3) * nParts + i / 3] = value[k];
       }
-      area[(i % 3) * nParts + i / 3] = value;
     }
     failed = __syncthreads_or(!ok);
-    for (int c = tid / 32; c < 3; c += NT / 32) {
-      const double* q = area + c * nParts;
-      const double t = whole ? scene_sum(nGroups, [&](int g) { return q[g]; }) : scene_sum(nGroups, [&](int g) {
-        return group_sum<TV>([&](int i) { return g * kG + i < ntiles ? q[g * kG + i] : 0.0; });
-      });
-      if (tid % 32 == 0) sums[c] = t;
+    const int nTrees = scene_trees<TV>(ntiles);
+    if constexpr (kF32) {
+      for (int c = tid / 32; c < 3; c += NT / 32) {
+        const double* q = area + c * nParts;
+        const double t = whole ? scene_sum(nGroups, [&](int g) { return q[g]; }) : scene_sum(nGroups, [&](int g) {
+          return group_sum<TV>([&](int i) { return g * kG + i < ntiles ? q[g * kG + i] : 0.0; });
+        });
+        if (tid % 32 == 0) sums[c] = t;
+      }
+    } else {
+      scene_tree32<TV>(ntiles, [&](int c, int i) { return area[c * nParts + i]; }, trees);
     }
     T M[9];
     if (valid)
 #pragma unroll
       for (int e = 0; e < 9; e++) M[e] = v.minv[9 * (size_t)u + e];
     __syncthreads();
+    if (!kF32 && tid < 3) {
+      sums[tid] = chain(trees + tid * nTrees, nTrees);
+      __syncwarp(7u);
+    }
     if (tid == 0) {
-      stop = pcg_decide<T>(ss, sums[0], sums[1], sums[2]) ? 1 : 0;
+      stop = pcg_decide<T>(ss, sums[0], sums[1], sums[2], recip[0], recip[1]) ? 1 : 0;
       if constexpr (kF32) {
         sAlpha = ss.alphaF;
         sBeta = ss.betaF;
@@ -482,6 +508,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
       __syncthreads();
       if (tid == 0) st_flag(flags + cta.y, it + 1);  // after the barrier: covers the whole CTA's u
     }
+    publish_ru(it + 1);
 #pragma unroll
     for (int i = 0; i < 3; i++) d[i] = d[i] + alpha * p[i];
   }
@@ -537,7 +564,8 @@ GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, int longestRow, bool 
     const int threads = tpc * tileV;
     g.ctas = (int)ctas;
     g.tpc = tpc;
-    g.scratch = (3 * std::max(most, threads) + 1) / 2 * 2;
+    // the partials of a scene; in FP64 the row products, nine a thread
+    g.scratch = (3 * std::max(most, (mixed ? 1 : 3) * threads) + 1) / 2 * 2;
     const size_t row = (size_t)threads * (9 * (mixed ? sizeof(float) : sizeof(double)) + sizeof(int));
     int rows = (int)std::min<size_t>(longestRow, (kGridSmemMax - sizeof(double) * g.scratch) / row);
     if (!mixed) rows = longestRow % 2 && rows == longestRow && (rows + 1) * row + sizeof(double) * g.scratch <= kGridSmemMax

@@ -617,7 +617,6 @@ __device__ __forceinline__ void spmv_decide(const DeviceBatch& b, SolveState& st
                                             double delta) {
   if (st.innerThreshold < 0.0) return;
   if (pcg_decide<T>(st, rho, gamma, delta)) atomicSub(b.active, 1);
-  else pcg_reciprocals(st);
 }
 
 // FP64: w = A u, one thread per scalar row (9 DFMA per block over the row's
@@ -626,7 +625,7 @@ __device__ __forceinline__ void spmv_decide(const DeviceBatch& b, SolveState& st
 // (10 vertices) read three lines per load.
 template <int TV, typename T>
 __device__ __forceinline__ void spmv_tile_rows(const DeviceBatch& b, const PcgVecs<T>& v, int tile, double* sh,
-                                               T* rows, int* flag) {
+                                               double* vals, int* flag) {
   // before the dependency wait: what the previous kernel does not write
   const int s = b.tileScene[tile];
   const int row = 3 * b.tileV0[tile] + threadIdx.x;
@@ -671,49 +670,36 @@ __device__ __forceinline__ void spmv_tile_rows(const DeviceBatch& b, const PcgVe
         }
       }
     }
-    rows[threadIdx.x] = acc0 + acc1;
-  }
-  __syncthreads();
-  // per vertex from here on (the order of every PCG path): contact rows, w
-  // and the three dot products
-  const int vt = b.tileV0[tile] + threadIdx.x;
-  if (threadIdx.x < TV && vt < b.tileV1[tile]) {
-    const T* __restrict__ uu = v.u;
-    T a0 = rows[3 * threadIdx.x], a1 = rows[3 * threadIdx.x + 1], a2 = rows[3 * threadIdx.x + 2];
-    if (b.collOn && b.freeMask[vt]) {
+    T acc = acc0 + acc1;
+    if (b.collOn && b.freeMask[u]) {
       double cr[3];
-      collision_rows<T>(b, vt, [&](int id, T* x) { x[0] = uu[3 * id], x[1] = uu[3 * id + 1], x[2] = uu[3 * id + 2]; },
-                        cr);
-      a0 += T(cr[0]);
-      a1 += T(cr[1]);
-      a2 += T(cr[2]);
+      collision_rows<T>(
+          b, u, [&](int id, T (&x)[3]) { x[0] = uu[3 * id], x[1] = uu[3 * id + 1], x[2] = uu[3 * id + 2]; }, cr);
+      acc += T(i == 0 ? cr[0] : i == 1 ? cr[1] : cr[2]);
     }
-    v.w[3 * vt] = a0;
-    v.w[3 * vt + 1] = a1;
-    v.w[3 * vt + 2] = a2;
-    const T u0 = uu[3 * vt], u1 = uu[3 * vt + 1], u2 = uu[3 * vt + 2];
-    const T r0 = r[3 * vt], r1 = r[3 * vt + 1], r2 = r[3 * vt + 2];
-    dl = dot3v(a0, a1, a2, u0, u1, u2);
-    gl = dot3v(r0, r1, r2, u0, u1, u2);
-    rl = dot3v(r0, r1, r2, r0, r1, r2);
+    v.w[row] = acc;
+    const T ui = uu[row], ri = r[row];
+    dl = acc * ui;
+    gl = ri * ui;
+    rl = ri * ri;
   }
+  constexpr int NT = 3 * TV, kTrees = NT / 32;
+  vals[threadIdx.x] = rl;
+  vals[NT + threadIdx.x] = gl;
+  vals[2 * NT + threadIdx.x] = dl;
   __syncthreads();
-  if (threadIdx.x < TV) {  // 3 * TV values, component by component
-    rows[threadIdx.x] = rl;
-    rows[TV + threadIdx.x] = gl;
-    rows[2 * TV + threadIdx.x] = dl;
-  }
+  tree32(3 * kTrees, [&](int g, int l) { return vals[32 * g + l]; }, sh);
   __syncthreads();
-  if (threadIdx.x < 96) {
-    const double t = tile_sum64<TV>(rows + TV * (threadIdx.x / 32));
-    if (threadIdx.x % 32 == 0) b.partial[kPartials * tile + threadIdx.x / 32] = t;
-  }
+  if (threadIdx.x < 3) b.partial[kPartials * tile + threadIdx.x] = chain(sh + kTrees * threadIdx.x, kTrees);
   __syncthreads();  // last_tile's fence by thread 0 covers the three writers
   const SceneParams& sp = b.scenes[s];
   if (!last_tile(&st.ticketA, sp.ntiles, flag)) return;
-  double tot[3];
-  scene_sums<3 * TV, TV>(b.partial, sp.tile0, sp.ntiles, sh, tot);
-  if (threadIdx.x == 0) spmv_decide<T>(b, st, tot[0], tot[1], tot[2]);
+  const int n = sp.ntiles, trees = scene_trees<TV>(n);
+  const double* part = b.partial + (size_t)kPartials * sp.tile0;
+  scene_tree32<TV>(n, [&](int c, int i) { return __ldcg(&part[kPartials * (size_t)i + c]); }, sh);
+  __syncthreads();
+  if (threadIdx.x == 0)
+    spmv_decide<T>(b, st, chain(sh, trees), chain(sh + trees, trees), chain(sh + 2 * trees, trees));
 }
 
 // FP32: w = A u, one thread per vertex (its three rows; 9 FMA per block), and
@@ -781,8 +767,8 @@ __device__ __forceinline__ void spmv_tile(const DeviceBatch& b, const PcgVecs<T>
     }
     if (b.collOn && b.freeMask[u]) {
       double cr[3];
-      collision_rows<T>(b, u, [&](int id, T* x) { x[0] = uu[3 * id], x[1] = uu[3 * id + 1], x[2] = uu[3 * id + 2]; },
-                        cr);
+      collision_rows<T>(
+          b, u, [&](int id, T (&x)[3]) { x[0] = uu[3 * id], x[1] = uu[3 * id + 1], x[2] = uu[3 * id + 2]; }, cr);
       a0 += T(cr[0]);
       a1 += T(cr[1]);
       a2 += T(cr[2]);
@@ -831,8 +817,8 @@ __global__ void __launch_bounds__(spmv_threads<T>(TV)) k_spmv(DeviceBatch b, Pcg
   if constexpr (sizeof(T) == sizeof(float)) {
     spmv_tile<TV, T>(b, v, tile, sh, &flag);
   } else {
-    __shared__ T rows[3 * TV];
-    spmv_tile_rows<TV, T>(b, v, tile, sh, rows, &flag);
+    __shared__ double vals[9 * TV];
+    spmv_tile_rows<TV, T>(b, v, tile, sh, vals, &flag);
   }
 }
 
@@ -997,8 +983,8 @@ __global__ void __launch_bounds__(3 * TV) k_residual(DeviceBatch b) {
     if (b.collOn && b.freeMask[u]) {
       double cr[3];
       collision_rows<double>(
-          b, u, [&](int id, double* x) { x[0] = b.y[3 * id], x[1] = b.y[3 * id + 1], x[2] = b.y[3 * id + 2]; }, cr);
-      acc += cr[i];
+          b, u, [&](int id, double (&x)[3]) { x[0] = b.y[3 * id], x[1] = b.y[3 * id + 1], x[2] = b.y[3 * id + 2]; }, cr);
+      acc += i == 0 ? cr[0] : i == 1 ? cr[1] : cr[2];
     }
     const double ri = b.rhs[row] - acc;
     b.r64[row] = ri;
