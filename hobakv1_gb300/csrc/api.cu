@@ -292,9 +292,10 @@ int alloc_precision(hobak_batch_t* B) {
   Arena A;
   const size_t oEH = A.reserve(w * kElemHessStride * nt);
   const size_t oLhs = A.reserve(w * vals);
-  const size_t oMinv = A.reserve(w * 9 * nv);
+  const size_t oMinv = A.reserve(w * kSlotVals * ((nv + kSlice - 1) / kSlice));
   size_t oVec[6];
   for (int k = 0; k < (mixed ? 6 : 4); k++) oVec[k] = A.reserve(w * 3 * nv);
+  const size_t oHalo = mixed ? A.reserve(sizeof(int) * 4 * nv) : 0;  // one-launch PCG
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, A.used);
   if (e != cudaSuccess)
@@ -318,6 +319,7 @@ int alloc_precision(hobak_batch_t* B) {
                             carve<double>(base, oVec[0]), carve<double>(base, oVec[1]), carve<double>(base, oVec[2]),
                             carve<double>(base, oVec[3]), d.y};
   }
+  d.gridHalo = mixed ? carve<int>(base, oHalo) : nullptr;
   B->precMixed = mixed;
   B->gridDirty = true;
   return HOBAK_OK;
@@ -576,6 +578,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   const size_t oPsi = A.reserve(sizeof(double) * nt);
   const size_t oGridP = A.reserve(96 * (size_t)ntilesCap), oGridF = A.reserve(sizeof(int) * ntilesCap);
   const size_t oGridL = A.reserve(sizeof(int2) * ntilesCap);
+  const size_t oGridHc = A.reserve(sizeof(int) * (ntilesCap + 1));
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, A.used);
   if (e != cudaSuccess)
@@ -651,6 +654,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   d.gridFlags = carve<int>(base, oGridF);
   d.gridTilesCap = ntilesCap;
   B->gridList = carve<int2>(base, oGridL);
+  d.gridHaloCount = carve<int>(base, oGridHc);
   d.anyAniso = anyAniso;
   d.anyArap = anyArap;
   d.anySvdFree = anySvdFree;
@@ -895,8 +899,8 @@ int prepare_grid_plan(hobak_batch_t* B) {
   const int n = (int)B->scenes.size();
   std::vector<int> tiles(n);
   for (int s = 0; s < n; s++) tiles[s] = B->sceneParams[s].pcgCluster ? 0 : B->sceneParams[s].ntiles;
-  GridPlan g = plan_grid_pcg(tiles.data(), n, B->d.tileV, B->longestRow,
-                             B->opts.precision == HOBAK_PRECISION_MIXED, sms);
+  const bool mixed = B->opts.precision == HOBAK_PRECISION_MIXED;
+  GridPlan g = plan_grid_pcg(tiles.data(), n, B->d.tileV, mixed, sms);
   if (g.ctas) {
     std::vector<int2> list;
     for (int s = 0; s < n; s++)
@@ -904,9 +908,18 @@ int prepare_grid_plan(hobak_batch_t* B) {
     CUDA_TRY(cudaStreamSynchronize(B->stream));
     CUDA_TRY(cudaMemcpy(B->gridList, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice));
     g.list = B->gridList;
+    if (mixed) {
+      int* largest = B->d.gridHaloCount + B->d.gridTilesCap;
+      CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(int), B->stream));
+      launch_grid_halo(B->d, g, largest, B->stream);
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaMemcpyAsync(&g.halo, largest, sizeof(int), cudaMemcpyDeviceToHost, B->stream));
+      CUDA_TRY(cudaStreamSynchronize(B->stream));
+    }
+    plan_grid_smem(g, B->d.tileV, B->longestRow, mixed);
   }
   if (g.ctas != B->grid.ctas || g.tpc != B->grid.tpc || g.rows != B->grid.rows || g.smem != B->grid.smem ||
-      g.scratch != B->grid.scratch)
+      g.scratch != B->grid.scratch || g.halo != B->grid.halo)
     drop_graphs(B);
   B->grid = g;
   B->d.gridOn = g.ctas ? 1 : 0;

@@ -406,10 +406,10 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
         m.s[3 * lv + i] = T(0);
         rr += r3[i] * r3[i];
       }
-      const T* M = v.minv + 9 * (size_t)u;
+      const T* M = v.minv + minv_slot(u);
 #pragma unroll
       for (int i = 0; i < 3; i++) {
-        const T ui = M[3 * i] * r3[0] + M[3 * i + 1] * r3[1] + M[3 * i + 2] * r3[2];
+        const T ui = M[kSlice * (3 * i)] * r3[0] + M[kSlice * (3 * i + 1)] * r3[1] + M[kSlice * (3 * i + 2)] * r3[2];
         m.u[4 * lv + i] = ui;
         ru += r3[i] * ui;
       }
@@ -539,9 +539,11 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
           r3[i] = m.r[j] - ta * sv;
           m.r[j] = r3[i];
         }
-        const T* M = v.minv + 9 * (size_t)u;
+        const T* M = v.minv + minv_slot(u);
   #pragma unroll
-        for (int i = 0; i < 3; i++) m.u[4 * lv + i] = M[3 * i] * r3[0] + M[3 * i + 1] * r3[1] + M[3 * i + 2] * r3[2];
+        for (int i = 0; i < 3; i++)
+          m.u[4 * lv + i] =
+              M[kSlice * (3 * i)] * r3[0] + M[kSlice * (3 * i + 1)] * r3[1] + M[kSlice * (3 * i + 2)] * r3[2];
       }
       // the new u reaches the other CTAs' SpMV
       cluster.sync();

@@ -11,7 +11,7 @@ namespace hobak {
 template <typename T>
 struct PcgVecs {
   T* lhs;   // [B][9] row major
-  T* minv;  // [V][9] row major
+  T* minv;  // 3x3 blocks, row major, in the slices of the LHS (minv_slot)
   T* r;     // residual of the inner solve
   T* u;     // preconditioned residual
   T* p;     // search direction
@@ -43,6 +43,7 @@ struct GridPlan {
   int ctas, tpc;     // CTAs, tiles per CTA (one scene per CTA)
   int rows;          // blocks of every matrix row kept in shared memory
   int scratch;       // doubles of its exchange area
+  int halo;          // FP32: most other vertices a CTA reads
   size_t smem;       // dynamic shared memory of a CTA
   const int2* list;  // device: per CTA its scene and its first tile in the scene
 };
@@ -162,6 +163,12 @@ struct DeviceBatch {
   int* gridFlags;
   int gridTilesCap;
   int gridOn;  // the tile-path scenes take that path
+  // FP32: per CTA the vertices of other CTAs that its rows' columns name (at
+  // 4 x its first vertex), their number (per tile: a CTA's is its first
+  // tile's), and every column as the CTA's own index of it (k_grid_halo; the
+  // slots of clusterGather, which only cluster scenes use otherwise)
+  int* gridHalo;
+  int* gridHaloCount;
   double* psi;          // [T] energy density scratch
   int anyAniso;          // some scene has an anisotropic energy (k_element_aniso)
   int anyArap, anySvdFree;  // some scene has ARAP / another isotropic energy (mixed element kernels)
@@ -178,6 +185,11 @@ __device__ __forceinline__ size_t lhs_slot(const DeviceBatch& b, int u, int j) {
 }
 __device__ __forceinline__ size_t col_slot(const DeviceBatch& b, int u, int j) {
   return (size_t)(b.sliceRow[u >> 5] + j) * kSlice + (u & (kSlice - 1));
+}
+
+// Offset of entry 0 of vertex u's preconditioner block (entry e at + kSlice * e).
+__device__ __forceinline__ size_t minv_slot(int u) {
+  return (size_t)(u >> 5) * kSlotVals + (u & (kSlice - 1));
 }
 
 // Weight of the collision Hessian H_coll in the step's matrix A, with
@@ -266,7 +278,10 @@ void launch_element_eval(int nt, const int4* tets, const double* rest, const dou
 template <typename T>
 int launch_cluster_pcg(const DeviceBatch& b, const PcgVecs<T>& v, const ClusterClass* classes, int k,
                        cudaStream_t s);
-GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, int longestRow, bool mixed, int sms);
+GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, bool mixed, int sms);
+void plan_grid_smem(GridPlan& g, int tileV, int longestRow, bool mixed);
+// FP32: the halo lists of a plan's CTAs (largest: a device word)
+void launch_grid_halo(const DeviceBatch& b, const GridPlan& g, int* largest, cudaStream_t s);
 int configure_grid_pcg();
 // Every iteration of the inner solves that launch_inner_init has started, for
 // all scenes of the plan.  Returns a cudaError_t value (0 on success).

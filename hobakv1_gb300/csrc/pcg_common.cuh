@@ -134,13 +134,19 @@ __device__ __forceinline__ void tree32_warp(int g0, int n, Get get, double* out)
 // ... of all n groups by the CTA's warps
 template <typename Get>
 __device__ __forceinline__ void tree32(int n, Get get, double* out) {
+#pragma unroll 1
   for (int g0 = 8 * (threadIdx.x / 32); g0 < n; g0 += 8 * (blockDim.x / 32)) tree32_warp(g0, n, get, out);
 }
 
-// Sum of n values in order.
+// Sum of n <= 12 values in order, their loads ahead of the adds.
 __device__ __forceinline__ double chain(const double* v, int n) {
-  double t = v[0];
-  for (int i = 1; i < n; i++) t += v[i];
+  double x[12];
+#pragma unroll
+  for (int i = 0; i < 12; i++) x[i] = i < n ? v[i] : 0.0;
+  double t = x[0];
+#pragma unroll
+  for (int i = 1; i < 12; i++)
+    if (i < n) t += x[i];
   return t;
 }
 
@@ -151,20 +157,20 @@ template <int TV>
 __device__ __forceinline__ int scene_trees(int n) {
   return n < 3 * TV ? (n + 31) / 32 : 3 * TV / 32;
 }
+// lanes: 9 TV doubles of shared memory.  All threads of the CTA.
 template <int TV, typename Tile>
-__device__ __forceinline__ void scene_tree32(int n, Tile tile, double* out) {
-  const int trees = scene_trees<TV>(n), per = (trees + 7) / 8;
-  for (int k = threadIdx.x / 32; k < 3 * per; k += blockDim.x / 32) {
-    const int c = k >= 2 * per ? 2 : k >= per ? 1 : 0;
-    tree32_warp(
-        8 * (k - c * per), trees,
-        [&](int g, int l) {
-          double s = 32 * g + l < n ? tile(c, 32 * g + l) : 0.0;
-          for (int i = 32 * g + l + 3 * TV; i < n; i += 3 * TV) s += tile(c, i);
-          return s;
-        },
-        out + trees * c);
+__device__ __forceinline__ void scene_tree32(int n, Tile tile, double* lanes, double* out) {
+  const int trees = scene_trees<TV>(n), width = 32 * trees;
+#pragma unroll 1
+  for (int k = threadIdx.x; k < 3 * width; k += blockDim.x) {
+    const int c = k >= 2 * width ? 2 : k >= width ? 1 : 0, l = k - c * width;
+    double s = l < n ? tile(c, l) : 0.0;
+#pragma unroll 1
+    for (int i = l + 3 * TV; i < n; i += 3 * TV) s += tile(c, i);
+    lanes[k] = s;
   }
+  __syncthreads();
+  tree32(3 * trees, [&](int g, int l) { return lanes[32 * g + l]; }, out);
 }
 
 // The sum of a group's tiles, get(i) its i-th (0 past the scene's last tile).
@@ -179,6 +185,7 @@ __device__ __forceinline__ double group_sum(Get get) {
 template <typename Group>
 __device__ __forceinline__ double scene_sum(int n, Group group) {
   double s = 0.0;
+#pragma unroll 1
   for (int g = threadIdx.x % 32; g < n; g += 32) s += group(g);
   return warp_tree(s);
 }
@@ -204,18 +211,17 @@ __device__ __forceinline__ void scene_sums(const double* partial, int tile0, int
 __device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
 // a / b, correctly rounded, from y = 1 / b correctly rounded (0: not given): a
-// quotient off by little and two of Markstein's corrections ("Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990), a chain
-// of five FMAs (320 cycles in one thread) where the division takes ~630.  Out
-// of the range where the residual is exact, the division.
+// quotient off by at most a few ulps and Markstein's correction ("Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990), a
+// chain of three FMAs (200 cycles in one thread) where the division takes
+// ~630.  Outside the range where the residual is exact, the division.
 __device__ __forceinline__ double divide(double a, double b, double y) {
   const auto plain = [](double x) {
     const int e = (__double2hiint(x) >> 20) & 0x7ff;
     return e > 523 && e < 1523;
   };
   if (!(plain(a) && plain(b) && plain(y))) return a / b;
-  double q = a * y;
-  q = fma(fma(-q, b, a), y, q);
+  const double q = a * y;
   return fma(fma(-q, b, a), y, q);
 }
 
@@ -262,8 +268,10 @@ __device__ __forceinline__ bool pcg_decide(SolveState& st, double rho, double ga
   }
   st.gammaOld = st.gamma;
   st.gamma = gamma;
-  st.alphaF = float(st.alpha);
-  st.betaF = float(st.beta);
+  if (sizeof(T) == sizeof(float)) {
+    st.alphaF = float(st.alpha);
+    st.betaF = float(st.beta);
+  }
   st.iters += 1;
   st.totalIters += 1;
   return false;
@@ -323,6 +331,7 @@ __device__ __forceinline__ void collision_rows(const DeviceBatch& b, int u, Load
   const int k0 = c.incCount[u], k1 = c.incCount[u + 1];
   out[0] = out[1] = out[2] = 0.0;
   if (k0 == k1) return;
+#pragma unroll 1
   for (int k = k0; k < k1; k++) {
     double t[3];
     const double w = collision_incidence<T>(c, k, load, t);

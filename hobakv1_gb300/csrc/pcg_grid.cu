@@ -8,13 +8,15 @@
 // one scene) for the whole solve, one per thread.  A vertex's u, p, s, d, r
 // stay in registers; the first blocks of its matrix row and their columns in
 // shared memory (as many as fit, the same count for every row), in FP32 the
-// next four in registers; the rest of the row comes from L2.  Per iteration the CTAs of a scene meet twice:
+// next six in registers; the rest of the row comes from L2.  Per iteration the CTAs of a scene meet twice:
 //   * the partial sums of the three dot products go out as 16-byte words
 //     {value, iteration}, |r|^2 and (r, u) before the SpMV, (w, u) after it, written and polled with
 //     single-copy-atomic 128-bit accesses, so a reader needs no flag and no
 //     fence; every CTA adds them in the same order and takes the same decision;
 //   * after the update the new u: in FP32 the same way, each vertex's u carries
-//     its iteration and a gather repeats until it fits; in FP64 (two words a
+//     its iteration; a CTA reads its halo (the other CTAs' vertices in its
+//     rows' columns, listed once) into shared memory, each vertex once and
+//     not up to 15 times, and a load repeats until the iteration fits; in FP64 (two words a
 //     vertex) a CTA releases a flag, and a CTA waits for the flags of the CTAs
 //     its rows' columns lie in (with contact: all of the scene's).
 // The partials' exchange also orders u's reuse: a CTA overwrites its u only
@@ -25,11 +27,14 @@
 //
 // What bounds it: in FP64 the SM's FP64 pipe, 19 cycles per warp instruction
 // (16 warps x 135 products of 512 vertices' rows are 41,000 of an iteration's
-// 70,000 cycles); in FP32 latency and the gathers (row sums 9,000 of 19,000
-// cycles, the two meetings and the scalars most of the rest).  68,921 vertices,
-// us an iteration: FP64 45.8 -> 34 (365 iterations: step 19.4 -> 14.4 ms),
-// FP32 17.0 -> 9.2 (383: 7.0 -> 4.4 ms); two cubes in contact, 31,250
-// vertices, FP64 56 -> 26; 1,331 vertices FP64 23 -> 15.
+// 65,000 cycles); in FP32 latency: the row sums from shared memory are 4,600 of
+// 16,200 cycles, the halo 1,700, the partials' exchange 2,100, the scalars
+// 3,600.  The phases between barriers run once an iteration on few warps, so
+// loops there are kept rolled: 108 KB of code cost 4,000 cycles more an
+// iteration in instruction fetches than 53 KB.  68,921 vertices, us an
+// iteration: FP64 45.8 -> 31.3 (365 iterations: step 19.9 -> 13.7 ms), FP32
+// 17.0 -> 7.9 (383: 7.2 -> 3.8 ms); two cubes in contact, 31,250 vertices,
+// FP64 56 -> 25; 1,331 vertices FP64 23 -> 15.
 //
 // Every wait is bounded; a wait that runs out ends the CTA's part, and the
 // scene's solve is marked failed.  All CTAs are resident (cooperative launch,
@@ -47,6 +52,7 @@ constexpr int kGridThreads = 512;      // vertices of a CTA, at most (128 regist
 constexpr int kGridSmemMax = 224 * 1024;
 constexpr int kSpinLimit = 1 << 21;    // polls of one wait (about a second), then the solve fails
 constexpr int kMaxCtas = 256;          // CTAs of a launch, at most (one per SM)
+constexpr int kHaloMax = 3072;         // halo vertices of a CTA, at most (48 KB of shared memory)
 
 __device__ __forceinline__ void st_word(ulonglong2* p, double value, unsigned long long tag) {
   asm volatile(
@@ -83,6 +89,7 @@ struct Gather32 {
   // repeats the load of vertex() until it fits; clears ok when it does not
   template <typename Vertex>
   __device__ __forceinline__ void get(const float* u4, Vertex vertex, int it, float (&x)[3], bool& ok) {
+#pragma unroll 1
     for (int n = 0; (int)(hi >> 32) != it && ok; n++) {
       if (n > kSpinLimit) ok = false;
       load(u4, vertex());
@@ -149,10 +156,10 @@ struct RowSums {
 // scratch: doubles of the exchange area.
 template <int TV, typename T>
 __global__ void __launch_bounds__(kGridThreads, 1)
-    k_pcg_grid(DeviceBatch b, PcgVecs<T> v, const int2* __restrict__ ctas, int tpc, int rows, int scratch) {
+    k_pcg_grid(DeviceBatch b, PcgVecs<T> v, const int2* __restrict__ ctas, int tpc, int rows, int scratch, int halo) {
   constexpr bool kF32 = sizeof(T) == sizeof(float);
-  constexpr int kTail = 4;  // FP32: row blocks past the shared ones, in registers
-  constexpr int kQ = kF32 ? 6 : 2;
+  constexpr int kTail = 6;  // FP32: row blocks past the shared ones, in registers
+  constexpr int kQ = 2;     // FP64: blocks per trip
   constexpr int kG = kGroupVerts / TV;
   using Gather = typename GatherOf<T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -178,7 +185,8 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   const int own = valid ? u : v0;  // a vertex that any gather may read
 
   double* area = reinterpret_cast<double*>(smem);
-  T* mat = reinterpret_cast<T*>(area + scratch);
+  float4* us = reinterpret_cast<float4*>(area + scratch);  // FP32: u of the CTA's and of its halo's vertices
+  T* mat = reinterpret_cast<T*>(us + (kF32 ? NT + halo : 0));
   int* col = reinterpret_cast<int*>(mat + (size_t)9 * rows * NT);  // both [entry][thread]
 
   if (tid == 0) {
@@ -194,6 +202,8 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   T* u4 = v.p;  // p and s live in registers here: their buffers hold the shared u
   int len = 0;
   size_t lb = 0, cb = 0;
+  const int* cols = kF32 ? b.clusterGather : b.colS;  // FP32: indices into us
+  const int self = kF32 ? tid : own;
   T un[3], p[3], sv[3], d[3], r[3];
 #pragma unroll
   for (int i = 0; i < 3; i++) un[i] = p[i] = sv[i] = d[i] = r[i] = T(0);
@@ -203,6 +213,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     lb = lhs_slot(b, u, 0);
     cb = col_slot(b, u, 0);
     if (!kF32)
+#pragma unroll 1
       for (int j = 0; j < len; j++) {
         const int c = (__ldg(&b.colS[cb + kSlice * j]) - v0) / ctaVerts;
         if (!((nbrBits[c / 32] >> (c % 32)) & 1u)) atomicOr(&nbrBits[c / 32], 1u << (c % 32));
@@ -213,8 +224,9 @@ __global__ void __launch_bounds__(kGridThreads, 1)
       r[i] = rsrc[3 * u + i];
     }
   }
+#pragma unroll 1
   for (int j = 0; j < rows; j++) {  // zeros past the row's end
-    col[(size_t)j * NT + tid] = j < len ? __ldg(&b.colS[cb + kSlice * j]) : own;
+    col[(size_t)j * NT + tid] = j < len ? __ldg(&cols[cb + kSlice * j]) : self;
 #pragma unroll
     for (int e = 0; e < 9; e++)
       mat[((size_t)9 * j + e) * NT + tid] = j < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * j + kSlice * e]) : T(0);
@@ -224,13 +236,14 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   if constexpr (kF32)
 #pragma unroll
     for (int q = 0; q < kTail; q++) {
-      tailCol[q] = rows + q < len ? __ldg(&b.colS[cb + kSlice * (rows + q)]) : own;
+      tailCol[q] = rows + q < len ? __ldg(&cols[cb + kSlice * (rows + q)]) : self;
 #pragma unroll
       for (int e = 0; e < 9; e++)
         tail[q][e] = rows + q < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * (rows + q) + kSlice * e]) : T(0);
     }
   __syncthreads();
   if (!kF32)
+#pragma unroll 1
     for (int c = tid; c < nCta; c += NT)
       if ((b.collOn || ((nbrBits[c / 32] >> (c % 32)) & 1u)) && c != cta.y / tpc) nbr[atomicAdd(&nNbr, 1)] = c;
   // the CTA's contact incidences (CSR by vertex, its vertices are consecutive)
@@ -249,6 +262,9 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   const int lenMax = __reduce_max_sync(0xffffffffu, len);
   __syncthreads();
   int* flags = b.gridFlags + sp.tile0;  // a CTA's flag: that of its first tile
+  const int* haloList = b.gridHalo + 4 * (size_t)b.tileV0[sp.tile0 + cta.y];
+  const int nHalo = kF32 ? b.gridHaloCount[sp.tile0 + cta.y] : 0;
+  if constexpr (kF32) us[tid] = make_float4(un[0], un[1], un[2], 0.f);
   const bool whole = kF32 && tpc == kG;  // partials: one per group, else one per tile
   const int nGroups = (ntiles + kG - 1) / kG, nParts = whole ? nGroups : ntiles;
   constexpr int kTrees = 3 * TV / 32;  // FP64: trees of a tile's rows
@@ -308,54 +324,70 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   };
   bool ok = true;  // this thread's waits
   int failed = 0;  // some thread's wait ran out (the same in all threads)
+  T alpha = T(0);
 
-  publish_ru(1);
+#pragma unroll 1
   for (int it = 1;; it++) {
-    if (it > 1 && tid >= NT - 2) recip[NT - 1 - tid] = 1.0 / (tid == NT - 1 ? ss.gamma : ss.alpha);
+    publish_ru(it);
+    auto reciprocals = [&] {
+      if (it > 1 && tid >= NT - 2) recip[NT - 1 - tid] = 1.0 / (tid == NT - 1 ? ss.gamma : ss.alpha);
+    };
     RowSums<T> acc;
     if constexpr (kF32) {
-      // the tail's gathers go out with the last of the shared blocks'
-      Gather gt[kTail];
+      // the halo's u to shared memory, four loads in flight
+#pragma unroll 1
+      for (int i0 = tid; i0 < nHalo; i0 += 4 * NT) {
+        Gather g[4];
+        int w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (i0 + k * NT < nHalo) g[k].load(u4, w[k] = __ldg(&haloList[i0 + k * NT]));
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (i0 + k * NT >= nHalo) break;
+          T x[3];
+          g[k].get(u4, [&] { return w[k]; }, it, x, ok);
+          us[NT + i0 + k * NT] = make_float4(x[0], x[1], x[2], 0.f);
+        }
+      }
+      reciprocals();
+      if ((failed = __syncthreads_or(!ok))) break;
+      auto vec = [&](int c, float (&x)[3]) {
+        const float4 t = us[c];
+        x[0] = t.x, x[1] = t.y, x[2] = t.z;
+      };
       const int nsm = min(lenMax, rows);
-      for (int j = 0; j < nsm; j += kQ) {
-        Gather g[kQ];
+#pragma unroll 3
+      for (int j = 0; j < nsm; j++) {
+        T x[3], m[9];
+        vec(col[(size_t)j * NT + tid], x);
 #pragma unroll
-        for (int q = 0; q < kQ; q++) g[q].load(u4, j + q < nsm ? col[(size_t)(j + q) * NT + tid] : own);
-        if (j + kQ >= nsm && lenMax > rows)
-#pragma unroll
-          for (int q = 0; q < kTail; q++) gt[q].load(u4, tailCol[q]);
-#pragma unroll
-        for (int q = 0; q < kQ; q++)
-          if (j + q < nsm) {
-            T x[3], m[9];
-            g[q].get(u4, [&] { return col[(size_t)(j + q) * NT + tid]; }, it, x, ok);
-#pragma unroll
-            for (int e = 0; e < 9; e++) m[e] = mat[((size_t)9 * (j + q) + e) * NT + tid];
-            acc.add(m, x, false);
-          }
+        for (int e = 0; e < 9; e++) m[e] = mat[((size_t)9 * j + e) * NT + tid];
+        acc.add(m, x, false);
       }
       if (lenMax > rows) {
 #pragma unroll
         for (int q = 0; q < kTail; q++) {
           T x[3];
-          gt[q].get(u4, [&] { return tailCol[q]; }, it, x, ok);
+          vec(tailCol[q], x);
           acc.add(tail[q], x, false);
         }
+#pragma unroll 1
         for (int j = rows + kTail; j < len; j++) {  // rows longer than the mesh's usual
           T m[9], x[3];
-          Gather g;
-          const int w = __ldg(&b.colS[cb + kSlice * j]);
-          g.load(u4, w);
 #pragma unroll
           for (int e = 0; e < 9; e++) m[e] = __ldg(&v.lhs[lb + (size_t)kSlotVals * j + kSlice * e]);
-          g.get(u4, [&] { return w; }, it, x, ok);
+          vec(__ldg(&cols[cb + kSlice * j]), x);
           acc.add(m, x, false);
         }
       }
     } else {
+      reciprocals();
+#pragma unroll 1
       for (int i = tid; i < nNbr; i += NT) {
         const int* f = flags + nbr[i] * tpc;
         int n = 0;
+#pragma unroll 1
         while (ld_flag(f) < it && ok)
           if (++n > kSpinLimit) ok = false;
       }
@@ -374,6 +406,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
         }
       };
       gather(0);
+#pragma unroll 1
       for (int j = 0; j < lenMax; j += kQ) {
         T m[kQ][9], x[kQ][3];
         if (j < rows) {
@@ -401,6 +434,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
       // contact: an incidence per thread, then every vertex adds its own in order
       double cr[3] = {0.0, 0.0, 0.0};
       const int chunk = min(NT, scratch / 4);
+#pragma unroll 1
       for (int base = inc0; base < inc1; base += chunk) {
         if (tid < chunk && base + tid < inc1) {
           double t[3];
@@ -416,6 +450,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
           for (int i = 0; i < 3; i++) area[4 * tid + i] = t[i];
         }
         __syncthreads();
+#pragma unroll 1
         for (int k = max(my0, base); k < min(my1, base + chunk); k++)
 #pragma unroll
           for (int i = 0; i < 3; i++) cr[i] = fma(area[4 * (k - base) + 3], area[4 * (k - base) + i], cr[i]);
@@ -439,7 +474,11 @@ __global__ void __launch_bounds__(kGridThreads, 1)
       __syncthreads();
       publish64(2, 1, it);
     }
+    if (it > 1)  // the last update's d, in the exchange's shadow
+#pragma unroll
+      for (int i = 0; i < 3; i++) d[i] = d[i] + alpha * p[i];
     const ulonglong2* in = words(it);
+#pragma unroll 1
     for (int i0 = tid; i0 < 3 * nParts; i0 += 4 * NT) {
       double value[4];
       unsigned long long tag[4];
@@ -450,6 +489,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
       for (int k = 0; k < 4; k++) {
         const int i = i0 + k * NT;
         if (i >= 3 * nParts) break;
+#pragma unroll 1
         for (int n = 0; tag[k] != (unsigned long long)it && ok; n++) {
           if (n > kSpinLimit) ok = false;
           ld_word(in + i, value[k], tag[k]);
@@ -460,6 +500,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     failed = __syncthreads_or(!ok);
     const int nTrees = scene_trees<TV>(ntiles);
     if constexpr (kF32) {
+#pragma unroll 1
       for (int c = tid / 32; c < 3; c += NT / 32) {
         const double* q = area + c * nParts;
         const double t = whole ? scene_sum(nGroups, [&](int g) { return q[g]; }) : scene_sum(nGroups, [&](int g) {
@@ -468,12 +509,12 @@ __global__ void __launch_bounds__(kGridThreads, 1)
         if (tid % 32 == 0) sums[c] = t;
       }
     } else {
-      scene_tree32<TV>(ntiles, [&](int c, int i) { return area[c * nParts + i]; }, trees);
+      scene_tree32<TV>(ntiles, [&](int c, int i) { return area[c * nParts + i]; }, area + 3 * nParts, trees);
     }
     T M[9];
-    if (valid)
+    if (kF32 && valid)
 #pragma unroll
-      for (int e = 0; e < 9; e++) M[e] = v.minv[9 * (size_t)u + e];
+      for (int e = 0; e < 9; e++) M[e] = v.minv[minv_slot(u) + kSlice * e];
     __syncthreads();
     if (!kF32 && tid < 3) {
       sums[tid] = chain(trees + tid * nTrees, nTrees);
@@ -492,8 +533,12 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     __syncthreads();
     if (stop || failed) break;
     // ---- p = u + beta p, s = w + beta s, d += alpha p, r -= alpha s, u = Minv r ----
-    const T alpha = sAlpha, beta = sBeta;
+    alpha = sAlpha;
+    const T beta = sBeta;
     if (valid) {
+      if (!kF32)  // (18 registers: not held across the scalars)
+#pragma unroll
+        for (int e = 0; e < 9; e++) M[e] = v.minv[minv_slot(u) + kSlice * e];
 #pragma unroll
       for (int i = 0; i < 3; i++) {
         p[i] = un[i] + beta * p[i];
@@ -503,14 +548,12 @@ __global__ void __launch_bounds__(kGridThreads, 1)
 #pragma unroll
       for (int i = 0; i < 3; i++) un[i] = M[3 * i] * r[0] + M[3 * i + 1] * r[1] + M[3 * i + 2] * r[2];
       publish_u(u4, u, un, it + 1);
+      if constexpr (kF32) us[tid] = make_float4(un[0], un[1], un[2], 0.f);
     }
     if (!kF32) {
       __syncthreads();
       if (tid == 0) st_flag(flags + cta.y, it + 1);  // after the barrier: covers the whole CTA's u
     }
-    publish_ru(it + 1);
-#pragma unroll
-    for (int i = 0; i < 3; i++) d[i] = d[i] + alpha * p[i];
   }
   if (valid)
 #pragma unroll
@@ -539,7 +582,7 @@ cudaError_t launch_tv(const DeviceBatch& b, const PcgVecs<T>& v, const GridPlan&
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_pcg_grid<TV, T>, b, v, g.list, g.tpc, g.rows, g.scratch);
+  return cudaLaunchKernelEx(&cfg, k_pcg_grid<TV, T>, b, v, g.list, g.tpc, g.rows, g.scratch, g.halo);
 }
 
 }  // namespace
@@ -547,12 +590,12 @@ cudaError_t launch_tv(const DeviceBatch& b, const PcgVecs<T>& v, const GridPlan&
 // The line between the one launch and the loop: whether the tiles are resident
 // at once, one CTA of at most 512 threads (128 registers each) per SM; below it
 // the launch was the faster at every size measured (343 to 68,921 vertices,
-// 1.3 to 2.0 times an iteration).
+// 1.3 to 2.1 times an iteration).
 // Tiles per CTA so that the tiles of the given scenes (their tile counts) take
 // at most one CTA per SM, the fewest that does (an SM's FP64 pipe and L2 port
 // are what an iteration runs at); none: they do not fit, and solver.cu's loop
-// runs them.  rows: the blocks of each row that then fit in shared memory.
-GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, int longestRow, bool mixed, int sms) {
+// runs them.
+GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, bool mixed, int sms) {
   GridPlan g{};
   int most = 0;
   for (int s = 0; s < n; s++) most = std::max(most, tiles[s]);
@@ -561,21 +604,100 @@ GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, int longestRow, bool 
     long long ctas = 0;
     for (int s = 0; s < n; s++) ctas += (tiles[s] + tpc - 1) / tpc;
     if (ctas > std::min(sms, kMaxCtas)) continue;
-    const int threads = tpc * tileV;
     g.ctas = (int)ctas;
     g.tpc = tpc;
-    // the partials of a scene; in FP64 the row products, nine a thread
-    g.scratch = (3 * std::max(most, (mixed ? 1 : 3) * threads) + 1) / 2 * 2;
-    const size_t row = (size_t)threads * (9 * (mixed ? sizeof(float) : sizeof(double)) + sizeof(int));
-    int rows = (int)std::min<size_t>(longestRow, (kGridSmemMax - sizeof(double) * g.scratch) / row);
-    if (!mixed) rows = longestRow % 2 && rows == longestRow && (rows + 1) * row + sizeof(double) * g.scratch <= kGridSmemMax
-                           ? rows + 1
-                           : rows / 2 * 2;
-    g.rows = rows;
-    g.smem = sizeof(double) * g.scratch + row * rows;
+    // the partials of a scene (in FP64 beside its tree's lanes); in FP64 the row
+    // products, nine a thread
+    const int threads = tpc * tileV;
+    g.scratch = mixed ? 3 * std::max(most, threads) : std::max(9 * threads, 3 * most + 9 * tileV);
+    g.scratch += g.scratch % 2;
     return g;
   }
   return g;
+}
+
+// Shared memory: the exchange area, in FP32 the u of the CTA's vertices and of
+// its halo, and of every row as many blocks and columns as still fit.
+void plan_grid_smem(GridPlan& g, int tileV, int longestRow, bool mixed) {
+  if (g.halo > kHaloMax) {
+    g = GridPlan{};
+    return;
+  }
+  const size_t threads = (size_t)g.tpc * tileV;
+  const size_t fixed = sizeof(double) * g.scratch + (mixed ? sizeof(float4) * (threads + g.halo) : 0);
+  const size_t row = threads * (9 * (mixed ? sizeof(float) : sizeof(double)) + sizeof(int));
+  const int fit = (int)((kGridSmemMax - fixed) / row);
+  // FP64 takes two blocks a trip
+  g.rows = mixed ? std::min(longestRow, fit) : std::min(longestRow + longestRow % 2, fit / 2 * 2);
+  g.smem = fixed + row * g.rows;
+}
+
+// A CTA's halo: the vertices of other CTAs in its rows' columns, ascending (a
+// bit per vertex of the scene, then ranks), and every column's index in the
+// shared u: the thread of an own vertex, or past the threads the halo's rank.
+// A list longer than its room (four times the CTA's vertices, kHaloMax) leaves
+// the batch to solver.cu's loop.
+constexpr int kHaloWords = 152 * kGridThreads / 32 + 8 * kMaxCtas;
+__global__ void __launch_bounds__(kGridThreads) k_grid_halo(DeviceBatch b, const int2* __restrict__ ctas, int tpc,
+                                                            int* largest) {
+  __shared__ unsigned bits[kHaloWords];
+  __shared__ int rank[kHaloWords];
+  __shared__ int warpTot[kGridThreads / 32];
+  const int tid = threadIdx.x, NT = blockDim.x;
+  const int2 cta = ctas[blockIdx.x];
+  const SceneParams& sp = b.scenes[cta.x];
+  const int v0 = sp.v0, words = (sp.nv + 31) / 32;
+  const int a = b.tileV0[sp.tile0 + cta.y], z = b.tileV1[sp.tile0 + min(sp.ntiles, cta.y + tpc) - 1];
+  if (words > kHaloWords) return;  // (a scene of a plan has at most one CTA's vertices per SM)
+  for (int i = tid; i < words; i += NT) bits[i] = 0u;
+  __syncthreads();
+  const int u = a + tid;
+  const int len = u < z ? b.rowptr[u + 1] - b.rowptr[u] : 0;
+  const size_t cb = u < z ? col_slot(b, u, 0) : 0;
+  for (int j = 0; j < len; j++) {
+    const int w = b.colS[cb + kSlice * j];
+    if (w < a || w >= z) atomicOr(&bits[(w - v0) / 32], 1u << ((w - v0) % 32));
+  }
+  __syncthreads();
+  // exclusive ranks of the words: each thread a run of them, then the runs
+  const int per = (words + NT - 1) / NT, i0 = min(words, tid * per), i1 = min(words, i0 + per);
+  int mine = 0;
+  for (int i = i0; i < i1; i++) mine += __popc(bits[i]);
+  int x = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (tid % 32 >= o) x += y;
+  }
+  if (tid % 32 == 31) warpTot[tid / 32] = x;
+  __syncthreads();
+  int at = x - mine;
+  for (int i = 0; i < tid / 32; i++) at += warpTot[i];
+  const int cap = min(kHaloMax, 4 * (z - a));
+  int* list = b.gridHalo + 4 * (size_t)a;
+  for (int i = i0; i < i1; i++) {
+    rank[i] = at;
+    for (unsigned m = bits[i]; m; m &= m - 1, at++)
+      if (at < cap) list[at] = v0 + 32 * i + __ffs(m) - 1;
+  }
+  if (tid == NT - 1) {
+    b.gridHaloCount[sp.tile0 + cta.y] = at;
+    atomicMax(largest, at <= cap ? at : kHaloMax + 1);
+  }
+  __syncthreads();
+  for (int j = 0; j < len; j++) {
+    const int w = b.colS[cb + kSlice * j], l = w - v0;
+    int c = w - a;
+    if (w < a || w >= z) {
+      const int r = rank[l / 32] + __popc(bits[l / 32] & ((1u << (l % 32)) - 1u));
+      c = NT + r;
+    }
+    b.clusterGather[cb + kSlice * j] = c;
+  }
+}
+
+void launch_grid_halo(const DeviceBatch& b, const GridPlan& g, int* largest, cudaStream_t s) {
+  k_grid_halo<<<g.ctas, g.tpc * b.tileV, 0, s>>>(b, g.list, g.tpc, largest);
 }
 
 // Dynamic shared-memory opt-in (once per process, outside capture).

@@ -361,7 +361,7 @@ __global__ void k_diag_inverse(DeviceBatch b, const T* __restrict__ lhs, T* __re
 #pragma unroll
     for (int i = 0; i < 9; i++) D[i] += b.coll.diag[9 * (size_t)u + i];
   }
-  T* M = minv + 9 * (size_t)u;
+  T* M = minv + minv_slot(u);
   if (precond == 1) {
     const double c00 = D[4] * D[8] - D[5] * D[7];
     const double c01 = D[5] * D[6] - D[3] * D[8];
@@ -369,19 +369,19 @@ __global__ void k_diag_inverse(DeviceBatch b, const T* __restrict__ lhs, T* __re
     const double det = D[0] * c00 + D[1] * c01 + D[2] * c02;
     const double id = 1.0 / det;
     M[0] = T(c00 * id);
-    M[1] = T((D[2] * D[7] - D[1] * D[8]) * id);
-    M[2] = T((D[1] * D[5] - D[2] * D[4]) * id);
-    M[3] = T(c01 * id);
-    M[4] = T((D[0] * D[8] - D[2] * D[6]) * id);
-    M[5] = T((D[2] * D[3] - D[0] * D[5]) * id);
-    M[6] = T(c02 * id);
-    M[7] = T((D[1] * D[6] - D[0] * D[7]) * id);
-    M[8] = T((D[0] * D[4] - D[1] * D[3]) * id);
+    M[kSlice * 1] = T((D[2] * D[7] - D[1] * D[8]) * id);
+    M[kSlice * 2] = T((D[1] * D[5] - D[2] * D[4]) * id);
+    M[kSlice * 3] = T(c01 * id);
+    M[kSlice * 4] = T((D[0] * D[8] - D[2] * D[6]) * id);
+    M[kSlice * 5] = T((D[2] * D[3] - D[0] * D[5]) * id);
+    M[kSlice * 6] = T(c02 * id);
+    M[kSlice * 7] = T((D[1] * D[6] - D[0] * D[7]) * id);
+    M[kSlice * 8] = T((D[0] * D[4] - D[1] * D[3]) * id);
   } else {
 #pragma unroll
-    for (int i = 0; i < 9; i++) M[i] = T(0);
+    for (int i = 0; i < 9; i++) M[kSlice * i] = T(0);
 #pragma unroll
-    for (int i = 0; i < 3; i++) M[4 * i] = T(D[4 * i] != 0.0 ? 1.0 / D[4 * i] : 1.0);
+    for (int i = 0; i < 3; i++) M[kSlice * 4 * i] = T(D[4 * i] != 0.0 ? 1.0 / D[4 * i] : 1.0);
   }
 }
 
@@ -562,11 +562,11 @@ __global__ void __launch_bounds__(TV) k_inner_init(DeviceBatch b, PcgVecs<T> v) 
       }
       rr += r3[i] * r3[i];
     }
-    const T* M = v.minv + 9 * (size_t)u;
+    const T* M = v.minv + minv_slot(u);
     T u3[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-      u3[i] = M[3 * i] * r3[0] + M[3 * i + 1] * r3[1] + M[3 * i + 2] * r3[2];
+      u3[i] = M[kSlice * (3 * i)] * r3[0] + M[kSlice * (3 * i + 1)] * r3[1] + M[kSlice * (3 * i + 2)] * r3[2];
       v.u[3 * u + i] = u3[i];
       ru += r3[i] * u3[i];
     }
@@ -696,7 +696,7 @@ __device__ __forceinline__ void spmv_tile_rows(const DeviceBatch& b, const PcgVe
   if (!last_tile(&st.ticketA, sp.ntiles, flag)) return;
   const int n = sp.ntiles, trees = scene_trees<TV>(n);
   const double* part = b.partial + (size_t)kPartials * sp.tile0;
-  scene_tree32<TV>(n, [&](int c, int i) { return __ldcg(&part[kPartials * (size_t)i + c]); }, sh);
+  scene_tree32<TV>(n, [&](int c, int i) { return __ldcg(&part[kPartials * (size_t)i + c]); }, vals, sh);
   __syncthreads();
   if (threadIdx.x == 0)
     spmv_decide<T>(b, st, chain(sh, trees), chain(sh + trees, trees), chain(sh + 2 * trees, trees));
@@ -836,10 +836,11 @@ __device__ __forceinline__ void update_tile(const DeviceBatch& b, const PcgVecs<
   const bool valid = lane < 30 && row < 3 * b.tileV1[tile];
   T M0 = T(0), M1 = T(0), M2 = T(0);
   if (valid) {
-    const T* M = v.minv + 3 * (size_t)row;  // row i of the vertex's block
+    const int u = row / 3;
+    const T* M = v.minv + minv_slot(u) + kSlice * 3 * (row - 3 * u);  // row i of the vertex's block
     M0 = M[0];
-    M1 = M[1];
-    M2 = M[2];
+    M1 = M[kSlice];
+    M2 = M[2 * kSlice];
   }
   pdl_wait();
   // the solve state and the row's six vectors in one round of loads; the
