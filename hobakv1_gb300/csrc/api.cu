@@ -1330,6 +1330,7 @@ int build_collisions(hobak_batch_t* B) {
   const size_t oCell = A.reserve(sizeof(unsigned) * n), oInv = A.reserve(nv), oSkip = A.reserve(ntri);
   const size_t oBucket = A.reserve(sizeof(int) * (hash + 1)), oCursor = A.reserve(sizeof(int) * hash);
   const size_t oEntry = A.reserve(sizeof(int) * 8 * (size_t)ntri);
+  const size_t oTriBox = A.reserve(2 * sizeof(float4) * (size_t)ntri);
   const size_t oSvCount = A.reserve(sizeof(int) * (nsv + 1));
   const size_t oCand = A.reserve(sizeof(int) * (size_t)kMaxPairsPerVertex * nsv);
   const size_t oOver = A.reserve(sizeof(int)), oNp = A.reserve(sizeof(int));
@@ -1347,6 +1348,8 @@ int build_collisions(hobak_batch_t* B) {
   const size_t oEeAB = A.reserve(sizeof(double4) * (size_t)nedge), oEeCount = A.reserve(sizeof(int) * (nedge + 1));
   const size_t oEeCell = A.reserve(sizeof(unsigned) * n), oEeBucket = A.reserve(sizeof(int) * (eeHash + 1));
   const size_t oEeCursor = A.reserve(sizeof(int) * eeHash), oEeEntry = A.reserve(sizeof(int) * 8 * (size_t)nedge);
+  const size_t oEeBox = A.reserve(2 * sizeof(float4) * (size_t)nedge), oEeLow = A.reserve(sizeof(int4) * (size_t)nedge);
+  const size_t oEeSeg = A.reserve(2 * sizeof(float4) * (size_t)nedge);
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, A.used);
   if (e != cudaSuccess)
@@ -1376,6 +1379,7 @@ int build_collisions(hobak_batch_t* B) {
   c.bucketCount = carve<int>(base, oBucket);
   c.bucketCursor = carve<int>(base, oCursor);
   c.entryTri = carve<int>(base, oEntry);
+  c.triBox = carve<float4>(base, oTriBox);
   c.svCount = carve<int>(base, oSvCount);
   c.svCand = carve<int>(base, oCand);
   c.overflow = carve<int>(base, oOver);
@@ -1405,6 +1409,9 @@ int build_collisions(hobak_batch_t* B) {
   c.eeBucketCount = carve<int>(base, oEeBucket);
   c.eeBucketCursor = carve<int>(base, oEeCursor);
   c.eeEntry = carve<int>(base, oEeEntry);
+  c.eeBox = carve<float4>(base, oEeBox);
+  c.eeSeg = carve<float4>(base, oEeSeg);
+  c.eeCell = carve<int4>(base, oEeLow);
   B->collScenes.assign(n, CollisionScene{0, 0, 0, 0, 0, 0.01, 1.0, 0.001});
   for (int s = 0; s < n; s++) {
     B->collScenes[s].tri0 = B->surfTriStart[s];

@@ -43,6 +43,10 @@ struct DeviceCollisions {
   unsigned* cellBits;      // [nscenes] largest triangle extent (float bits) -> cell size
   unsigned char* vInverted;  // [nv]
   unsigned char* triSkip;    // [ntri] degenerate or all-inverted
+  // FP32 boxes for the queries, rounded outward: lo.xyz and the scene id, hi.xyz
+  // and the skip flag (triangles) or the cell of the box's lower corner (edges,
+  // eeCell); a triangle's box inflated by eps and a margin, an edge's by eps
+  float4* triBox;          // [2 ntri]
   int* bucketCount;        // [hashSize + 1] then exclusive scan
   int* bucketCursor;       // [hashSize]
   int* entryTri;           // [8 * ntri]
@@ -69,6 +73,9 @@ struct DeviceCollisions {
   // edge-edge broad phase: each edge's eps-inflated box hashed into cells no
   // smaller than the scene's largest inflated edge extent (<= 8 cells each)
   int eeHashSize;
+  float4* eeBox;           // [2 nedge]
+  float4* eeSeg;           // [2 nedge] FP32 end points
+  int4* eeCell;            // [nedge] lowest cell of the inflated box
   unsigned* eeCellBits;    // [nscenes] largest inflated edge extent (float bits)
   int* eeBucketCount;      // [eeHashSize + 1] then exclusive scan
   int* eeBucketCursor;     // [eeHashSize]
