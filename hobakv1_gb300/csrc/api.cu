@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -44,6 +45,59 @@ namespace {
                   std::string(#expr) + ": " + cudaGetErrorString(_e));                          \
   } while (0)
 
+// Scratch of the calls that evaluate elements or materials: from a pool of the
+// device, ordered on the default stream these calls run on, where cudaMalloc and
+// cudaFree cost 100 us of a 150 us call.  The pool keeps at most kScratchKept
+// bytes between calls (the rest goes back at the next synchronisation), all of
+// it goes back before a batch allocates, and the driver serialises its users.
+constexpr unsigned long long kScratchKept = 64ull << 20;
+
+cudaMemPool_t scratch_pool(bool make) {
+  constexpr int kDevices = 64;
+  static std::mutex lock;
+  static cudaMemPool_t pools[kDevices];
+  static bool made[kDevices];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices) return nullptr;
+  std::lock_guard<std::mutex> g(lock);
+  if (made[dev] || !make) return pools[dev];
+  made[dev] = true;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t p = nullptr;
+  unsigned long long keep = kScratchKept;
+  if (cudaMemPoolCreate(&p, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    (void)cudaGetLastError();
+    if (p) cudaMemPoolDestroy(p);
+    p = nullptr;  // such a device allocates each time
+  }
+  return pools[dev] = p;
+}
+
+void scratch_trim() {
+  if (cudaMemPool_t p = scratch_pool(false)) cudaMemPoolTrimTo(p, 0);
+}
+
+struct DeviceScratch {
+  void* p = nullptr;
+  bool pooled = false;
+  cudaError_t get(size_t bytes) {
+    if (cudaMemPool_t pool = scratch_pool(true)) {
+      if (cudaMallocFromPoolAsync(&p, bytes, pool, 0) == cudaSuccess) {
+        pooled = true;
+        return cudaSuccess;
+      }
+      (void)cudaGetLastError();
+    }
+    return cudaMalloc(&p, bytes);
+  }
+  ~DeviceScratch() {
+    if (p) pooled ? cudaFreeAsync(p, 0) : cudaFree(p);
+  }
+};
 // One device allocation carved into aligned sub-buffers.
 struct Arena {
   char* base = nullptr;
@@ -1594,6 +1648,7 @@ int hobak_batch_create(const hobak_scene_desc* scenes, int nscenes, const hobak_
   for (int s = 0; s < nscenes; s++)
     if ((rc = validate_scene(scenes[s], s))) return rc;
   if ((rc = hobak_device_check(nullptr, nullptr, nullptr))) return rc;
+  scratch_trim();
   std::unique_ptr<hobak_batch_t> B(new hobak_batch_t);
   if (opts)
     B->opts = *opts;
@@ -2268,12 +2323,6 @@ int hobak_batch_set_tuning(hobak_batch b, const hobak_tuning* t) {
 }
 
 namespace {
-struct DeviceScratch {
-  void* p = nullptr;
-  ~DeviceScratch() {
-    if (p) cudaFree(p);
-  }
-};
 struct EventPair {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   ~EventPair() {
@@ -2451,7 +2500,7 @@ int material_eval(const hobak_material* m, int n, const double* F, const double*
   const size_t nin = U ? 21 : 9;
   const size_t nout = (psi ? 1 : 0) + (P ? 9 : 0) + (H ? 81 : 0) + (Hu ? 81 : 0);
   DeviceScratch scratch;
-  CUDA_TRY(cudaMalloc(&scratch.p, (nin + nout) * N * sizeof(double)));
+  CUDA_TRY(scratch.get((nin + nout) * N * sizeof(double)));
   double* cur = static_cast<double*>(scratch.p);
   auto take = [&](size_t per) {
     double* p = cur;
@@ -2521,39 +2570,31 @@ int hobak_element_eval(int nv, int nt, const double* rest, const int* tets, cons
     if (tets[k] < 0 || tets[k] >= nv) return fail(HOBAK_ERR_INVALID, "tet vertex id out of range");
   int rc = hobak_device_check(nullptr, nullptr, nullptr);
   if (rc) return rc;
-  std::vector<double> Dm(9 * (size_t)nt), vol(nt);
-  for (int t = 0; t < nt; t++) {
-    const double* p[4];
-    for (int a = 0; a < 4; a++) p[a] = rest + 3 * (size_t)tets[4 * (size_t)t + a];
-    vol[t] = tet_volume(p[0], p[1], p[2], p[3]);
-    dm_inverse(p[0], p[1], p[2], p[3], &Dm[9 * (size_t)t]);
-  }
   const size_t T = (size_t)nt, V = (size_t)nv;
-  double *dRest, *dX, *dDm, *dVol, *dF = nullptr, *dS = nullptr, *dFo = nullptr, *dH = nullptr;
-  int4* dTets;
-  CUDA_TRY(cudaMalloc(&dRest, 3 * V * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&dX, 3 * V * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&dDm, 9 * T * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&dVol, T * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&dTets, T * sizeof(int4)));
-  if (F) CUDA_TRY(cudaMalloc(&dF, 9 * T * sizeof(double)));
-  if (sigma) CUDA_TRY(cudaMalloc(&dS, 3 * T * sizeof(double)));
-  if (force) CUDA_TRY(cudaMalloc(&dFo, 12 * T * sizeof(double)));
-  if (hessian) CUDA_TRY(cudaMalloc(&dH, 144 * T * sizeof(double)));
-  CUDA_TRY(cudaMemcpy(dRest, rest, 3 * V * sizeof(double), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(dX, x, 3 * V * sizeof(double), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(dDm, Dm.data(), 9 * T * sizeof(double), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(dVol, vol.data(), T * sizeof(double), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(dTets, tets, T * sizeof(int4), cudaMemcpyHostToDevice));
-  launch_element_eval(nt, dTets, dRest, dX, dDm, dVol, m->kind, m->mu, m->lambda, m->fiber, dF, dS, dFo, dH, 0);
+  // tets first (16-byte aligned), then doubles
+  const size_t per = (F ? 9 : 0) + (sigma ? 3 : 0) + (force ? 12 : 0) + (hessian ? 144 : 0);
+  DeviceScratch scratch;
+  CUDA_TRY(scratch.get(T * sizeof(int4) + (6 * V + per * T) * sizeof(double)));
+  int4* dTets = static_cast<int4*>(scratch.p);
+  double* cur = reinterpret_cast<double*>(dTets + T);
+  auto take = [&](size_t n) {
+    double* p = cur;
+    cur += n;
+    return p;
+  };
+  double *dRest = take(3 * V), *dX = take(3 * V);
+  double *dF = F ? take(9 * T) : nullptr, *dS = sigma ? take(3 * T) : nullptr;
+  double *dFo = force ? take(12 * T) : nullptr, *dH = hessian ? take(144 * T) : nullptr;
+  CUDA_TRY(cudaMemcpyAsync(dRest, rest, 3 * V * sizeof(double), cudaMemcpyHostToDevice, 0));
+  CUDA_TRY(cudaMemcpyAsync(dX, x, 3 * V * sizeof(double), cudaMemcpyHostToDevice, 0));
+  CUDA_TRY(cudaMemcpyAsync(dTets, tets, T * sizeof(int4), cudaMemcpyHostToDevice, 0));
+  launch_element_eval(nt, dTets, dRest, dX, nullptr, nullptr, m->kind, m->mu, m->lambda, m->fiber, dF, dS, dFo, dH, 0);
   CUDA_TRY(cudaGetLastError());
-  if (F) CUDA_TRY(cudaMemcpy(F, dF, 9 * T * sizeof(double), cudaMemcpyDeviceToHost));
-  if (sigma) CUDA_TRY(cudaMemcpy(sigma, dS, 3 * T * sizeof(double), cudaMemcpyDeviceToHost));
-  if (force) CUDA_TRY(cudaMemcpy(force, dFo, 12 * T * sizeof(double), cudaMemcpyDeviceToHost));
-  if (hessian) CUDA_TRY(cudaMemcpy(hessian, dH, 144 * T * sizeof(double), cudaMemcpyDeviceToHost));
-  for (void* p : {(void*)dRest, (void*)dX, (void*)dDm, (void*)dVol, (void*)dTets, (void*)dF, (void*)dS,
-                  (void*)dFo, (void*)dH})
-    cudaFree(p);
+  if (F) CUDA_TRY(cudaMemcpyAsync(F, dF, 9 * T * sizeof(double), cudaMemcpyDeviceToHost, 0));
+  if (sigma) CUDA_TRY(cudaMemcpyAsync(sigma, dS, 3 * T * sizeof(double), cudaMemcpyDeviceToHost, 0));
+  if (force) CUDA_TRY(cudaMemcpyAsync(force, dFo, 12 * T * sizeof(double), cudaMemcpyDeviceToHost, 0));
+  if (hessian) CUDA_TRY(cudaMemcpyAsync(hessian, dH, 144 * T * sizeof(double), cudaMemcpyDeviceToHost, 0));
+  CUDA_TRY(cudaStreamSynchronize(0));
   return HOBAK_OK;
 }
 

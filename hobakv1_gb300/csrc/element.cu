@@ -613,15 +613,45 @@ __global__ void k_material_eval(MatParams m, int n, const double* Fin, const dou
   }
 }
 
+// Rest volume and DmInv by cofactors of a tet (TET_MESH.cpp:121-191), as
+// build_batch forms them on the host.
+__device__ __forceinline__ double rest_shape(const int4 tv, const double* rest, double* Ai) {
+  const double *x0 = rest + 3 * (size_t)tv.x, *x1 = rest + 3 * (size_t)tv.y, *x2 = rest + 3 * (size_t)tv.z,
+               *x3 = rest + 3 * (size_t)tv.w;
+  double A[9];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    A[i] = x1[i] - x0[i];
+    A[3 + i] = x2[i] - x0[i];
+    A[6 + i] = x3[i] - x0[i];
+  }
+  const double det = det3(A), id = 1.0 / det;
+  Ai[0] = (A[4] * A[8] - A[5] * A[7]) * id;
+  Ai[1] = (A[2] * A[7] - A[1] * A[8]) * id;
+  Ai[2] = (A[1] * A[5] - A[2] * A[4]) * id;
+  Ai[3] = (A[5] * A[6] - A[3] * A[8]) * id;
+  Ai[4] = (A[0] * A[8] - A[2] * A[6]) * id;
+  Ai[5] = (A[2] * A[3] - A[0] * A[5]) * id;
+  Ai[6] = (A[3] * A[7] - A[4] * A[6]) * id;
+  Ai[7] = (A[1] * A[6] - A[0] * A[7]) * id;
+  Ai[8] = (A[0] * A[4] - A[1] * A[3]) * id;
+  return det / 6.0;
+}
+
 // Standalone: per-tet F, sigma, element force and full 12x12 element Hessian.
+// DmInv, volume: null to form them here.
 __global__ void k_element_eval(int nt, const int4* tets, const double* rest, const double* x, const double* DmInv,
                                const double* volume, MatParams m, double* Fo, double* So, double* fo, double* Ho) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
-  double Dinv[9];
+  double Dinv[9], vol;
+  if (DmInv) {
 #pragma unroll
-  for (int k = 0; k < 9; k++) Dinv[k] = DmInv[9 * (size_t)t + k];
-  const double vol = volume[t];
+    for (int k = 0; k < 9; k++) Dinv[k] = DmInv[9 * (size_t)t + k];
+    vol = volume[t];
+  } else {
+    vol = rest_shape(tets[t], rest, Dinv);
+  }
   double X[4][3];
   load_tet(tets[t], rest, x, X);
   double F[9], U[9], S[3], V[9], P[9], f[12];
@@ -742,16 +772,18 @@ void launch_material_eval(int kind, double mu, double lambda, const double* fibe
                           const double* U, const double* S, const double* V, double* psi, double* P, double* H,
                           double* Hu, cudaStream_t s) {
   if (n <= 0) return;
-  k_material_eval<<<(n + 127) / 128, 128, 0, s>>>(make_material(kind, mu, lambda, fiber), n, F, U, S, V, psi, P,
-                                                   H, Hu);
+  const int cta = 128;
+  k_material_eval<<<(n + cta - 1) / cta, cta, 0, s>>>(make_material(kind, mu, lambda, fiber), n, F, U, S, V, psi, P, H,
+                                                      Hu);
 }
 
 void launch_element_eval(int nt, const int4* tets, const double* rest, const double* x, const double* DmInv,
                          const double* vol, int kind, double mu, double lambda, const double* fiber, double* F,
                          double* sigma, double* force, double* hessian, cudaStream_t s) {
   if (nt <= 0) return;
-  k_element_eval<<<(nt + 127) / 128, 128, 0, s>>>(nt, tets, rest, x, DmInv, vol,
-                                                   make_material(kind, mu, lambda, fiber), F, sigma, force, hessian);
+  const int cta = 128;
+  k_element_eval<<<(nt + cta - 1) / cta, cta, 0, s>>>(nt, tets, rest, x, DmInv, vol,
+                                                      make_material(kind, mu, lambda, fiber), F, sigma, force, hessian);
 }
 
 }  // namespace hobak
