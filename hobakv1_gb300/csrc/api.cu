@@ -164,6 +164,8 @@ struct hobak_batch_t {
   int longestRow = 0;        // blocks of the longest matrix row
   cudaStream_t classStream[kClusterClasses] = {};  // classes run beside the tile path (fork/join)
   cudaEvent_t evFork = nullptr, evJoin[kClusterClasses] = {};
+  cudaStream_t rhsStream = nullptr;  // the right-hand side beside assembly and preconditioner
+  cudaEvent_t evTerms = nullptr, evRhs = nullptr;
   int lastStatus = HOBAK_OK;
   std::vector<SolveState> lastSolve;
   std::vector<int> hostRowptr, hostCols;
@@ -1129,6 +1131,32 @@ int enqueue_solve_t(hobak_batch_t* B, cudaStream_t s, bool capture, const PcgVec
   return HOBAK_OK;
 }
 
+// From the element and contact terms to the linear system: the matrix and its
+// preconditioner on s, the right-hand side beside them on its own stream (both
+// only read the terms; on a small scene each is 15-30 us of latency on a few
+// SMs).  `timed` keeps them one after the other, for the phase events.
+template <typename T>
+int enqueue_system(hobak_batch_t* B, cudaStream_t s, const PcgVecs<T>& v, bool timed, unsigned evFlags) {
+  const DeviceBatch& d = B->d;
+  if (!timed) {
+    CUDA_TRY(cudaEventRecord(B->evTerms, s));
+    CUDA_TRY(cudaStreamWaitEvent(B->rhsStream, B->evTerms, 0));
+    launch_rhs(d, B->rhsStream);
+    CUDA_TRY(cudaEventRecord(B->evRhs, B->rhsStream));
+  }
+  launch_assemble<T>(d, v, s);
+  if (d.collOn) launch_collision_diag(d, d.coll, s);
+  launch_diag_inverse<T>(d, v, B->opts.preconditioner, s);
+  if (timed) {
+    CUDA_TRY(cudaEventRecordWithFlags(B->ev[2], s, evFlags));
+    launch_rhs(d, s);
+    CUDA_TRY(cudaEventRecordWithFlags(B->ev[3], s, evFlags));
+  } else {
+    CUDA_TRY(cudaStreamWaitEvent(s, B->evRhs, 0));
+  }
+  return HOBAK_OK;
+}
+
 // One Newton iteration of NEWMARK::solveRayleighDamped (NEWMARK.cpp:216-318):
 // element terms at the current x, assembly, preconditioner, rhs and its
 // |rhs|^2, the linear solve, x -= y and the per-scene Newton test.
@@ -1140,10 +1168,7 @@ int enqueue_newton_body(hobak_batch_t* B, cudaStream_t s, bool capture, const Pc
   launch_green_damping(d, s);
   // contact at the iterate (NEWMARK.cpp:226-242)
   if (d.collOn) launch_collisions(d, d.coll, s);
-  launch_assemble<T>(d, v, s);
-  if (d.collOn) launch_collision_diag(d, d.coll, s);
-  launch_diag_inverse<T>(d, v, B->opts.preconditioner, s);
-  launch_rhs(d, s);
+  if (int rc = enqueue_system<T>(B, s, v, false, 0)) return rc;
   if (int rc = enqueue_solve_t<T>(B, s, capture, v)) return rc;
   launch_newton_update(d, s);
   return HOBAK_OK;
@@ -1198,12 +1223,7 @@ int enqueue_step_t(hobak_batch_t* B, cudaStream_t s, bool capture, bool timed, c
     else launch_element(d, s);
     if (d.collOn) launch_collisions(d, d.coll, s);
     if (timed) CUDA_TRY(cudaEventRecordWithFlags(B->ev[1], s, evFlags));
-    launch_assemble<T>(d, v, s);
-    if (d.collOn) launch_collision_diag(d, d.coll, s);
-    launch_diag_inverse<T>(d, v, B->opts.preconditioner, s);
-    if (timed) CUDA_TRY(cudaEventRecordWithFlags(B->ev[2], s, evFlags));
-    launch_rhs(d, s);
-    if (timed) CUDA_TRY(cudaEventRecordWithFlags(B->ev[3], s, evFlags));
+    if (int rc = enqueue_system<T>(B, s, v, timed, evFlags)) return rc;
     if (int rc = enqueue_solve_t<T>(B, s, capture, v)) return rc;
   }
   if (timed) CUDA_TRY(cudaEventRecordWithFlags(B->ev[4], s, evFlags));
@@ -1660,6 +1680,9 @@ int hobak_batch_create(const hobak_scene_desc* scenes, int nscenes, const hobak_
   CUDA_TRY(cudaStreamCreateWithFlags(&B->captureStreamN, cudaStreamNonBlocking));
   for (auto& cs : B->classStream) CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   CUDA_TRY(cudaEventCreateWithFlags(&B->evFork, cudaEventDisableTiming));
+  CUDA_TRY(cudaStreamCreateWithFlags(&B->rhsStream, cudaStreamNonBlocking));
+  CUDA_TRY(cudaEventCreateWithFlags(&B->evTerms, cudaEventDisableTiming));
+  CUDA_TRY(cudaEventCreateWithFlags(&B->evRhs, cudaEventDisableTiming));
   for (auto& e : B->evJoin) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   CUDA_TRY(cudaMallocHost(&B->pinnedActive, 2 * sizeof(int)));
   CUDA_TRY(cudaMallocHost(&B->solvePinned, sizeof(SolveState) * nscenes));
@@ -1690,6 +1713,9 @@ int hobak_batch_destroy(hobak_batch b) {
   for (auto& cs : b->classStream)
     if (cs) cudaStreamDestroy(cs);
   if (b->evFork) cudaEventDestroy(b->evFork);
+  if (b->rhsStream) cudaStreamDestroy(b->rhsStream);
+  if (b->evTerms) cudaEventDestroy(b->evTerms);
+  if (b->evRhs) cudaEventDestroy(b->evRhs);
   for (auto& e : b->evJoin)
     if (e) cudaEventDestroy(e);
   for (auto& e : b->ev)
