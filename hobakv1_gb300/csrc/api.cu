@@ -635,6 +635,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   const size_t oGridP = A.reserve(96 * (size_t)ntilesCap), oGridF = A.reserve(sizeof(int) * ntilesCap);
   const size_t oGridL = A.reserve(sizeof(int2) * ntilesCap);
   const size_t oGridHc = A.reserve(sizeof(int) * (ntilesCap + 1));
+  const size_t oGridRw = A.reserve(sizeof(ulonglong2) * grid_row_words());
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, A.used);
   if (e != cudaSuccess)
@@ -711,6 +712,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   d.gridTilesCap = ntilesCap;
   B->gridList = carve<int2>(base, oGridL);
   d.gridHaloCount = carve<int>(base, oGridHc);
+  d.gridRowWords = carve<ulonglong2>(base, oGridRw);
   d.anyAniso = anyAniso;
   d.anyArap = anyArap;
   d.anySvdFree = anySvdFree;
@@ -768,6 +770,8 @@ int upload_solver_opts(hobak_batch_t* B) {
     s.maxSweeps = sweeps_of(B->opts);
   }
   CUDA_TRY(cudaMemcpy(B->d.solve, st.data(), sizeof(SolveState) * st.size(), cudaMemcpyHostToDevice));
+  // the scenes' solves count from zero again: no tag of theirs may be left
+  CUDA_TRY(cudaMemset(B->d.gridRowWords, 0, sizeof(ulonglong2) * grid_row_words()));
   return HOBAK_OK;
 }
 
@@ -956,11 +960,22 @@ int prepare_grid_plan(hobak_batch_t* B) {
   std::vector<int> tiles(n);
   for (int s = 0; s < n; s++) tiles[s] = B->sceneParams[s].pcgCluster ? 0 : B->sceneParams[s].ntiles;
   const bool mixed = B->opts.precision == HOBAK_PRECISION_MIXED;
-  GridPlan g = plan_grid_pcg(tiles.data(), n, B->d.tileV, mixed, sms);
+  GridPlan g{};
+  if (!mixed) {
+    if (const int ce = configure_rows_pcg())
+      return fail(HOBAK_ERR_CUDA, std::string("PCG set-up: ") + cudaGetErrorString((cudaError_t)ce));
+    std::vector<int> nv(n);
+    for (int s = 0; s < n; s++) nv[s] = B->sceneParams[s].pcgCluster ? 0 : B->sceneParams[s].nv;
+    g = plan_rows_pcg(nv.data(), n, B->longestRow, sms);
+  }
+  if (!g.ctas) g = plan_grid_pcg(tiles.data(), n, B->d.tileV, mixed, sms);
   if (g.ctas) {
     std::vector<int2> list;
     for (int s = 0; s < n; s++)
-      for (int t = 0; t < tiles[s]; t += g.tpc) list.push_back(make_int2(s, t));
+      if (g.rowVerts)
+        for (int t = 0; tiles[s] && t * g.rowVerts < B->sceneParams[s].nv; t++) list.push_back(make_int2(s, t));
+      else
+        for (int t = 0; t < tiles[s]; t += g.tpc) list.push_back(make_int2(s, t));
     CUDA_TRY(cudaStreamSynchronize(B->stream));
     CUDA_TRY(cudaMemcpy(B->gridList, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice));
     g.list = B->gridList;
@@ -972,13 +987,14 @@ int prepare_grid_plan(hobak_batch_t* B) {
       CUDA_TRY(cudaMemcpyAsync(&g.halo, largest, sizeof(int), cudaMemcpyDeviceToHost, B->stream));
       CUDA_TRY(cudaStreamSynchronize(B->stream));
     }
-    plan_grid_smem(g, B->d.tileV, B->longestRow, mixed);
+    if (!g.rowVerts) plan_grid_smem(g, B->d.tileV, B->longestRow, mixed);
   }
   if (g.ctas != B->grid.ctas || g.tpc != B->grid.tpc || g.rows != B->grid.rows || g.smem != B->grid.smem ||
-      g.scratch != B->grid.scratch || g.halo != B->grid.halo)
+      g.scratch != B->grid.scratch || g.halo != B->grid.halo ||
+      g.rowVerts != B->grid.rowVerts)
     drop_graphs(B);
   B->grid = g;
-  B->d.gridOn = g.ctas ? 1 : 0;
+  B->d.gridOn = !g.ctas ? 0 : g.rowVerts ? 2 : 1;
   B->gridDirty = false;
   return HOBAK_OK;
 }
@@ -1116,7 +1132,11 @@ int enqueue_solve_t(hobak_batch_t* B, cudaStream_t s, bool capture, const PcgVec
   for (int k = 0; k < sweeps && B->anyTileScene; k++) {
     if (B->grid.ctas) {
       launch_inner_init<T>(d, v, s);
-      const int ce = launch_grid_pcg<T>(d, v, B->grid, s);
+      int ce;
+      if constexpr (sizeof(T) == sizeof(double))
+        ce = B->grid.rowVerts ? launch_rows_pcg(d, v, B->grid, s) : launch_grid_pcg<T>(d, v, B->grid, s);
+      else
+        ce = launch_grid_pcg<T>(d, v, B->grid, s);
       if (ce) return fail(HOBAK_ERR_CUDA, std::string("PCG launch: ") + cudaGetErrorString((cudaError_t)ce));
     } else {
       launch_set_active(d, s);

@@ -84,6 +84,7 @@ struct SolveState {
   double gamma, gammaOld, delta, alpha, beta, rr, innerThreshold;
   float alphaF, betaF;  // FP32 copies for the mixed inner solve (no per-thread conversion)
   int iters, done;
+  int epoch;  // inner solves started (tags of pcg_rows.cu)
   unsigned ticketA, ticketB;
   // Newmark's Newton loop: iterations done, finished flag, |rhs|^2 of the last one
   int newtonStep, newtonDone;

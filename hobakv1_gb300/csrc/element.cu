@@ -743,8 +743,8 @@ __global__ void k_energy(DeviceBatch b) {
 // CTA size of a kernel with a thread per element: `most`, or fewer threads while
 // that leaves SMs without a CTA.  A warp alone on an SM issues an FP64
 // instruction every 64 cycles, four warps every 76 each, so a small mesh's
-// element kernel is ~15% shorter with its warps spread (1,296 tets: 57 -> 49 us;
-// 6,000: 88 -> 76 us).  Results do not depend on it.
+// element kernel is shorter with its warps spread (1,296 tets: 62 -> 58 us;
+// 6,000: 86 -> 82 us).  Results do not depend on it.
 static int element_cta(int n, int most) {
   constexpr int kSms = 152;
   int cta = most;

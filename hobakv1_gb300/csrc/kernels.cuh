@@ -44,6 +44,7 @@ struct GridPlan {
   int rows;          // blocks of every matrix row kept in shared memory
   int scratch;       // doubles of its exchange area
   int halo;          // FP32: most other vertices a CTA reads
+  int rowVerts;      // > 0: pcg_rows.cu, vertices of a CTA
   size_t smem;       // dynamic shared memory of a CTA
   const int2* list;  // device: per CTA its scene and its first tile in the scene
 };
@@ -162,7 +163,8 @@ struct DeviceBatch {
   double* gridPartials;
   int* gridFlags;
   int gridTilesCap;
-  int gridOn;  // the tile-path scenes take that path
+  int gridOn;  // the tile-path scenes take that path (2: pcg_rows.cu)
+  ulonglong2* gridRowWords;  // [2][CTAs][9] partials of pcg_rows.cu
   // FP32: per CTA the vertices of other CTAs that its rows' columns name (at
   // 4 x its first vertex), their number (per tile: a CTA's is its first
   // tile's), and every column as the CTA's own index of it (k_grid_halo; the
@@ -287,6 +289,11 @@ int configure_grid_pcg();
 // all scenes of the plan.  Returns a cudaError_t value (0 on success).
 template <typename T>
 int launch_grid_pcg(const DeviceBatch& b, const PcgVecs<T>& v, const GridPlan& g, cudaStream_t s);
+// ... and its form for small FP64 scenes (pcg_rows.cu)
+GridPlan plan_rows_pcg(const int* nv, int n, int longestRow, int sms);
+int configure_rows_pcg();
+int launch_rows_pcg(const DeviceBatch& b, const PcgVecs<double>& v, const GridPlan& g, cudaStream_t s);
+size_t grid_row_words();
 // Rebuilds the cluster kernels' gather table from the scenes' cluster sizes.
 void launch_cluster_gather(const DeviceBatch& b, cudaStream_t s);
 // Dynamic shared-memory opt-in of the cluster kernels (once, outside capture).

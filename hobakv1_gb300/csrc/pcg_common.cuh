@@ -292,6 +292,24 @@ __device__ __forceinline__ void publish_u(double* u4, int w, const double (&x)[3
   __stcg(u4 + 4 * (size_t)w + 2, x[2]);
 }
 
+// Words of the one-launch PCGs: a value and the tag it belongs to, written and
+// read at once.
+constexpr int kSpinLimit = 1 << 21;  // polls of one wait (about a second), then the solve fails
+__device__ __forceinline__ void st_word(ulonglong2* p, double value, unsigned long long tag) {
+  asm volatile(
+      "{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
+      "l"(__double_as_longlong(value)), "l"(tag)
+      : "memory");
+}
+__device__ __forceinline__ void ld_word(const ulonglong2* p, double& value, unsigned long long& tag) {
+  unsigned long long bits;
+  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+               : "=l"(bits), "=l"(tag)
+               : "l"(p)
+               : "memory");
+  value = __longlong_as_double((long long)bits);
+}
+
 // a . b of two 3-vectors, as the compiler contracts a0 b0 + a1 b1 + a2 b2
 template <typename T>
 __device__ __forceinline__ T dot3v(T a0, T a1, T a2, T b0, T b1, T b2) {

@@ -50,24 +50,9 @@ namespace {
 
 constexpr int kGridThreads = 512;      // vertices of a CTA, at most (128 registers each)
 constexpr int kGridSmemMax = 224 * 1024;
-constexpr int kSpinLimit = 1 << 21;    // polls of one wait (about a second), then the solve fails
 constexpr int kMaxCtas = 256;          // CTAs of a launch, at most (one per SM)
 constexpr int kHaloMax = 3072;         // halo vertices of a CTA, at most (48 KB of shared memory)
 
-__device__ __forceinline__ void st_word(ulonglong2* p, double value, unsigned long long tag) {
-  asm volatile(
-      "{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
-      "l"(__double_as_longlong(value)), "l"(tag)
-      : "memory");
-}
-__device__ __forceinline__ void ld_word(const ulonglong2* p, double& value, unsigned long long& tag) {
-  unsigned long long bits;
-  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
-               : "=l"(bits), "=l"(tag)
-               : "l"(p)
-               : "memory");
-  value = __longlong_as_double((long long)bits);
-}
 __device__ __forceinline__ int ld_flag(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

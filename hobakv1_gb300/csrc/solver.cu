@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(TV) k_inner_init(DeviceBatch b, PcgVecs<T> v) 
     }
     return;
   }
-  if (b.gridOn) {  // the one-launch PCG (pcg_grid.cu): no partials yet, the first u published
+  if (b.gridOn == 1) {  // the one-launch PCG (pcg_grid.cu): no partials yet, the first u published
     if (threadIdx.x < 6) {
       const size_t word = 3 * ((threadIdx.x / 3) * (size_t)b.gridTilesCap + tile) + threadIdx.x % 3;
       reinterpret_cast<ulonglong2*>(b.gridPartials)[word] = make_ulonglong2(0ull, 0ull);
@@ -570,7 +570,11 @@ __global__ void __launch_bounds__(TV) k_inner_init(DeviceBatch b, PcgVecs<T> v) 
       v.u[3 * u + i] = u3[i];
       ru += r3[i] * u3[i];
     }
-    if (b.gridOn) publish_u(v.p, u, u3, 1);
+    if (b.gridOn == 1) publish_u(v.p, u, u3, 1);
+    if constexpr (sizeof(T) == sizeof(double))
+      if (b.gridOn == 2)  // pcg_rows.cu: a word per row
+#pragma unroll
+        for (int i = 0; i < 3; i++) st_word(reinterpret_cast<ulonglong2*>(v.p) + 3 * (size_t)u + i, u3[i], 1ull);
   }
   const double trr = block_sum<TV>(rr, sh);
   const double tru = block_sum<TV>(ru, sh);
@@ -592,6 +596,7 @@ __global__ void __launch_bounds__(TV) k_inner_init(DeviceBatch b, PcgVecs<T> v) 
     st.alphaF = 1.0f;
     st.betaF = 0.0f;
     st.iters = 0;
+    st.epoch += 1;
     st.innerThreshold = fmax(itol * itol * srr, DBL_MIN);
     st.done = 0;
     if (srr == 0.0 || srr < st.innerThreshold) {

@@ -1,4 +1,5 @@
-"""The tile path's one-launch PCG (pcg_grid.cu) against its loop of two kernels
+"""The tile path's one-launch PCGs (pcg_grid.cu; pcg_rows.cu for small FP64
+batches) against its loop of two kernels
 (solver.cu): a batch with more scenes than the GPU has SMs takes the loop, the
 scene alone takes the one launch, and both give the same bits."""
 import numpy as np
@@ -18,8 +19,9 @@ def moving(N, material, seed):
 
 
 # vertices (N + 1)^3 against tiles of 128 (64): less than one tile, exactly one
-# or four of them, ragged; 27, 34 and 40: two, three and four tiles a CTA
-@pytest.mark.parametrize("N", [1, 3, 4, 7, 9, 27, 34, 40])
+# or four of them, ragged; 15 and 16: the last size with 32 vertices a CTA in
+# FP64 and the first past it; 27, 34 and 40: two, three and four tiles a CTA
+@pytest.mark.parametrize("N", [1, 3, 4, 7, 9, 15, 16, 27, 34, 40])
 @pytest.mark.parametrize("precision", [hobak.PRECISION_FP64, hobak.PRECISION_MIXED], ids=["fp64", "mixed"])
 def test_one_launch_equals_the_loop(N, precision):
     s = moving(N, "snh" if N % 2 else "arap", N)
@@ -38,8 +40,9 @@ def test_one_launch_equals_the_loop(N, precision):
 
 
 @pytest.mark.parametrize("precision", [hobak.PRECISION_FP64, hobak.PRECISION_MIXED], ids=["fp64", "mixed"])
-def test_one_launch_equals_the_loop_in_contact(precision):
-    s = scenes.two_cubes_scene(9, offset=0.05)
+@pytest.mark.parametrize("N", [9, 13])  # 63 CTAs of 32 vertices, and past 152
+def test_one_launch_equals_the_loop_in_contact(N, precision):
+    s = scenes.two_cubes_scene(N, offset=0.05)
     tiny = [scenes.config1_scene(1) for _ in range(200)]
     out = []
     for group in ([s], [s] + tiny):
