@@ -633,7 +633,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   const size_t oPart = A.reserve(sizeof(double) * kPartials * (size_t)ntilesCap);
   const size_t oPsi = A.reserve(sizeof(double) * nt);
   const size_t oGridP = A.reserve(96 * (size_t)ntilesCap), oGridF = A.reserve(sizeof(int) * ntilesCap);
-  const size_t oGridL = A.reserve(sizeof(int2) * ntilesCap);
+  const size_t oGridL = A.reserve(sizeof(int2) * kGridCtas);
   const size_t oGridHc = A.reserve(sizeof(int) * (ntilesCap + 1));
   const size_t oGridRw = A.reserve(sizeof(ulonglong2) * grid_row_words());
   void* base = nullptr;
@@ -976,6 +976,7 @@ int prepare_grid_plan(hobak_batch_t* B) {
         for (int t = 0; tiles[s] && t * g.rowVerts < B->sceneParams[s].nv; t++) list.push_back(make_int2(s, t));
       else
         for (int t = 0; t < tiles[s]; t += g.tpc) list.push_back(make_int2(s, t));
+    if ((int)list.size() != g.ctas || g.ctas > kGridCtas) return fail(HOBAK_ERR_CUDA, "PCG plan: wrong CTA count");
     CUDA_TRY(cudaStreamSynchronize(B->stream));
     CUDA_TRY(cudaMemcpy(B->gridList, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice));
     g.list = B->gridList;

@@ -39,6 +39,7 @@ struct ClusterClass {
 
 // The tile path's PCG in one cooperative launch (pcg_grid.cu): ctas == 0 where
 // the batch's tiles do not fit the GPU at once.
+constexpr int kGridCtas = 256;  // CTAs of a launch, at most (one per SM; the CTA table's room)
 struct GridPlan {
   int ctas, tpc;     // CTAs, tiles per CTA (one scene per CTA)
   int rows;          // blocks of every matrix row kept in shared memory

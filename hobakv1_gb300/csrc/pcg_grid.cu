@@ -50,7 +50,7 @@ namespace {
 
 constexpr int kGridThreads = 512;      // vertices of a CTA, at most (128 registers each)
 constexpr int kGridSmemMax = 224 * 1024;
-constexpr int kMaxCtas = 256;          // CTAs of a launch, at most (one per SM)
+constexpr int kMaxCtas = kGridCtas;
 constexpr int kHaloMax = 3072;         // halo vertices of a CTA, at most (48 KB of shared memory)
 
 __device__ __forceinline__ int ld_flag(const int* p) {

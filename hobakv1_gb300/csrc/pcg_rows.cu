@@ -26,7 +26,7 @@ namespace {
 
 constexpr int kRowVerts = 32;                // vertices of a CTA
 constexpr int kRowThreads = 3 * kRowVerts;
-constexpr int kRowCtas = 256;                // CTAs of a launch, at most
+constexpr int kRowCtas = kGridCtas;
 constexpr int kRowSmemMax = 200 * 1024;
 constexpr int kBatch = 4;                    // blocks whose u is in flight
 constexpr int kWords = 8;                    // partials a thread polls at a time

@@ -19,9 +19,9 @@ def moving(N, material, seed):
 
 
 # vertices (N + 1)^3 against tiles of 128 (64): less than one tile, exactly one
-# or four of them, ragged; 15 and 16: the last size with 32 vertices a CTA in
-# FP64 and the first past it; 27, 34 and 40: two, three and four tiles a CTA
-@pytest.mark.parametrize("N", [1, 3, 4, 7, 9, 15, 16, 27, 34, 40])
+# or four of them, ragged; 14, 15 and 16: more CTAs of 32 vertices in FP64
+# than tiles, the last such size and the first past it; 27, 34 and 40: two, three and four tiles a CTA
+@pytest.mark.parametrize("N", [1, 3, 4, 7, 9, 14, 15, 16, 27, 34, 40])
 @pytest.mark.parametrize("precision", [hobak.PRECISION_FP64, hobak.PRECISION_MIXED], ids=["fp64", "mixed"])
 def test_one_launch_equals_the_loop(N, precision):
     s = moving(N, "snh" if N % 2 else "arap", N)
