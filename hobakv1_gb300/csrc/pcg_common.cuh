@@ -138,15 +138,15 @@ __device__ __forceinline__ void tree32(int n, Get get, double* out) {
   for (int g0 = 8 * (threadIdx.x / 32); g0 < n; g0 += 8 * (blockDim.x / 32)) tree32_warp(g0, n, get, out);
 }
 
-// Sum of n <= 12 values in order, their loads ahead of the adds.
+// Sum of n values in order, each loaded ahead of the add before it.
 __device__ __forceinline__ double chain(const double* v, int n) {
-  double x[12];
-#pragma unroll
-  for (int i = 0; i < 12; i++) x[i] = i < n ? v[i] : 0.0;
-  double t = x[0];
-#pragma unroll
-  for (int i = 1; i < 12; i++)
-    if (i < n) t += x[i];
+  double t = v[0], next = n > 1 ? v[1] : 0.0;
+#pragma unroll 1
+  for (int i = 1; i < n; i++) {
+    const double x = next;
+    if (i + 1 < n) next = v[i + 1];
+    t += x;
+  }
   return t;
 }
 
