@@ -310,6 +310,29 @@ __device__ __forceinline__ void ld_word(const ulonglong2* p, double& value, unsi
   value = __longlong_as_double((long long)bits);
 }
 
+// N words whose tags must all be `tag`: use(k) says which of them, at(k) where.
+// All are loaded at once, and those not there yet again at once, so a wait costs
+// the latency of the last one and not of each.  Clears ok when they never come.
+template <int N, typename Use, typename At>
+__device__ __forceinline__ void ld_words(Use use, At at, unsigned long long tag, double (&value)[N], bool& ok) {
+  unsigned long long got[N];
+#pragma unroll
+  for (int k = 0; k < N; k++)
+    if (use(k)) ld_word(at(k), value[k], got[k]);
+#pragma unroll 1
+  for (int n = 0; ok; n++) {
+    bool missing = false;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (use(k) && got[k] != tag) missing = true;
+    if (!missing) break;
+    if (n > kSpinLimit) ok = false;
+#pragma unroll
+    for (int k = 0; k < N; k++)
+      if (use(k) && got[k] != tag) ld_word(at(k), value[k], got[k]);
+  }
+}
+
 // a . b of two 3-vectors, as the compiler contracts a0 b0 + a1 b1 + a2 b2
 template <typename T>
 __device__ __forceinline__ T dot3v(T a0, T a1, T a2, T b0, T b1, T b2) {

@@ -466,20 +466,12 @@ __global__ void __launch_bounds__(kGridThreads, 1)
 #pragma unroll 1
     for (int i0 = tid; i0 < 3 * nParts; i0 += 4 * NT) {
       double value[4];
-      unsigned long long tag[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        if (i0 + k * NT < 3 * nParts) ld_word(in + i0 + k * NT, value[k], tag[k]);
+      ld_words<4>([&](int k) { return i0 + k * NT < 3 * nParts; }, [&](int k) { return in + i0 + k * NT; },
+                  (unsigned long long)it, value, ok);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         const int i = i0 + k * NT;
-        if (i >= 3 * nParts) break;
-#pragma unroll 1
-        for (int n = 0; tag[k] != (unsigned long long)it && ok; n++) {
-          if (n > kSpinLimit) ok = false;
-          ld_word(in + i, value[k], tag[k]);
-        }
-        area[(i % 3) * nParts + i / 3] = value[k];
+        if (i < 3 * nParts) area[(i % 3) * nParts + i / 3] = value[k];
       }
     }
     failed = __syncthreads_or(!ok);
