@@ -351,7 +351,7 @@ int alloc_precision(hobak_batch_t* B) {
   const size_t oMinv = A.reserve(w * kSlotVals * ((nv + kSlice - 1) / kSlice));
   size_t oVec[6];
   for (int k = 0; k < (mixed ? 6 : 4); k++) oVec[k] = A.reserve(w * 3 * nv);
-  const size_t oHalo = mixed ? A.reserve(sizeof(int) * 4 * nv) : 0;  // one-launch PCG
+  const size_t oHalo = mixed ? A.reserve(sizeof(int) * 4 * nv) : 0;  // clusters and the one-launch PCG
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, A.used);
   if (e != cudaSuccess)
@@ -377,6 +377,7 @@ int alloc_precision(hobak_batch_t* B) {
   }
   d.gridHalo = mixed ? carve<int>(base, oHalo) : nullptr;
   B->precMixed = mixed;
+  B->clusterDirty = true;
   B->gridDirty = true;
   return HOBAK_OK;
 }
@@ -636,6 +637,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   const size_t oGridL = A.reserve(sizeof(int2) * kGridCtas);
   const size_t oGridHc = A.reserve(sizeof(int) * (ntilesCap + 1));
   const size_t oGridRw = A.reserve(sizeof(ulonglong2) * grid_row_words());
+  const size_t oClHalo = A.reserve(sizeof(int) * (16 * (size_t)n + kClusterClasses));
   void* base = nullptr;
   cudaError_t e = cudaMalloc(&base, A.used);
   if (e != cudaSuccess)
@@ -713,6 +715,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   B->gridList = carve<int2>(base, oGridL);
   d.gridHaloCount = carve<int>(base, oGridHc);
   d.gridRowWords = carve<ulonglong2>(base, oGridRw);
+  d.clusterHaloCount = carve<int>(base, oClHalo);
   d.anyAniso = anyAniso;
   d.anyArap = anyArap;
   d.anySvdFree = anySvdFree;
@@ -933,12 +936,44 @@ int prepare_cluster_classes(hobak_batch_t* B) {
   CUDA_TRY(cudaStreamSynchronize(B->stream));
   if (!list.empty())
     CUDA_TRY(cudaMemcpy(B->clusterList, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(const_cast<SceneParams*>(B->d.scenes), B->sceneParams.data(), sizeof(SceneParams) * n,
-                      cudaMemcpyHostToDevice));
+  auto upload = [&]() -> int {
+    CUDA_TRY(cudaMemcpy(const_cast<SceneParams*>(B->d.scenes), B->sceneParams.data(), sizeof(SceneParams) * n,
+                        cudaMemcpyHostToDevice));
+    return HOBAK_OK;
+  };
+  for (auto& p : B->sceneParams) p.pcgHalo = 0;
+  if (int rc = upload()) return rc;
   if (!list.empty()) {
-    launch_cluster_gather(B->d, B->stream);
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaStreamSynchronize(B->stream));
+    // the halos, then which classes have room for theirs
+    int* dLargest = B->d.clusterHaloCount + 16 * (size_t)n;
+    int largest[kClusterClasses];
+    std::fill(largest, largest + kClusterClasses, 0x7fffffff);
+    if (mixed) {
+      CUDA_TRY(cudaMemsetAsync(dLargest, 0, sizeof(largest), B->stream));
+      launch_cluster_halo(B->d, dLargest, B->stream);
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaMemcpyAsync(largest, dLargest, sizeof(largest), cudaMemcpyDeviceToHost, B->stream));
+      CUDA_TRY(cudaStreamSynchronize(B->stream));
+    }
+    bool all = true;
+    for (int k = 0; k < kClusterClasses; k++) {
+      ClusterClass& c = B->classes[k];
+      const int halo = largest[k] <= (int)cluster_halo_room(c.vpcMax) ? largest[k] : -1;
+      if (halo != c.halo) changed = true;
+      c.halo = halo;
+      all = all && (c.count == 0 || halo >= 0);
+    }
+    for (int s = 0; s < n; s++) {
+      int k = 0;
+      while (k + 1 < kClusterClasses && sizes[k] < cl[s]) k++;
+      B->sceneParams[s].pcgHalo = cl[s] > 0 && B->classes[k].halo >= 0 ? 1 : 0;
+    }
+    if (int rc = upload()) return rc;
+    if (!all) {
+      launch_cluster_gather(B->d, B->stream);
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaStreamSynchronize(B->stream));
+    }
   }
   if (changed) drop_graphs(B);
   B->clusterDirty = false;

@@ -3,8 +3,8 @@
 // One thread-block cluster solves one scene's linear system from start to
 // finish in a single launch: the scene's vertices are split into CL
 // contiguous ranges, one per CTA; the Krylov vectors of a range live in that
-// CTA's shared memory, the SpMV gathers the search vector of neighbouring
-// ranges from the other CTAs' shared memory (distributed shared memory), and
+// CTA's shared memory, the search vector of neighbouring ranges comes from the
+// other CTAs' shared memory (distributed shared memory), and
 // every dot product is a CTA tree followed by a fixed-order sum of the CL CTA
 // partials read through distributed shared memory.  An iteration is two
 // cluster barriers (the fused reduction after the SpMV, and the publication
@@ -28,7 +28,7 @@
 #include <atomic>
 #include <cfloat>
 
-#include "kernels.cuh"
+#include "pcg_common.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -40,7 +40,8 @@ __device__ __forceinline__ bool finite_d(double x) { return x == x && fabs(x) <=
 
 // Shared memory of one CTA:
 //   [slots: 8 doubles][warp partials: 3 * kClusterWarps doubles][ubase: 16 u32]
-//   [u: 4 * vpc T (x, y, z, 0 per vertex: one vector load per gather)]
+//   [u: 4 * vpc T (x, y, z, 0 per vertex: one vector load per gather), then the
+//    halo's u the same way (haloMax vertices)]
 //   [p, s, w, d, r: 3 * vpc T each]
 constexpr int kSlotBytes = 8 * sizeof(double) + 3 * kClusterWarps * sizeof(double) + 16 * sizeof(uint32_t);
 
@@ -53,7 +54,7 @@ struct ClusterSmem {
 };
 
 template <typename T>
-__device__ __forceinline__ ClusterSmem<T> carve_smem(unsigned char* base, int vpc) {
+__device__ __forceinline__ ClusterSmem<T> carve_smem(unsigned char* base, int vpc, int haloMax) {
   ClusterSmem<T> m;
   m.slots = reinterpret_cast<double*>(base);
   m.warp = reinterpret_cast<T*>(base + 8 * sizeof(double));
@@ -61,7 +62,7 @@ __device__ __forceinline__ ClusterSmem<T> carve_smem(unsigned char* base, int vp
   T* v = reinterpret_cast<T*>(base + kSlotBytes);
   const int n = 3 * vpc;
   m.u = v;
-  m.p = v + 4 * vpc;
+  m.p = v + 4 * (vpc + haloMax);
   m.s = m.p + n;
   m.w = m.s + n;
   m.d = m.w + n;
@@ -82,6 +83,15 @@ __device__ __forceinline__ void ld_u(uint32_t a, double* x) {
   asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "r"(a));
   asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(x[2]), "=d"(pad) : "r"(a + 16));
 }
+// u of a vertex of this CTA or its halo
+__device__ __forceinline__ void local_u(const float* u, int c, float* x) {
+  const float4 t = *reinterpret_cast<const float4*>(u + 4 * c);
+  x[0] = t.x, x[1] = t.y, x[2] = t.z;
+}
+__device__ __forceinline__ void local_u(const double* u, int c, double* x) {
+  const double2 t = *reinterpret_cast<const double2*>(u + 4 * c);
+  x[0] = t.x, x[1] = t.y, x[2] = u[4 * c + 2];
+}
 __device__ __forceinline__ uint32_t map_cluster(const void* p, int rank) {
   uint32_t out;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
@@ -93,6 +103,29 @@ __device__ __forceinline__ double ld_cluster_f64(uint32_t a) {
   double x;
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x) : "r"(a));
   return x;
+}
+
+// FP32: the halo's u (the vertices of other CTAs that this CTA's rows name: list
+// of owner << 20 | local index) copied once from their CTAs' shared memory, so
+// that the row sums gather from this CTA's alone; after a cluster barrier that
+// published u.  A vertex of the halo is named by several rows, and a gather
+// from another CTA goes through the same port as the matrix, which the row sums
+// load at ~32 bytes a cycle and SM, what L2 gives when all SMs ask: at 1,954
+// vertices a CTA they went from 31,200 to 27,200 cycles an iteration.  Steps of
+// 8 to 96 scenes: 1.01x (32 scenes in clusters of 4) to 1.12x (16 scenes of up
+// to 15,625 vertices), 96 scenes 6.73 -> 6.49 ms.  Not in FP64, where the
+// arithmetic covers the gathers: 48 scenes 0.98x with it.
+template <typename T>
+__device__ __forceinline__ void fetch_halo(const ClusterSmem<T>& m, const int* list, int n, int vpc) {
+  constexpr int kUShift = sizeof(T) == 4 ? 4 : 5;
+  for (int i = threadIdx.x; i < n; i += kClusterThreads) {
+    const int c = __ldg(list + i);
+    T x[3];
+    ld_u(m.ubase[c >> 20] + ((uint32_t)(c & 0xFFFFF) << kUShift), x);
+    T* h = m.u + 4 * (vpc + i);
+    h[0] = x[0], h[1] = x[1], h[2] = x[2];
+  }
+  __syncthreads();
 }
 
 // The contact rows of vertex u of w H_coll x (w = collision_lhs_scale of the
@@ -254,12 +287,12 @@ __device__ __forceinline__ void dot2_step(float a, float x, float& s, float& c) 
 // over the cluster (valid in warp 0).  r64 starts as rhs (y = 0), so it is
 // rhs - A y up to FP64 rounding of the updates.  Not inlined: its registers
 // stay out of the PCG loop's allocation.
-template <int CL>
+template <int CL, bool HALO>
 __device__ __noinline__ double sweep_residual(cg::cluster_group& cluster, const ClusterSmem<float>& m, double* y,
                                               double* r64, const int* gather, const int* sliceRow, const int* rowptr,
                                               const float* lhs, int u0, int n, double rsc,
                                               bool contact, ContactRefs coll, const unsigned char* freeMask,
-                                              int v0, int vpc, double collScale) {
+                                              int v0, int vpc, double collScale, const int* halo, int nHalo) {
   for (int lv = threadIdx.x; lv < n; lv += kClusterThreads) {
     const int u = u0 + lv;
 #pragma unroll
@@ -271,6 +304,7 @@ __device__ __noinline__ double sweep_residual(cg::cluster_group& cluster, const 
     m.u[4 * lv + 3] = 0.0f;
   }
   cluster.sync();
+  if (HALO) fetch_halo(m, halo, nHalo, vpc);
   double rl = 0.0;
   for (int lv = threadIdx.x; lv < n; lv += kClusterThreads) {
     const int u = u0 + lv;
@@ -282,7 +316,8 @@ __device__ __noinline__ double sweep_residual(cg::cluster_group& cluster, const 
     for (int j = 0; j < len; j++) {
       const int g = __ldg(G + j * kSlice);
       float x[3];
-      ld_u(m.ubase[g >> 20] + ((uint32_t)(g & 0xFFFFF) << 4), x);
+      if (HALO) local_u(m.u, g, x);
+      else ld_u(m.ubase[g >> 20] + ((uint32_t)(g & 0xFFFFF) << 4), x);
       const float* Bj = B + (size_t)kSlotVals * j;
 #pragma unroll
       for (int i = 0; i < 3; i++)
@@ -300,10 +335,10 @@ __device__ __noinline__ double sweep_residual(cg::cluster_group& cluster, const 
   }
   return cluster_sum_f64<CL>(cluster, m, rl, 7);
 }
-template <int CL>
+template <int CL, bool HALO>
 __device__ double sweep_residual(cg::cluster_group&, const ClusterSmem<double>&, double*, double*, const int*,
                                  const int*, const int*, const double*, int, int, double, bool, ContactRefs,
-                                 const unsigned char*, int, int, double) {
+                                 const unsigned char*, int, int, double, const int*, int) {
   return 0.0;  // FP64: one inner solve is the solve; never called
 }
 
@@ -321,10 +356,11 @@ struct Broadcast {
   int stop;      // 1: the inner solve (or the sweeps) ended; 2: non-finite, the step failed
 };
 
-// Owner CTA and local vertex index of every slot's column for the scenes
-// solved in clusters (gather[slot] = owner << 20 | local index; the owner is
-// the CTA whose range [owner * vpc, (owner + 1) * vpc) holds the column), in
-// the sliced layout of colS.  Built when the cluster assignment changes.
+// The scenes whose row sums gather through distributed shared memory (FP64, or
+// the halo of their class does not fit): owner CTA and local vertex index of
+// every slot's column (gather[slot] = owner << 20 | local index; the owner is the
+// CTA whose range [owner * vpc, (owner + 1) * vpc) holds the column), in the
+// sliced layout of colS.  Built when the cluster assignment changes.
 __global__ void k_cluster_gather(DeviceBatch b, int* __restrict__ gather) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)b.nslotRows * kSlice) return;
@@ -332,6 +368,7 @@ __global__ void k_cluster_gather(DeviceBatch b, int* __restrict__ gather) {
   int g = 0;
   if (u < b.nv) {
     const SceneParams& sp = b.scenes[b.vertexScene[u]];
+    if (sp.pcgCluster > 0 && sp.pcgHalo) return;  // k_cluster_halo
     if (sp.pcgCluster > 0) {
       const int vpc = (sp.nv + sp.pcgCluster - 1) / sp.pcgCluster;
       const int w = b.colS[i] - sp.v0;
@@ -342,10 +379,80 @@ __global__ void k_cluster_gather(DeviceBatch b, int* __restrict__ gather) {
   gather[i] = g;
 }
 
-template <int CL, typename T>
+// A cluster CTA's halo and its slots' columns as indices into the CTA's u (own
+// vertices, then the halo in ascending order): a bit per vertex of the scene,
+// then ranks.  CTA (scene, rank).  largest[class]: the largest halo of the
+// class, INT_MAX where one exceeds its list (four times the CTA's vertices).
+constexpr int kHaloWords = 2048;  // 65,536 vertices: more than 16 CTAs hold
+__global__ void __launch_bounds__(256) k_cluster_halo(DeviceBatch b, int* __restrict__ gather, int* largest) {
+  __shared__ unsigned bits[kHaloWords];
+  __shared__ int rank[kHaloWords];
+  __shared__ int warpTot[8];
+  const int sc = blockIdx.x, r = blockIdx.y, tid = threadIdx.x;
+  const SceneParams& sp = b.scenes[sc];
+  const int CL = sp.pcgCluster;
+  if (r >= CL) return;
+  const int vpc = (sp.nv + CL - 1) / CL, v0 = sp.v0, words = (sp.nv + 31) / 32;
+  const int a = v0 + min(sp.nv, r * vpc), z = v0 + min(sp.nv, (r + 1) * vpc);
+  int cls = 0;
+  while (1 << cls < CL) cls++;
+  if (words > kHaloWords) {
+    if (tid == 0) atomicMax(&largest[cls], 0x7fffffff);
+    return;
+  }
+  for (int i = tid; i < words; i += 256) bits[i] = 0u;
+  __syncthreads();
+  for (int u = a + tid; u < z; u += 256) {
+    const int len = b.rowptr[u + 1] - b.rowptr[u];
+    const size_t cb = col_slot(b, u, 0);
+    for (int j = 0; j < len; j++) {
+      const int w = b.colS[cb + kSlice * j];
+      if (w < a || w >= z) atomicOr(&bits[(w - v0) / 32], 1u << ((w - v0) % 32));
+    }
+  }
+  __syncthreads();
+  const int per = (words + 255) / 256, i0 = min(words, tid * per), i1 = min(words, i0 + per);
+  int mine = 0;
+  for (int i = i0; i < i1; i++) mine += __popc(bits[i]);
+  int x = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (tid % 32 >= o) x += y;
+  }
+  if (tid % 32 == 31) warpTot[tid / 32] = x;
+  __syncthreads();
+  int at = x - mine;
+  for (int i = 0; i < tid / 32; i++) at += warpTot[i];
+  const int cap = 4 * (z - a);
+  int* list = b.gridHalo + 4 * (size_t)a;
+  for (int i = i0; i < i1; i++) {
+    rank[i] = at;
+    for (unsigned m = bits[i]; m; m &= m - 1, at++) {
+      const int l = 32 * i + __ffs(m) - 1, owner = l / vpc;
+      if (at < cap) list[at] = owner << 20 | (l - owner * vpc);
+    }
+  }
+  if (tid == 255) {
+    b.clusterHaloCount[16 * sc + r] = at;
+    atomicMax(&largest[cls], at <= cap ? at : 0x7fffffff);
+  }
+  __syncthreads();
+  for (int u = a + tid; u < z; u += 256) {
+    const int len = b.rowptr[u + 1] - b.rowptr[u];
+    const size_t cb = col_slot(b, u, 0);
+    for (int j = 0; j < len; j++) {
+      const int w = b.colS[cb + kSlice * j], l = w - v0;
+      gather[cb + kSlice * j] =
+          w >= a && w < z ? w - a : vpc + rank[l / 32] + __popc(bits[l / 32] & ((1u << (l % 32)) - 1u));
+    }
+  }
+}
+
+template <int CL, typename T, bool HALO>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
     k_pcg_cluster(DeviceBatch b, PcgVecs<T> v, const int* __restrict__ sceneList,
-                  const int* __restrict__ gather) {
+                  const int* __restrict__ gather, int haloMax) {
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int sc = sceneList[blockIdx.x / CL];
@@ -362,18 +469,21 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
   __shared__ Broadcast<T> bc;
   const int v0 = sp.v0, nvS = sp.nv;
   const int vpc = (nvS + CL - 1) / CL;  // the scene's own split: alone == in any batch
-  const ClusterSmem<T> m = carve_smem<T>(smem, vpc);
+  const ClusterSmem<T> m = carve_smem<T>(smem, vpc, haloMax);
   const int my0 = min(nvS, rank * vpc), my1 = min(nvS, (rank + 1) * vpc);
   const int nmine = my1 - my0;
   // contact on this scene: its rows add w H_coll u (collision_lhs_scale)
   const bool contact = b.collOn && (b.coll.scenes[sc].vfOn || b.coll.scenes[sc].eeOn);
   constexpr int kUShift = sizeof(T) == 4 ? 4 : 5;  // bytes of one u entry: 16 (float4) or 32
+  const int* halo = HALO ? b.gridHalo + 4 * (size_t)(v0 + my0) : nullptr;
+  const int nHalo = HALO ? b.clusterHaloCount[16 * sc + rank] : 0;
   if (threadIdx.x < CL) m.ubase[threadIdx.x] = map_cluster(m.u, threadIdx.x);
 
   // The scene's scalar state, kept by thread 0 of every CTA in shared memory
   // (identical copies, computed from the same cluster sums in the same
   // order); registers stay with the SpMV.
   __shared__ Scalars ss;
+  __shared__ double recip[2];  // of the last iteration's gamma and alpha
   if (t0) {
     ss = Scalars{};
     ss.maxit = st.maxit;
@@ -432,6 +542,10 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
     __syncthreads();
     while (!bc.stop) {
       // ---- w = A u over my vertices; delta = (w, u), gamma = (r, u), |r|^2 ----
+      if (HALO) fetch_halo(m, halo, nHalo, vpc);
+      // (not in FP64: there the pipe is the row sums', and the chain would hold its warp back)
+      if (HALO && threadIdx.x >= kClusterThreads - 2 && ss.iters > 0)
+        recip[kClusterThreads - 1 - threadIdx.x] = 1.0 / (threadIdx.x == kClusterThreads - 1 ? ss.gamma : ss.alpha);
       T dl = T(0), gl = T(0), rl = T(0);
       for (int lv = threadIdx.x; lv < nmine; lv += kClusterThreads) {
         const int u = v0 + my0 + lv;
@@ -456,8 +570,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
           T x[4][3];
   #pragma unroll
           for (int q = 0; q < 4; q++) {
-            const uint32_t a = m.ubase[gq[q] >> 20] + ((uint32_t)(gq[q] & 0xFFFFF) << kUShift);
-            ld_u(a, x[q]);
+            if (HALO) local_u(m.u, gq[q], x[q]);
+            else ld_u(m.ubase[gq[q] >> 20] + ((uint32_t)(gq[q] & 0xFFFFF) << kUShift), x[q]);
           }
   #pragma unroll
           for (int q = 0; q < 4; q++) {
@@ -509,8 +623,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
             ss.beta = 0.0;
             ss.alpha = g / delta;
           } else {
-            ss.beta = g / ss.gamma;
-            ss.alpha = g / (delta - ss.beta * g / ss.alpha);
+            ss.beta = HALO ? divide(g, ss.gamma, recip[0]) : g / ss.gamma;
+            const double q = ss.beta * g;
+            ss.alpha = g / (delta - (HALO ? divide(q, ss.alpha, recip[1]) : q / ss.alpha));
           }
           ss.gammaOld = ss.gamma;
           ss.gamma = g;
@@ -551,11 +666,11 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
     if (sizeof(T) == sizeof(double)) break;  // FP64: the inner solve is the solve
     if (bc.stop == 2) break;                 // non-finite: the step has failed
     // ---- mixed: y += rsc d, r64 -= rsc A d, |r64|^2 ----
-    const double s64 = sweep_residual<CL>(cluster, m, b.y, b.r64, gather, b.sliceRow, b.rowptr, v.lhs, v0 + my0,
+    const double s64 = sweep_residual<CL, HALO>(cluster, m, b.y, b.r64, gather, b.sliceRow, b.rowptr, v.lhs, v0 + my0,
                                           nmine, rsc, contact,
                                           ContactRefs{b.coll.incCount, b.coll.incList, b.coll.pairTet, b.coll.pairC,
                                                       b.coll.pairG},
-                                          b.freeMask, v0, vpc, contact ? collision_lhs_scale(b, sc) : 0.0);
+                                          b.freeMask, v0, vpc, contact ? collision_lhs_scale(b, sc) : 0.0, halo, nHalo);
     if (t0) {
       // the outer test (tile path: k_residual)
       ss.sweep += 1;
@@ -616,42 +731,51 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
   cluster.sync();
 }
 
+// Shared memory a cluster kernel may have; kClusterSmemMax bounds the vectors
+// alone (which decides the scenes' cluster sizes), the halo takes what is left.
+constexpr size_t kClusterSmemAll = 224 * 1024;
+
 template <int CL, typename T>
 int launch_class(const DeviceBatch& b, const PcgVecs<T>& v, const ClusterClass& c, cudaStream_t s) {
   if (c.count == 0) return 0;
   const size_t smem = kSlotBytes + cluster_vertex_bytes(sizeof(T) == 4) * c.vpcMax;
-  k_pcg_cluster<CL, T><<<c.count * CL, kClusterThreads, smem, s>>>(b, v, c.scenes, b.clusterGather);
+  if (sizeof(T) == sizeof(float) && c.halo >= 0)
+    k_pcg_cluster<CL, float, true><<<c.count * CL, kClusterThreads, smem + sizeof(float4) * c.halo, s>>>(
+        b, b.v32, c.scenes, b.clusterGather, c.halo);
+  else
+    k_pcg_cluster<CL, T, false><<<c.count * CL, kClusterThreads, smem, s>>>(b, v, c.scenes, b.clusterGather, 0);
   return 0;
 }
 
-template <int CL, typename T>
-cudaError_t allow_smem() {
-  cudaError_t e = cudaFuncSetAttribute(k_pcg_cluster<CL, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kClusterSmemMax);
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kernel, int CL) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmemAll);
   if (e == cudaSuccess && CL > 8)  // 16-CTA clusters are a non-portable size
-    e = cudaFuncSetAttribute(k_pcg_cluster<CL, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+template <int CL>
+cudaError_t allow_smem() {
+  cudaError_t e = allow_smem(k_pcg_cluster<CL, float, true>, CL);
+  if (e == cudaSuccess) e = allow_smem(k_pcg_cluster<CL, float, false>, CL);
+  if (e == cudaSuccess) e = allow_smem(k_pcg_cluster<CL, double, false>, CL);
   return e;
 }
 
 }  // namespace
 
-// Opt every cluster kernel into kClusterSmemMax bytes of dynamic shared
+// Opt every cluster kernel into kClusterSmemAll bytes of dynamic shared
 // memory (once per process; outside any stream capture; batches may be
 // created and stepped from several host threads).
 int configure_cluster_pcg() {
   static std::atomic<int> done{0};
   if (done.load()) return 0;
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = allow_smem<1, float>();
-  if (e == cudaSuccess) e = allow_smem<2, float>();
-  if (e == cudaSuccess) e = allow_smem<4, float>();
-  if (e == cudaSuccess) e = allow_smem<8, float>();
-  if (e == cudaSuccess) e = allow_smem<16, float>();
-  if (e == cudaSuccess) e = allow_smem<1, double>();
-  if (e == cudaSuccess) e = allow_smem<2, double>();
-  if (e == cudaSuccess) e = allow_smem<4, double>();
-  if (e == cudaSuccess) e = allow_smem<8, double>();
-  if (e == cudaSuccess) e = allow_smem<16, double>();
+  if (e == cudaSuccess) e = allow_smem<1>();
+  if (e == cudaSuccess) e = allow_smem<2>();
+  if (e == cudaSuccess) e = allow_smem<4>();
+  if (e == cudaSuccess) e = allow_smem<8>();
+  if (e == cudaSuccess) e = allow_smem<16>();
   if (e != cudaSuccess) return (int)e;
   done.store(1);
   return 0;
@@ -666,6 +790,13 @@ void launch_cluster_gather(const DeviceBatch& b, cudaStream_t s) {
   k_cluster_gather<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b, b.clusterGather);
 }
 size_t cluster_fixed_bytes() { return kSlotBytes; }
+size_t cluster_halo_room(int vpcMax) {
+  const size_t used = kSlotBytes + cluster_vertex_bytes(true) * vpcMax;
+  return used < kClusterSmemAll ? (kClusterSmemAll - used) / sizeof(float4) : 0;
+}
+void launch_cluster_halo(const DeviceBatch& b, int* largest, cudaStream_t s) {
+  k_cluster_halo<<<dim3((unsigned)b.nscenes, 16), 256, 0, s>>>(b, b.clusterGather, largest);
+}
 
 template <typename T>
 int launch_cluster_pcg(const DeviceBatch& b, const PcgVecs<T>& v, const ClusterClass* classes, int k, cudaStream_t s) {

@@ -51,6 +51,7 @@ struct SceneParams {
   int kind;            // material
   int active;          // 0: the scene is parked (serving) and every kernel skips it
   int pcgCluster;      // > 0: the inner PCG runs in a cluster of this many CTAs (cluster_pcg.cu)
+  int pcgHalo;         // ... whose CTAs keep a copy of their halo's u
   int integrator;      // kIntegratorVelocity or kIntegratorPosition
   double mu, lambda, alpha;  // reparameterised material constants
   double dt;

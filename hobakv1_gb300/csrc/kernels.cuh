@@ -34,6 +34,7 @@ constexpr int kClusterSmemMax = 200 * 1024;  // dynamic shared memory per CTA, a
 struct ClusterClass {
   int count;          // scenes of this cluster size
   int vpcMax;         // largest vertices per CTA among them (shared-memory sizing)
+  int halo;           // most halo vertices of a CTA; -1: they do not fit, gathers go to their CTAs
   const int* scenes;  // device list of their scene ids
 };
 
@@ -166,12 +167,13 @@ struct DeviceBatch {
   int gridTilesCap;
   int gridOn;  // the tile-path scenes take that path (2: pcg_rows.cu)
   ulonglong2* gridRowWords;  // [2][CTAs][9] partials of pcg_rows.cu
-  // FP32: per CTA the vertices of other CTAs that its rows' columns name (at
-  // 4 x its first vertex), their number (per tile: a CTA's is its first
-  // tile's), and every column as the CTA's own index of it (k_grid_halo; the
-  // slots of clusterGather, which only cluster scenes use otherwise)
+  // FP32 (pcg_grid.cu and clusters): per CTA the vertices of other CTAs that its
+  // rows' columns name (at 4 x its first vertex), their number (per tile: a
+  // CTA's is its first tile's), and every column as the CTA's own index of it
+  // (k_grid_halo, k_cluster_halo; the slots of clusterGather)
   int* gridHalo;
   int* gridHaloCount;
+  int* clusterHaloCount;  // cluster scenes' halos (lists in gridHalo): [scene][16]
   double* psi;          // [T] energy density scratch
   int anyAniso;          // some scene has an anisotropic energy (k_element_aniso)
   int anyArap, anySvdFree;  // some scene has ARAP / another isotropic energy (mixed element kernels)
@@ -302,5 +304,9 @@ int configure_cluster_pcg();
 // Shared memory a cluster CTA needs: fixed part + per-vertex part.
 size_t cluster_vertex_bytes(bool mixed);
 size_t cluster_fixed_bytes();
+// FP32: halo lists and columns of the cluster scenes; largest: five device words,
+// one per class.  Halo vertices that fit beside vpcMax vertices.
+void launch_cluster_halo(const DeviceBatch& b, int* largest, cudaStream_t s);
+size_t cluster_halo_room(int vpcMax);
 
 }  // namespace hobak

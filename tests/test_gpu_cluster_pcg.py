@@ -194,3 +194,25 @@ def test_contact_in_a_cluster_with_the_other_integrators(integrator):
 
     xc, xt = run_path(True), run_path(False)
     assert rel(xc, xt) < 1e-9, rel(xc, xt)
+
+
+@pytest.mark.parametrize("N", [12, 24, 30])  # 138, 977 and 1,862 vertices a CTA
+def test_gathers_from_the_halo_and_from_the_other_ctas_give_the_same_bits(N):
+    """FP32 clusters copy their halo once per iteration; beside a scene whose
+    halo has no room in shared memory (42,875 vertices: 2,680 a CTA) the whole
+    class gathers from the other CTAs instead.  Same arithmetic, same bits."""
+    s = scenes.config2_scene(N, "snh")
+    rng = np.random.default_rng(N)
+    s.v0 = rng.normal(size=s.rest.shape) * 0.1
+    s.v0[s.pinned] = 0.0
+    out = []
+    for group in ([s], [s, scenes.config2_scene(34, "arap")]):
+        b = hobak.BATCH(group, hobak.solver_opts(precision=hobak.PRECISION_MIXED))
+        b.set_tuning(cluster_pcg=1)
+        b.set_scene_cluster(0, 16)
+        assert (b.pcg_path() == 16).all()
+        st = b.step(2)[0]
+        out.append((st, *b.get_state(0)))
+        b.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
