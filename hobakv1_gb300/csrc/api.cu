@@ -287,6 +287,9 @@ void set_integrator(SceneParams& p, const hobak_solver_opts& o) {
   p.nm[3] = gamma / (beta * dt);
   p.nm[4] = 1.0 - gamma / beta;
   p.nm[5] = (1.0 - gamma / (2.0 * beta)) * dt;
+  p.invDt = 1.0 / dt;
+  p.lhsK = o.integrator == HOBAK_INTEGRATOR_VELOCITY ? -(dt * dt) : -1.0;
+  p.lhsK0 = -(p.rayBeta * p.invDt);
   p.newtonEps = o.newton_tolerance;
   p.maxNewton = o.max_newton;
 }
@@ -384,7 +387,7 @@ int alloc_precision(hobak_batch_t* B) {
 
 int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   // ---- host precompute ----
-  std::vector<int> vtxptr, vtxinc, rowptr, cols, blkRow, blkptr, blksrc, tileScene, tileV0, tileV1;
+  std::vector<int> vtxptr, vtxinc, rowptr, cols, blkMirror, blkptr, blksrc, tileScene, tileV0, tileV1;
   std::vector<int> tetScene, vertexScene;
   std::vector<double> rest, x, v, fext, mass, pinTarget, DmInv, vol;
   std::vector<SceneParams> sparams;
@@ -516,9 +519,14 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   }
   for (int u = nv; u < nslices * kSlice; u++)  // lanes past the last vertex
     for (int r = sliceRow[u / kSlice]; r < sliceRow[u / kSlice + 1]; r++) colS[(size_t)r * kSlice + u % kSlice] = 0;
-  blkRow.resize(nblocks);
-  for (int u = 0; u < nv; u++)
-    for (int k = rowptr[u]; k < rowptr[u + 1]; k++) blkRow[k] = u;
+  // slot row of block (w, u) for every block (u, w): the rows name u in ascending order of u
+  blkMirror.resize(nblocks);
+  {
+    std::vector<int> seen(nv, 0);
+    for (int u = 0; u < nv; u++)
+      for (int k = rowptr[u]; k < rowptr[u + 1]; k++)
+        blkMirror[k] = sliceRow[cols[k] / kSlice] + seen[cols[k]]++;
+  }
   // block <- (tet, a, b) contributions in ascending tet order
   {
     std::vector<int> where(16 * (size_t)nt);
@@ -615,7 +623,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   const size_t oStageLocal = A.reserve(4 * (size_t)nt);
   const size_t oVol = A.reserve(sizeof(double) * nt), oTS = A.reserve(sizeof(int) * nt);
   const size_t oRowptr = A.reserve(sizeof(int) * (nv + 1)), oCols = A.reserve(sizeof(int) * nblocks);
-  const size_t oBlkRow = A.reserve(sizeof(int) * nblocks), oBlkptr = A.reserve(sizeof(int) * (nblocks + 1));
+  const size_t oBlkMirror = A.reserve(sizeof(int) * nblocks), oBlkptr = A.reserve(sizeof(int) * (nblocks + 1));
   const size_t oBlksrc = A.reserve(sizeof(int) * 16 * (size_t)nt);
   const size_t oVtxptr = A.reserve(sizeof(int) * (nv + 1)), oVtxinc = A.reserve(sizeof(int) * 4 * (size_t)nt);
   const size_t oSliceRow = A.reserve(sizeof(int) * (nslices + 1)), oSlotSlice = A.reserve(sizeof(int) * nslotRows);
@@ -686,7 +694,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   d.tetScene = carve<int>(base, oTS);
   d.rowptr = carve<int>(base, oRowptr);
   d.cols = carve<int>(base, oCols);
-  d.blkRow = carve<int>(base, oBlkRow);
+  d.blkMirror = carve<int>(base, oBlkMirror);
   d.blkptr = carve<int>(base, oBlkptr);
   d.blksrc = carve<int>(base, oBlksrc);
   d.vtxptr = carve<int>(base, oVtxptr);
@@ -743,7 +751,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   CUDA_TRY(up(d.tetScene, tetScene.data(), sizeof(int) * nt));
   CUDA_TRY(up(d.rowptr, rowptr.data(), sizeof(int) * (nv + 1)));
   CUDA_TRY(up(d.cols, cols.data(), sizeof(int) * nblocks));
-  CUDA_TRY(up(d.blkRow, blkRow.data(), sizeof(int) * nblocks));
+  CUDA_TRY(up(d.blkMirror, blkMirror.data(), sizeof(int) * nblocks));
   CUDA_TRY(up(d.blkptr, blkptr.data(), sizeof(int) * (nblocks + 1)));
   CUDA_TRY(up(d.blksrc, blksrc.data(), sizeof(int) * 16 * (size_t)nt));
   CUDA_TRY(up(d.vtxptr, vtxptr.data(), sizeof(int) * (nv + 1)));

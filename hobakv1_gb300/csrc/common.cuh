@@ -56,6 +56,7 @@ struct SceneParams {
   double mu, lambda, alpha;  // reparameterised material constants
   double dt;
   double rayAlpha, rayBeta;  // Rayleigh damping C = rayAlpha M + rayBeta K0 (position integrator)
+  double invDt, lhsK, lhsK0;  // 1 / dt and the LHS's factors of the elements' K and of K0
   double nm[6];              // Newmark coefficients alpha_0..5 (NEWMARK.cpp:71-76) from dt
   double newtonEps;          // Newmark: Newton stops once |rhs|^2 <= newtonEps ...
   int maxNewton;             // ... or after maxNewton iterations

@@ -115,7 +115,7 @@ struct DeviceBatch {
   // block sparsity
   const int* rowptr;
   const int* cols;
-  const int* blkRow;
+  const int* blkMirror;  // block (u, w) -> slot row of (w, u)
   const int* blkptr;  // block <- contributions
   const int* blksrc;  // tet*16 + a*4 + b
   const int* vtxptr;  // vertex <- incidences

@@ -167,6 +167,9 @@ __device__ __forceinline__ HT gather_block_entry(const DeviceBatch& b, const HT*
   return sum;
 }
 
+// 0 + x without an add: -0 becomes +0 (the FP64 pipe takes 19 cycles for the add).
+__device__ __forceinline__ double plus_zero(double x) { return (__double_as_longlong(x) << 1) == 0 ? 0.0 : x; }
+
 // Slot of the sliced LHS -> CSR block: slot row r, lane -> vertex u, block
 // k = rowptr[u] + j; false for padding slots and lanes past the last vertex.
 __device__ __forceinline__ bool slot_block(const DeviceBatch& b, int r, int lane, int& u, int& k) {
@@ -183,37 +186,67 @@ __device__ __forceinline__ bool slot_block(const DeviceBatch& b, int r, int lane
 // FP64 assembly: one thread per (slot, entry), entries of a slot on nine
 // neighbouring lanes, so the nine entries of a contribution (72 contiguous
 // bytes) are read in one request; at FP64 width this coalescing beats a
-// thread per block.
+// thread per block.  The matrix is symmetric to the bit (block (w, u) sums the
+// transposes of block (u, w)'s terms in the same order), so only the slots with
+// w >= u are summed and each is written twice.  The adds were what bounded this
+// kernel: 136 an entry and vertex of a Kuhn mesh with lists padded to eights
+// (an add takes the FP64 pipe 19 cycles a warp whatever its lanes do), 61 now.
+// 384,000 tets, FP64: 250 -> 132 us (read and write once: 53 us); 48 scenes
+// 977 -> 515 us.  What is left is the latency of the chain of lookups.
 template <typename HT, typename T>
 __global__ void k_assemble_entry(DeviceBatch b, const HT* __restrict__ elemH, T* __restrict__ lhs) {
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (size_t)kSlotVals * b.nslotRows) return;
   const int r = (int)(g / kSlotVals), rem = (int)(g % kSlotVals);
   const int lane = rem / 9, e = rem % 9;
+  const int w = __ldg(&b.colS[(size_t)r * kSlice + lane]);
   int u, blk;
-  if (!slot_block(b, r, lane, u, blk)) return;
-  if (!b.scenes[b.vertexScene[u]].active || b.solve[b.vertexScene[u]].newtonDone) return;
-  const int rr = e / 3, c = e % 3;
-  const HT sum = gather_block_entry(b, elemH, blk, rr, c);
-  const int w = b.cols[blk];
+  if (w < kSlice * __ldg(&b.slotSlice[r]) + lane || !slot_block(b, r, lane, u, blk)) return;
   const SceneParams& sp = b.scenes[b.vertexScene[u]];
-  const double dt = sp.dt;
+  if (!sp.active || b.solve[b.vertexScene[u]].newtonDone) return;
+  const int rr = e / 3, c = e % 3;
+  // the terms in list order (ascending tet), two at a time with the next two
+  // loaded ahead: no add is issued for a term that is not there
+  const int k1 = b.blkptr[blk + 1];
+  const int eT = 3 * c + rr;
+  auto source = [&](int k) { return k < k1 ? __ldg(&b.blksrc[k]) : -1; };
+  auto value = [&](int src) {
+    if (src < 0) return HT(0);
+    const int ea = (src >> 2) & 3, eb = src & 3;
+    return elemH[(size_t)kElemHessStride * (src >> 4) +
+                 (ea <= eb ? 9 * upper_block(ea, eb) + e : 9 * upper_block(eb, ea) + eT)];
+  };
+  int k = b.blkptr[blk];
+  HT a0 = value(source(k)), a1 = value(source(k + 1));
+  HT n0 = value(source(k + 2)), n1 = value(source(k + 3));
+  int s0 = source(k + 4), s1 = source(k + 5);
+  HT sum = plus_zero(a0);
+  if (k + 1 < k1) sum += a1;
+#pragma unroll 1
+  for (k += 2; k < k1; k += 2) {
+    a0 = n0, a1 = n1;
+    n0 = value(s0), n1 = value(s1);
+    s0 = source(k + 4), s1 = source(k + 5);
+    sum += a0;
+    if (k + 1 < k1) sum += a1;
+  }
   const bool fu = b.freeMask[u] != 0, fw = b.freeMask[w] != 0;
-  HT val;
-  if (sp.integrator == kIntegratorPosition) {
-    // A = M (1/dt^2 - alpha/dt) - (beta/dt) K0 - K (BACKWARD_EULER_POSITION.cpp:207)
-    const double invDt = 1.0 / dt;
-    val = (fu && fw) ? HT(-(sp.rayBeta * invDt)) * HT(b.K0[9 * (size_t)blk + rr + 3 * c]) - sum : HT(0);
-    if (u == w && rr == c) val += fu ? HT(b.mass[u] * (invDt * invDt - sp.rayAlpha * invDt)) : HT(1);
-  } else if (sp.integrator == kIntegratorNewmark) {
-    // A = alpha_0 M - K (NEWMARK.cpp:262; its C is zeroed before use)
-    val = (fu && fw) ? -sum : HT(0);
-    if (u == w && rr == c) val += fu ? HT(sp.nm[0] * b.mass[u]) : HT(1);
-  } else {
-    val = (fu && fw) ? HT(-(dt * dt)) * sum : HT(0);
-    if (u == w && rr == c) val += fu ? HT(b.mass[u]) : HT(1);
+  const bool position = sp.integrator == kIntegratorPosition;
+  // A = S (w M + k0 K0 + k K) S + (I - S), its factors from the integrator:
+  // M - dt^2 K; M (1/dt^2 - alpha/dt) - (beta/dt) K0 - K (BACKWARD_EULER_POSITION.cpp:207);
+  // alpha_0 M - K (NEWMARK.cpp:262; its C is zeroed before use)
+  HT val = HT(0);
+  if (fu && fw) val = position ? HT(sp.lhsK0) * HT(b.K0[9 * (size_t)blk + rr + 3 * c]) - sum : HT(sp.lhsK) * sum;
+  if (u == w && rr == c) {
+    if (position)
+      val += fu ? HT(b.mass[u] * (sp.invDt * sp.invDt - sp.rayAlpha * sp.invDt)) : HT(1);
+    else if (sp.integrator == kIntegratorNewmark)
+      val += fu ? HT(sp.nm[0] * b.mass[u]) : HT(1);
+    else
+      val += fu ? HT(b.mass[u]) : HT(1);
   }
   lhs[(size_t)r * kSlotVals + kSlice * e + lane] = T(val);
+  if (u != w) lhs[(size_t)b.blkMirror[blk] * kSlotVals + kSlice * eT + w % kSlice] = T(val);
 }
 
 // FP32 assembly: one thread per slot (a warp per slot row of 32 vertices):
@@ -222,6 +255,9 @@ __global__ void k_assemble_entry(DeviceBatch b, const HT* __restrict__ elemH, T*
 // contribution is 9 contiguous values: a 3x3 block of one element Hessian,
 // transposed for the lower triangle), then LHS block = S(M - dt^2 K)S + (I - S)
 // written entry by entry, each entry of the warp's 32 slots one 128-byte line.
+// Only the slots with w >= u are summed, and written twice (k_assemble_entry):
+// 384,000 tets 86 -> 68 us, 96 scenes 468 -> 363 us (k_assemble_entry in FP32:
+// 124 and 795 us).
 // Blocks of parked scenes keep their old values.  The gathers are latency
 // bound, so registers are capped at 64 (no spills) for 32 resident warps per
 // SM instead of 28; the cap also keeps every tunable CTA size (up to 1024
@@ -231,8 +267,9 @@ __global__ void __maxnreg__(64) k_assemble(DeviceBatch b, const HT* __restrict__
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (size_t)kSlice * b.nslotRows) return;
   const int r = (int)(g / kSlice), lane = (int)(g % kSlice);
+  const int w = __ldg(&b.colS[g]);
   int u, blk;
-  if (slot_block(b, r, lane, u, blk)) {
+  if (w >= kSlice * __ldg(&b.slotSlice[r]) + lane && slot_block(b, r, lane, u, blk)) {
     const SceneParams& sp = b.scenes[b.vertexScene[u]];
     if (sp.active && !b.solve[b.vertexScene[u]].newtonDone) {
       HT sum[9];
@@ -286,39 +323,33 @@ __global__ void __maxnreg__(64) k_assemble(DeviceBatch b, const HT* __restrict__
 #pragma unroll
             for (int e = 0; e < 9; e++) sum[e] += val[q][e];
       }
-      const int w = b.cols[blk];
-      const double dt = sp.dt;
       const bool fu = b.freeMask[u] != 0, fw = b.freeMask[w] != 0;
       T* out = lhs + (size_t)r * kSlotVals + lane;
+      T* mirror = lhs + (size_t)b.blkMirror[blk] * kSlotVals + w % kSlice;
+      auto put = [&](int e, HT val) {
+        out[kSlice * e] = T(val);
+        if (u != w) mirror[kSlice * (3 * (e % 3) + e / 3)] = T(val);
+      };
       if (sp.integrator == kIntegratorPosition) {
         // A = M (1/dt^2 - alpha/dt) - (beta/dt) K0 - K (BACKWARD_EULER_POSITION.cpp:207)
-        const double invDt = 1.0 / dt;
-        const HT m = fu ? HT(b.mass[u] * (invDt * invDt - sp.rayAlpha * invDt)) : HT(1);
-        const HT cK0 = HT(-(sp.rayBeta * invDt));
+        const HT m = fu ? HT(b.mass[u] * (sp.invDt * sp.invDt - sp.rayAlpha * sp.invDt)) : HT(1);
+        const HT cK0 = HT(sp.lhsK0);
         const double* K0 = b.K0 + 9 * (size_t)blk;
 #pragma unroll
         for (int e = 0; e < 9; e++) {
           HT val = (fu && fw) ? cK0 * HT(K0[(e / 3) + 3 * (e % 3)]) - sum[e] : HT(0);
           if (u == w && e % 4 == 0) val += m;
-          out[kSlice * e] = T(val);
-        }
-      } else if (sp.integrator == kIntegratorNewmark) {
-        // A = alpha_0 M - K (NEWMARK.cpp:262; its C is zeroed before use)
-        const HT m = fu ? HT(sp.nm[0] * b.mass[u]) : HT(1);
-#pragma unroll
-        for (int e = 0; e < 9; e++) {
-          HT val = (fu && fw) ? -sum[e] : HT(0);
-          if (u == w && e % 4 == 0) val += m;
-          out[kSlice * e] = T(val);
+          put(e, val);
         }
       } else {
-        const HT m = fu ? HT(b.mass[u]) : HT(1);
-        const HT ndt2 = HT(-(dt * dt));
+        // M - dt^2 K, or Newmark's alpha_0 M - K (NEWMARK.cpp:262; its C is zeroed before use)
+        const HT m = !fu ? HT(1) : sp.integrator == kIntegratorNewmark ? HT(sp.nm[0] * b.mass[u]) : HT(b.mass[u]);
+        const HT cK = HT(sp.lhsK);
 #pragma unroll
         for (int e = 0; e < 9; e++) {
-          HT val = (fu && fw) ? ndt2 * sum[e] : HT(0);
+          HT val = (fu && fw) ? cK * sum[e] : HT(0);
           if (u == w && e % 4 == 0) val += m;
-          out[kSlice * e] = T(val);
+          put(e, val);
         }
       }
     }
