@@ -57,9 +57,6 @@ __device__ __forceinline__ void reduced_hessian(const MatParams& m, const IT* Ud
     L[6] = L3[0];
     L[7] = L3[1];
     L[8] = L3[2];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 9; k++) Q3[k] = (k % 4 == 0) ? T(1) : T(0);
   }
   // B(a, m) = sum_j DmInv(a, j) V(j, m), computed in T; U in T
   T U[9], B[9], Dt[9], Vt[9];
@@ -95,6 +92,12 @@ __device__ __forceinline__ void reduced_hessian(const MatParams& m, const IT* Ud
 #pragma unroll
         for (int c = 0; c < 3; c++)
           w[3 * a + c] = rs2 * (U[c + 3 * j] * B[a + 3 * i] + sgn * U[c + 3 * i] * B[a + 3 * j]);
+    } else if (!scalingMatrix) {  // the axes: the sum below with Q3 = I (ARAP, 40^3: 1,025 -> 965 us)
+      const int kk = k - 6;
+#pragma unroll
+      for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) w[3 * a + c] = U[c + 3 * kk] * B[a + 3 * kk];
     } else {
       const int kk = k - 6;
 #pragma unroll
@@ -270,9 +273,13 @@ __device__ __forceinline__ bool evaluates(int kind) {
 }
 
 template <typename HT, int KC>
-// FP32 Hessians fit 128 registers (4 CTAs per SM); the FP64 variant needs
-// ~208 and spills heavily below that.
-__global__ void __launch_bounds__(128, sizeof(HT) == 4 ? 4 : 1)
+// FP32 is bound by latency (the FP64 pipe is 59% busy with F, the stress and
+// the force, 16 warps an SM): six CTAs per SM at 80 registers, though they
+// spill ~500 bytes, take 177 us for 384,000 SNH tets where four at 128 took
+// 204 and five at 96 took 184; 96 scenes 1,224 -> 1,203 us.  FP64 is bound by its
+// pipe (88% busy at 8 warps an SM): 168 registers and 12 warps gain nothing
+// over the 216 it takes when left alone.
+__global__ void __launch_bounds__(128, sizeof(HT) == 4 ? 6 : 1)
     k_element(DeviceBatch b, int rawForces, HT* __restrict__ outH) {
   // The CTA's tets read their corners from shared memory: the distinct
   // vertices of its one or two staging blocks (host-built, ascending ids)
@@ -326,13 +333,21 @@ __global__ void __launch_bounds__(128, sizeof(HT) == 4 ? 4 : 1)
     for (int i = 0; i < 3; i++) X[a][i] = sx[a][i];
   double F[9], P[9], f[12];
   deformation_gradient(X, Dinv, F);
+  // FP32: the force waits in shared memory while the Hessian takes the registers
+  double* parked = stage + 6 * b.stageMax + threadIdx.x;
+  auto park = [&](const double* f) {
+#pragma unroll
+    for (int k = 0; k < 12; k++) parked[k * blockDim.x] = f[k];
+    asm volatile("" ::: "memory");  // (or the values stay in registers all the same)
+  };
   HT Hr[45];
   if (KC == kElemSvdFree) {
-    float U[9], S[3], V[9];
-    svd3_rv_f32(F, U, S, V);
     material_pk1_of_F(m, F, P);
     // dt f directly (the force scaled by dt * vol instead of vol)
     element_force(P, Dinv, velocityTerm ? dt * vol : vol, f);
+    park(f);
+    float U[9], S[3], V[9];
+    svd3_rv_f32(F, U, S, V);
     reduced_hessian<HT, float>(m, U, S, V, Dinv, Hr);
   } else if (KC == kElemArap) {
     // the FP32 factors feed the FP32 Hessian; the stress's rotation is
@@ -352,6 +367,7 @@ __global__ void __launch_bounds__(128, sizeof(HT) == 4 ? 4 : 1)
 #pragma unroll
     for (int k = 0; k < 9; k++) P[k] = 2.0 * m.mu * (F[k] - R[k]);
     element_force(P, Dinv, velocityTerm ? dt * vol : vol, f);
+    park(f);
     reduced_hessian<HT, float>(m, U, S, V, Dinv, Hr);
   } else {
     double U[9], S[3], V[9];
@@ -362,6 +378,10 @@ __global__ void __launch_bounds__(128, sizeof(HT) == 4 ? 4 : 1)
   }
 
   double* g = b.elemG + 12 * (size_t)t;
+  if (KC != kElemAll) {
+#pragma unroll
+    for (int k = 0; k < 12; k++) f[k] = parked[k * blockDim.x];
+  }
   if (!velocityTerm) {
     store12(g, f);
     store_blocks<HT, HT>(Hr, vol, outH + kElemHessStride * (size_t)t);
@@ -752,12 +772,15 @@ static int element_cta(int n, int most) {
   return cta;
 }
 
-static size_t stage_bytes(const DeviceBatch& b) { return sizeof(double) * 6 * (size_t)b.stageMax; }
+// threads: those that park their force there
+static size_t stage_bytes(const DeviceBatch& b, int threads) {
+  return sizeof(double) * (6 * (size_t)b.stageMax + 12 * threads);
+}
 
 void launch_element(const DeviceBatch& b, cudaStream_t s, int rawForces) {
   if (b.nt == 0) return;
   const int nt = element_cta(b.nt, b.elemThreads);
-  k_element<double, kElemAll><<<(b.nt + nt - 1) / nt, nt, stage_bytes(b), s>>>(b, rawForces, b.elemH);
+  k_element<double, kElemAll><<<(b.nt + nt - 1) / nt, nt, stage_bytes(b, 0), s>>>(b, rawForces, b.elemH);
   if (b.anyAniso) k_element_aniso<double><<<(b.nt + 127) / 128, 128, 0, s>>>(b, rawForces, b.elemH);
 }
 
@@ -765,8 +788,8 @@ void launch_element_mixed(const DeviceBatch& b, cudaStream_t s) {
   if (b.nt == 0) return;
   const int nt = element_cta(b.nt, b.elemThreads);
   if (b.anySvdFree)
-    k_element<float, kElemSvdFree><<<(b.nt + nt - 1) / nt, nt, stage_bytes(b), s>>>(b, 0, b.elemHf);
-  if (b.anyArap) k_element<float, kElemArap><<<(b.nt + nt - 1) / nt, nt, stage_bytes(b), s>>>(b, 0, b.elemHf);
+    k_element<float, kElemSvdFree><<<(b.nt + nt - 1) / nt, nt, stage_bytes(b, nt), s>>>(b, 0, b.elemHf);
+  if (b.anyArap) k_element<float, kElemArap><<<(b.nt + nt - 1) / nt, nt, stage_bytes(b, nt), s>>>(b, 0, b.elemHf);
   if (b.anyAniso) k_element_aniso<float><<<(b.nt + 127) / 128, 128, 0, s>>>(b, 0, b.elemHf);
 }
 

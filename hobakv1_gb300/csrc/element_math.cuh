@@ -20,11 +20,13 @@ __device__ __forceinline__ double det3(const double* A) {
 // Sort A's (orthogonal) columns by norm, form U = A / sigma (completing
 // vanishing columns), and fold reflections into S[2] (svd_rv convention).
 __device__ __forceinline__ void svd3_finish(double* A, double* U, double* S, double* V) {
+  bool odd = false;  // swaps; V comes in as a product of rotations
   double n[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) n[k] = A[3 * k] * A[3 * k] + A[3 * k + 1] * A[3 * k + 1] + A[3 * k + 2] * A[3 * k + 2];
   // sort columns by norm, descending (3-element network, swaps A and V columns)
   auto swapcols = [&](int a, int b) {
+    odd = !odd;
     double tn = n[a];
     n[a] = n[b];
     n[b] = tn;
@@ -83,7 +85,7 @@ __device__ __forceinline__ void svd3_finish(double* A, double* U, double* S, dou
     U[6] = -U[6]; U[7] = -U[7]; U[8] = -U[8];
     S[2] = -S[2];
   }
-  if (det3(V) < 0.0) {
+  if (odd) {  // det V < 0
     V[6] = -V[6]; V[7] = -V[7]; V[8] = -V[8];
     S[2] = -S[2];
   }
@@ -433,7 +435,8 @@ __device__ __forceinline__ void eig3sym(const T* Ain, T* Q, T* L) {
       T app = (p == 0) ? a00 : a11;
       T aqq = (q == 1) ? a11 : a22;
       const T theta = (aqq - app) / (T(2) * apq);
-      const T t = copysign(T(1), theta) / (fabs(theta) + sqrt(theta * theta + T(1)));
+      // 1 / x takes fewer FP64 instructions than a quotient: 40^3 SNH 1.365 -> 1.341 ms with it
+      const T t = copysign(T(1) / (fabs(theta) + sqrt(theta * theta + T(1))), theta);
       const T c = T(1) / sqrt(t * t + T(1)), s = t * c;
       // rotate: the remaining index m is the third one
       if (r == 0) {  // (0,1), m = 2
