@@ -14,8 +14,8 @@
 // y update, the residual update r -= A d in compensated FP32 and the outer
 // FP64 test, then the next inner solve, until the test passes.  A scene in
 // contact adds its rows' contact terms from the step's pair lists.  The tile
-// path (solver.cu: two grid-wide kernels per iteration, each ending in a
-// ticketed reduction) remains for scenes too large for a cluster.
+// path (pcg_grid.cu, pcg_rows.cu or solver.cu's loop of two grid-wide kernels)
+// remains for scenes too large for a cluster.
 //
 // The iteration is the same Chronopoulos-Gear PCG as the tile path, with the
 // same scalars, stopping rules and iteration accounting (ConjugateGradient.h

@@ -20,6 +20,8 @@
 // The test on |r_k|^2 thus runs at the start of iteration k rather than at
 // the end of k - 1: same decision, same iterates and iteration count; a
 // stopping scene computes one SpMV it does not use.
+// Where a batch's tiles are resident at once, pcg_grid.cu and pcg_rows.cu run
+// the same iteration, with the same bits, in one launch per inner solve.
 // On GB300 the FP64 pipe, not HBM, bounds the FP64 SpMV, so the product does
 // only the 9 DFMA per block it must (one thread per vertex, no lane
 // reductions).  The LHS is stored in 32-vertex slices (lhs_slot), so the
