@@ -25,6 +25,7 @@
 // branches and reaches every barrier.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cfloat>
 
@@ -43,6 +44,7 @@ __device__ __forceinline__ bool finite_d(double x) { return x == x && fabs(x) <=
 //   [u: 4 * vpc T (x, y, z, 0 per vertex: one vector load per gather), then the
 //    halo's u the same way (haloMax vertices)]
 //   [p, s, w, d, r: 3 * vpc T each]
+//   [FP64: the terms of the three sums, one a thread of the warps with vertices]
 constexpr int kSlotBytes = 8 * sizeof(double) + 3 * kClusterWarps * sizeof(double) + 16 * sizeof(uint32_t);
 
 template <typename T>
@@ -51,6 +53,7 @@ struct ClusterSmem {
   T* warp;           // 3 * kClusterWarps warp partials
   uint32_t* ubase;   // shared::cluster address of u in every CTA of the cluster
   T *u, *p, *s, *w, *d, *r;
+  T* terms;          // FP64
 };
 
 template <typename T>
@@ -67,6 +70,7 @@ __device__ __forceinline__ ClusterSmem<T> carve_smem(unsigned char* base, int vp
   m.w = m.s + n;
   m.d = m.w + n;
   m.r = m.d + n;
+  m.terms = m.r + n;
   return m;
 }
 
@@ -183,23 +187,44 @@ __device__ __forceinline__ void contact_rows(const ContactRefs& c, int u, int v0
 // reductions use slots 1..3 (the previous one's remote reads end before the
 // cluster barrier that closes its iteration); the initial one uses 4..6, so
 // no CTA overwrites a slot another may not have read yet.
+// FP64: 96 shuffle trees issue 480 adds, 9,000 cycles of the pipe whether a warp
+// has vertices or not; tree32 forms the same trees of the first n threads' warps
+// with 9 adds for eight.  Steps of FP64 batches: 32 scenes of up to 2,197 vertices
+// 4.97 -> 4.67 ms, 4 of up to 1,000 1.21 -> 1.07 ms, 48 of up to 15,625 unchanged
+// (their tile path is the longer one; with the terms' 24 KB for every class
+// it was 0.6% slower).  The cluster's own tree skips the levels above CL: 96
+// mixed scenes 6.04 -> 5.94 ms.
 template <int CL, typename T>
 __device__ __forceinline__ void cluster_sum3(cg::cluster_group& cluster, const ClusterSmem<T>& m, T a, T b, T c,
-                                             int slot, double (&out)[3]) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-  }
+                                             int n, int slot, double (&out)[3]) {
   const int wid = threadIdx.x / 32, lane = threadIdx.x % 32;
-  if (lane == 0) {
-    m.warp[3 * wid] = a;
-    m.warp[3 * wid + 1] = b;
-    m.warp[3 * wid + 2] = c;
+  if constexpr (sizeof(T) == sizeof(double)) {
+    const int warps = min(kClusterWarps, (n + 31) / 32);  // the others' terms are zeros
+    if (wid < warps) {
+      m.terms[threadIdx.x] = a;
+      m.terms[32 * warps + threadIdx.x] = b;
+      m.terms[64 * warps + threadIdx.x] = c;
+    }
+    __syncthreads();
+    tree32(3 * warps, [&](int g, int l) { return m.terms[32 * g + l]; }, m.warp);
+    __syncthreads();
+    if (wid == 0)
+      tree32_warp(0, 3, [&](int g, int l) { return l < warps ? m.warp[warps * g + l] : 0.0; }, m.slots + slot);
+  } else {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+      c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (lane == 0) {
+      m.warp[3 * wid] = a;
+      m.warp[3 * wid + 1] = b;
+      m.warp[3 * wid + 2] = c;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  if (wid == 0) {
+  if (sizeof(T) == sizeof(float) && wid == 0) {
     T ta = m.warp[3 * lane], tb = m.warp[3 * lane + 1], tc = m.warp[3 * lane + 2];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -224,7 +249,7 @@ __device__ __forceinline__ void cluster_sum3(cg::cluster_group& cluster, const C
       sc = ld_cluster_f64(sl + 16);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = CL / 2; o > 0; o >>= 1) {  // (the other lanes hold zeros)
       sa += __shfl_xor_sync(0xffffffffu, sa, o);
       sb += __shfl_xor_sync(0xffffffffu, sb, o);
       sc += __shfl_xor_sync(0xffffffffu, sc, o);
@@ -525,7 +550,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
       }
       m.u[4 * lv + 3] = T(0);
     }
-    cluster_sum3<CL, T>(cluster, m, rr, ru, T(0), 4, sums);
+    cluster_sum3<CL, T>(cluster, m, rr, ru, T(0), nmine, 4, sums);
     if (t0) {
       ss.srr = sums[0];
       double itol = st.tol;
@@ -600,7 +625,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
         gl += r0 * u0 + r1 * u1 + r2 * u2;
         rl += r0 * r0 + r1 * r1 + r2 * r2;
       }
-      cluster_sum3<CL, T>(cluster, m, rl, gl, dl, 1, sums);
+      cluster_sum3<CL, T>(cluster, m, rl, gl, dl, nmine, 1, sums);
       if (t0) {
         // after an update: the convergence test on its residual, then the
         // scalars of this iteration's update (tile path: spmv_decide)
@@ -732,13 +757,16 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
 }
 
 // Shared memory a cluster kernel may have; kClusterSmemMax bounds the vectors
-// alone (which decides the scenes' cluster sizes), the halo takes what is left.
+// alone (which decides the scenes' cluster sizes), the halo (FP32) or the sums'
+// terms (FP64) take what is left.
 constexpr size_t kClusterSmemAll = 224 * 1024;
+static_assert(kClusterSmemMax + 3 * sizeof(double) * kClusterThreads <= kClusterSmemAll, "the FP64 sums' terms fit");
 
 template <int CL, typename T>
 int launch_class(const DeviceBatch& b, const PcgVecs<T>& v, const ClusterClass& c, cudaStream_t s) {
   if (c.count == 0) return 0;
-  const size_t smem = kSlotBytes + cluster_vertex_bytes(sizeof(T) == 4) * c.vpcMax;
+  const size_t smem = kSlotBytes + cluster_vertex_bytes(sizeof(T) == 4) * c.vpcMax +
+                      (sizeof(T) == 4 ? 0 : 3 * sizeof(double) * std::min(kClusterThreads, (c.vpcMax + 31) / 32 * 32));
   if (sizeof(T) == sizeof(float) && c.halo >= 0)
     k_pcg_cluster<CL, float, true><<<c.count * CL, kClusterThreads, smem + sizeof(float4) * c.halo, s>>>(
         b, b.v32, c.scenes, b.clusterGather, c.halo);
