@@ -258,12 +258,12 @@ __global__ void k_assemble_entry(DeviceBatch b, const HT* __restrict__ elemH, T*
 // transposed for the lower triangle), then LHS block = S(M - dt^2 K)S + (I - S)
 // written entry by entry, each entry of the warp's 32 slots one 128-byte line.
 // Only the slots with w >= u are summed, and written twice (k_assemble_entry):
-// 384,000 tets 86 -> 68 us, 96 scenes 468 -> 363 us (k_assemble_entry in FP32:
+// 384,000 tets 86 -> 66 us, 96 scenes 468 -> 346 us (k_assemble_entry in FP32:
 // 124 and 795 us).
 // Blocks of parked scenes keep their old values.  The gathers are latency
-// bound, so registers are capped at 64 (no spills) for 32 resident warps per
-// SM instead of 28; the cap also keeps every tunable CTA size (up to 1024
-// threads) within the SM's 65,536 registers.
+// bound: two contributions at a time take 54 registers and 36 warps are resident
+// per SM (four: 64 and 32); the cap of 64 keeps every tunable CTA size (up to
+// 1024 threads) within the SM's 65,536 registers.
 template <typename HT, typename T>
 __global__ void __maxnreg__(64) k_assemble(DeviceBatch b, const HT* __restrict__ elemH, T* __restrict__ lhs) {
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -277,8 +277,9 @@ __global__ void __maxnreg__(64) k_assemble(DeviceBatch b, const HT* __restrict__
       HT sum[9];
 #pragma unroll
       for (int e = 0; e < 9; e++) sum[e] = HT(0);
-      // contributions in flight: 4 in FP32, 2 in FP64 (register budget)
-      constexpr int kQ = sizeof(HT) == sizeof(float) ? 4 : 2;
+      // contributions in flight: lists of 4 and 6 waste none of two (of four:
+      // 384,000 tets 68 us; 66 here)
+      constexpr int kQ = 2;
       const int k0 = b.blkptr[blk], k1 = b.blkptr[blk + 1];
       for (int k = k0; k < k1; k += kQ) {
         int src[kQ];
