@@ -26,8 +26,8 @@
 // both give the same bits and a scene's result does not depend on the batch.
 //
 // What bounds it: in FP64 the SM's FP64 pipe, 19 cycles per warp instruction
-// (16 warps x 135 products of 512 vertices' rows are 41,000 of an iteration's
-// 65,000 cycles); in FP32 latency: the row sums from shared memory are 4,600 of
+// (16 warps x 135 products of 512 vertices' rows are 39,000 of an iteration's
+// 64,000 cycles); in FP32 latency: the row sums from shared memory are 4,600 of
 // 16,200 cycles, the halo 1,700, the partials' exchange 2,100, the scalars
 // 3,600.  The phases between barriers run once an iteration on few warps, so
 // loops there are kept rolled: 108 KB of code cost 4,000 cycles more an
