@@ -771,6 +771,14 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
 
 int sweeps_of(const hobak_solver_opts& o);
 
+// No partial of pcg_rows.cu keeps a tag.  On the batch's stream: a memset returns
+// before it has run, and nothing orders one on the default stream before the next
+// step's solve, whose words it could wipe while their readers wait for them.
+int clear_row_words(hobak_batch_t* B) {
+  CUDA_TRY(cudaMemsetAsync(B->d.gridRowWords, 0, sizeof(ulonglong2) * grid_row_words(), B->stream));
+  return HOBAK_OK;
+}
+
 int upload_solver_opts(hobak_batch_t* B) {
   std::vector<SolveState> st(B->scenes.size());
   for (auto& s : st) {
@@ -782,8 +790,7 @@ int upload_solver_opts(hobak_batch_t* B) {
   }
   CUDA_TRY(cudaMemcpy(B->d.solve, st.data(), sizeof(SolveState) * st.size(), cudaMemcpyHostToDevice));
   // the scenes' solves count from zero again: no tag of theirs may be left
-  CUDA_TRY(cudaMemset(B->d.gridRowWords, 0, sizeof(ulonglong2) * grid_row_words()));
-  return HOBAK_OK;
+  return clear_row_words(B);
 }
 
 int check_opts(const hobak_solver_opts* o) {
@@ -1020,8 +1027,8 @@ int prepare_grid_plan(hobak_batch_t* B) {
       else
         for (int t = 0; t < tiles[s]; t += g.tpc) list.push_back(make_int2(s, t));
     if ((int)list.size() != g.ctas || g.ctas > kGridCtas) return fail(HOBAK_ERR_CUDA, "PCG plan: wrong CTA count");
-    CUDA_TRY(cudaStreamSynchronize(B->stream));
-    CUDA_TRY(cudaMemcpy(B->gridList, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice));
+    // (from pageable memory: the call returns once the table is staged)
+    CUDA_TRY(cudaMemcpyAsync(B->gridList, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice, B->stream));
     g.list = B->gridList;
     if (mixed) {
       int* largest = B->d.gridHaloCount + B->d.gridTilesCap;
