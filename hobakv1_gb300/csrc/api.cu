@@ -1038,7 +1038,13 @@ int prepare_grid_plan(hobak_batch_t* B) {
       CUDA_TRY(cudaMemcpyAsync(&g.halo, largest, sizeof(int), cudaMemcpyDeviceToHost, B->stream));
       CUDA_TRY(cudaStreamSynchronize(B->stream));
     }
-    if (!g.rowVerts) plan_grid_smem(g, B->d.tileV, B->longestRow, mixed);
+    if (g.rowVerts) {
+      // a CTA's words lie by its place in the launch and name a solve by its number in
+      // its scene: of another scene that had the place, they could pass for this one's
+      if (int rc = clear_row_words(B)) return rc;
+    } else {
+      plan_grid_smem(g, B->d.tileV, B->longestRow, mixed);
+    }
   }
   if (g.ctas != B->grid.ctas || g.tpc != B->grid.tpc || g.rows != B->grid.rows || g.smem != B->grid.smem ||
       g.scratch != B->grid.scratch || g.halo != B->grid.halo ||

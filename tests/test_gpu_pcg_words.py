@@ -54,3 +54,30 @@ def test_words_are_cleared_in_order_with_the_batchs_steps():
     finally:
         stop.set()
         t.join()
+
+
+def test_a_scene_that_takes_over_another_ones_place():
+    """Two FP64 scenes of two CTAs each; the second sits out a step, so that its
+    next solve has the number of the first one's last, which took two iterations
+    and left words of both.  The first then moves to a cluster and the second
+    takes its place in the launch: as alone, to the bit."""
+    first = moving(3, 2, dt=1e-7)  # A = M up to 1e-14: one iteration, and the test of its residual
+    second = moving(3, 3)
+    b = hobak.BATCH([first, second])
+    b.set_tuning(cluster_pcg=1)
+    for k in (0, 1):
+        b.set_scene_cluster(k, -1)
+    b.step(2)
+    b.set_active(1, False)
+    assert b.step(1)[0][0] <= 2
+    b.set_active(1, True)
+    b.set_scene_cluster(0, 1)
+    assert list(b.pcg_path()) == [1, 0]
+    st = b.step(1)[1]
+    got = b.get_state(1)
+    b.close()
+    alone = hobak.BATCH([second])
+    want = alone.step(3)[0]
+    assert st == want
+    assert all(np.array_equal(g, w) for g, w in zip(got, alone.get_state(0)))
+    alone.close()
