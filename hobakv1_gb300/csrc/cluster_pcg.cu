@@ -26,7 +26,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cfloat>
 
 #include "pcg_common.cuh"
@@ -793,20 +792,18 @@ cudaError_t allow_smem() {
 }  // namespace
 
 // Opt every cluster kernel into kClusterSmemAll bytes of dynamic shared
-// memory (once per process; outside any stream capture; batches may be
+// memory (once per device; outside any stream capture; batches may be
 // created and stepped from several host threads).
 int configure_cluster_pcg() {
-  static std::atomic<int> done{0};
-  if (done.load()) return 0;
-  cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = allow_smem<1>();
-  if (e == cudaSuccess) e = allow_smem<2>();
-  if (e == cudaSuccess) e = allow_smem<4>();
-  if (e == cudaSuccess) e = allow_smem<8>();
-  if (e == cudaSuccess) e = allow_smem<16>();
-  if (e != cudaSuccess) return (int)e;
-  done.store(1);
-  return 0;
+  static OncePerDevice once;
+  return once_on_this_device(once, [] {
+    cudaError_t e = allow_smem<1>();
+    if (e == cudaSuccess) e = allow_smem<2>();
+    if (e == cudaSuccess) e = allow_smem<4>();
+    if (e == cudaSuccess) e = allow_smem<8>();
+    if (e == cudaSuccess) e = allow_smem<16>();
+    return (int)e;
+  });
 }
 
 // u (4 wide) and p, s, w, d, r (3 wide) per vertex

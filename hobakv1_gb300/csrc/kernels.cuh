@@ -4,8 +4,17 @@
 
 #include "collision.cuh"
 #include "common.cuh"
+#include "once_per_device.h"
 
 namespace hobak {
+
+// A set-up of the current device, unless it was done.  Returns a cudaError_t value.
+template <typename SetUp>
+int once_on_this_device(OncePerDevice& once, SetUp setUp) {
+  int device = -1;
+  if (const cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return (int)e;
+  return once(device, setUp);
+}
 
 // Vectors and matrix of one inner PCG solve, in arithmetic type T.
 template <typename T>

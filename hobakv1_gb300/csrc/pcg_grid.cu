@@ -40,7 +40,6 @@
 // scene's solve is marked failed.  All CTAs are resident (cooperative launch,
 // at most one per SM), so no CTA waits for one that cannot run.
 #include <algorithm>
-#include <atomic>
 
 #include "pcg_common.cuh"
 
@@ -677,18 +676,17 @@ void launch_grid_halo(const DeviceBatch& b, const GridPlan& g, int* largest, cud
   k_grid_halo<<<g.ctas, g.tpc * b.tileV, 0, s>>>(b, g.list, g.tpc, largest);
 }
 
-// Dynamic shared-memory opt-in (once per process, outside capture).
+// Dynamic shared-memory opt-in (once per device, outside capture).
 int configure_grid_pcg() {
-  static std::atomic<int> done{0};
-  if (done.load()) return 0;
-  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(k_pcg_grid<64, float>, attr, kGridSmemMax);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<128, float>, attr, kGridSmemMax);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<64, double>, attr, kGridSmemMax);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<128, double>, attr, kGridSmemMax);
-  if (e != cudaSuccess) return (int)e;
-  done.store(1);
-  return 0;
+  static OncePerDevice once;
+  return once_on_this_device(once, [] {
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_pcg_grid<64, float>, attr, kGridSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<128, float>, attr, kGridSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<64, double>, attr, kGridSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_grid<128, double>, attr, kGridSmemMax);
+    return (int)e;
+  });
 }
 
 template <typename T>

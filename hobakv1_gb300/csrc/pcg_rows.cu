@@ -18,7 +18,6 @@
 // Waiting for a thread's words together and not one by one: 2,197 vertices, three
 // Newmark iterations 1,120 -> 990 us, 3,375 vertices 493 -> 466 us.
 #include <algorithm>
-#include <atomic>
 
 #include "pcg_common.cuh"
 
@@ -258,16 +257,15 @@ GridPlan plan_rows_pcg(const int* nv, int n, int longestRow, int sms) {
   return g;
 }
 
-// Dynamic shared-memory opt-in (once per process, outside capture).
+// Dynamic shared-memory opt-in (once per device, outside capture).
 int configure_rows_pcg() {
-  static std::atomic<int> done{0};
-  if (done.load()) return 0;
-  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(k_pcg_rows<64>, attr, kRowSmemMax);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_rows<128>, attr, kRowSmemMax);
-  if (e != cudaSuccess) return (int)e;
-  done.store(1);
-  return 0;
+  static OncePerDevice once;
+  return once_on_this_device(once, [] {
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_pcg_rows<64>, attr, kRowSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pcg_rows<128>, attr, kRowSmemMax);
+    return (int)e;
+  });
 }
 
 int launch_rows_pcg(const DeviceBatch& b, const PcgVecs<double>& v, const GridPlan& g, cudaStream_t s) {
