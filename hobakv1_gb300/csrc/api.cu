@@ -720,6 +720,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   d.gridPartials = carve<double>(base, oGridP);
   d.gridFlags = carve<int>(base, oGridF);
   d.gridTilesCap = ntilesCap;
+  d.waitPolls = kWaitPolls;
   B->gridList = carve<int2>(base, oGridL);
   d.gridHaloCount = carve<int>(base, oGridHc);
   d.gridRowWords = carve<ulonglong2>(base, oGridRw);
@@ -1851,8 +1852,8 @@ int hobak_batch_wait(hobak_batch b, hobak_step_stats* stats) {
   int status = HOBAK_OK;
   for (int s = 0; s < n; s++) {
     const SolveState& st = b->lastSolve[s];
-    if (st.converged == kSolveTimedOut) status = HOBAK_ERR_CUDA;
-    else if (st.converged < 0 && status != HOBAK_ERR_CUDA) status = HOBAK_ERR_NAN;
+    if (st.converged == kSolveTimedOut) status = HOBAK_ERR_TIMEOUT;
+    else if (st.converged < 0 && status != HOBAK_ERR_TIMEOUT) status = HOBAK_ERR_NAN;
     else if (st.converged == 0 && status == HOBAK_OK) status = HOBAK_WARN_NOT_CONVERGED;
     if (stats) {
       stats[s].iterations = st.totalIters;
@@ -1861,7 +1862,7 @@ int hobak_batch_wait(hobak_batch b, hobak_step_stats* stats) {
       stats[s].refinements = st.sweep > 0 ? st.sweep - 1 : 0;
     }
   }
-  if (status == HOBAK_ERR_CUDA) return fail(status, "a wait inside the PCG launch ran out");
+  if (status == HOBAK_ERR_TIMEOUT) return fail(status, "a wait inside the PCG launch ran out");
   if (status == HOBAK_ERR_NAN) return fail(status, "non-finite residual in PCG");
   if (b->d.collOn) {
     int over = 0;
@@ -2382,6 +2383,14 @@ int hobak_batch_set_scene_cluster(hobak_batch b, int scene, int ctas) {
     b->sceneCluster[scene] = ctas;
     b->clusterDirty = true;
   }
+  return HOBAK_OK;
+}
+
+int hobak_batch_set_wait_limit(hobak_batch b, int polls) {
+  if (!b || polls < 0) return fail(HOBAK_ERR_INVALID, "bad handle or polls < 0");
+  CUDA_TRY(cudaStreamSynchronize(b->stream));
+  if (b->d.waitPolls != polls) drop_graphs(b);
+  b->d.waitPolls = polls;
   return HOBAK_OK;
 }
 

@@ -59,6 +59,7 @@ struct GridPlan {
   size_t smem;       // dynamic shared memory of a CTA
   const int2* list;  // device: per CTA its scene and its first tile in the scene
 };
+constexpr int kWaitPolls = 1 << 21;   // polls of one wait (about a second), by default
 constexpr int kSolveTimedOut = -2;  // SolveState::converged: a wait of the one-launch PCG ran out
 
 // Device pointers of one packed batch.  Plain struct passed by value.
@@ -176,6 +177,7 @@ struct DeviceBatch {
   int gridTilesCap;
   int gridOn;  // the tile-path scenes take that path (2: pcg_rows.cu)
   ulonglong2* gridRowWords;  // [2][CTAs][9] partials of pcg_rows.cu
+  int waitPolls;  // polls after which a wait of these launches gives up
   // FP32 (pcg_grid.cu and clusters): per CTA the vertices of other CTAs that its
   // rows' columns name (at 4 x its first vertex), their number (per tile: a
   // CTA's is its first tile's), and every column as the CTA's own index of it

@@ -294,7 +294,6 @@ __device__ __forceinline__ void publish_u(double* u4, int w, const double (&x)[3
 
 // Words of the one-launch PCGs: a value and the tag it belongs to, written and
 // read at once.
-constexpr int kSpinLimit = 1 << 21;  // polls of one wait (about a second), then the solve fails
 __device__ __forceinline__ void st_word(ulonglong2* p, double value, unsigned long long tag) {
   asm volatile(
       "{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p),
@@ -312,9 +311,10 @@ __device__ __forceinline__ void ld_word(const ulonglong2* p, double& value, unsi
 
 // N words whose tags must all be `tag`: use(k) says which of them, at(k) where.
 // All are loaded at once, and those not there yet again at once, so a wait costs
-// the latency of the last one and not of each.  Clears ok when they never come.
+// the latency of the last one and not of each.  Clears ok when one is not there
+// after `limit` polls.
 template <int N, typename Use, typename At>
-__device__ __forceinline__ void ld_words(Use use, At at, unsigned long long tag, double (&value)[N], bool& ok) {
+__device__ __forceinline__ void ld_words(Use use, At at, unsigned long long tag, int limit, double (&value)[N], bool& ok) {
   unsigned long long got[N];
 #pragma unroll
   for (int k = 0; k < N; k++)
@@ -326,7 +326,7 @@ __device__ __forceinline__ void ld_words(Use use, At at, unsigned long long tag,
     for (int k = 0; k < N; k++)
       if (use(k) && got[k] != tag) missing = true;
     if (!missing) break;
-    if (n > kSpinLimit) ok = false;
+    if (n >= limit) ok = false;
 #pragma unroll
     for (int k = 0; k < N; k++)
       if (use(k) && got[k] != tag) ld_word(at(k), value[k], got[k]);

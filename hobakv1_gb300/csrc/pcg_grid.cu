@@ -72,10 +72,10 @@ struct Gather32 {
   }
   // repeats the load of vertex() until it fits; clears ok when it does not
   template <typename Vertex>
-  __device__ __forceinline__ void get(const float* u4, Vertex vertex, int it, float (&x)[3], bool& ok) {
+  __device__ __forceinline__ void get(const float* u4, Vertex vertex, int it, int limit, float (&x)[3], bool& ok) {
 #pragma unroll 1
     for (int n = 0; (int)(hi >> 32) != it && ok; n++) {
-      if (n > kSpinLimit) ok = false;
+      if (n >= limit) ok = false;
       load(u4, vertex());
     }
     x[0] = __uint_as_float((unsigned)lo);
@@ -91,7 +91,7 @@ struct Gather64 {  // the caller has waited for the owner's flag
     z = __ldcg(u4 + 4 * (size_t)w + 2);
   }
   template <typename Vertex>
-  __device__ __forceinline__ void get(const double*, Vertex, int, double (&x)[3], bool&) {
+  __device__ __forceinline__ void get(const double*, Vertex, int, int, double (&x)[3], bool&) {
     x[0] = a.x, x[1] = a.y, x[2] = z;
   }
 };
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
         for (int k = 0; k < 4; k++) {
           if (i0 + k * NT >= nHalo) break;
           T x[3];
-          g[k].get(u4, [&] { return w[k]; }, it, x, ok);
+          g[k].get(u4, [&] { return w[k]; }, it, b.waitPolls, x, ok);
           us[NT + i0 + k * NT] = make_float4(x[0], x[1], x[2], 0.f);
         }
       }
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
         int n = 0;
 #pragma unroll 1
         while (ld_flag(f) < it && ok)
-          if (++n > kSpinLimit) ok = false;
+          if (n++ >= b.waitPolls) ok = false;
       }
       if ((failed = __syncthreads_or(!ok))) break;
       // Two blocks per trip (the chains of even and odd blocks), the next
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
               m[q][e] = j + q < len ? __ldg(&v.lhs[lb + (size_t)kSlotVals * (j + q) + kSlice * e]) : T(0);
         }
 #pragma unroll
-        for (int q = 0; q < kQ; q++) g[q].get(u4, [] { return 0; }, it, x[q], ok);
+        for (int q = 0; q < kQ; q++) g[q].get(u4, [] { return 0; }, it, b.waitPolls, x[q], ok);
         if (j + kQ < lenMax) gather(j + kQ);
         acc.add(m[0], x[0], false);
         if (j + 1 < lenMax) acc.add(m[1], x[1], true);
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
               [&](int id, T (&x)[3]) {
                 Gather g;
                 g.load(u4, id);
-                g.get(u4, [&] { return id; }, it, x, ok);
+                g.get(u4, [&] { return id; }, it, b.waitPolls, x, ok);
               },
               t);
 #pragma unroll
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
     for (int i0 = tid; i0 < 3 * nParts; i0 += 4 * NT) {
       double value[4];
       ld_words<4>([&](int k) { return i0 + k * NT < 3 * nParts; }, [&](int k) { return in + i0 + k * NT; },
-                  (unsigned long long)it, value, ok);
+                  (unsigned long long)it, b.waitPolls, value, ok);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         const int i = i0 + k * NT;

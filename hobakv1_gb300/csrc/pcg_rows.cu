@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kRowThreads, 1)
 #pragma unroll
       for (int q = 0; q < kBatch; q++) w[q] = j0 + q < rows ? col[(j0 + q) * kRowVerts + lv] : own;
       ld_words<3 * kBatch>([&](int) { return true; }, [&](int k) { return uw + 3 * (size_t)w[k / 3] + k % 3; },
-                           (unsigned long long)it, x, ok);
+                           (unsigned long long)it, b.waitPolls, x, ok);
 #pragma unroll
       for (int q = 0; q < kBatch; q++)
         if (j0 + q < lenMax) {
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kRowThreads, 1)
               b.coll, base + tid,
               [&](int id, double (&x)[3]) {
                 ld_words<3>([&](int) { return true; }, [&](int c) { return uw + 3 * (size_t)id + c; },
-                            (unsigned long long)it, x, ok);
+                            (unsigned long long)it, b.waitPolls, x, ok);
               },
               t);
 #pragma unroll
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kRowThreads, 1)
     for (int k0 = tid; k0 < 3 * nTrees; k0 += kWords * kRowThreads) {
       double value[kWords];
       ld_words<kWords>([&](int k) { return k0 + k * kRowThreads < 3 * nTrees; },
-                       [&](int k) { return scene + par + k0 + k * kRowThreads; }, tag, value, ok);
+                       [&](int k) { return scene + par + k0 + k * kRowThreads; }, tag, b.waitPolls, value, ok);
 #pragma unroll
       for (int k = 0; k < kWords; k++) {
         const int q = k0 + k * kRowThreads;

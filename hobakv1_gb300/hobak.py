@@ -580,6 +580,10 @@ class BATCH:
         path, 0 by the batch's tuning."""
         check(_lib.load().hobak_batch_set_scene_cluster(self.h, scene, int(ctas)), "hobak_batch_set_scene_cluster")
 
+    def set_wait_limit(self, polls: int):
+        """Polls after which a wait inside a step gives up (HOBAK_ERR_TIMEOUT)."""
+        check(_lib.load().hobak_batch_set_wait_limit(self.h, int(polls)), "hobak_batch_set_wait_limit")
+
     def blocks(self, scene: int) -> int:
         """3x3 blocks of one scene's system matrix (its BSR pattern)."""
         n = ctypes.c_int()

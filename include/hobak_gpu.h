@@ -367,6 +367,12 @@ int hobak_batch_pcg_path(hobak_batch b, int* cluster_ctas);
  * the scene, so a scene given the same override alone and in a batch takes
  * the same path. */
 int hobak_batch_set_scene_cluster(hobak_batch b, int scene, int ctas);
+/* Polls after which a wait inside a step gives up (no reference counterpart):
+ * the tile path's PCG in one launch waits for the other CTAs' words; a wait that
+ * runs out ends its scene's solve, and the step returns HOBAK_ERR_TIMEOUT with
+ * that scene's state undefined and the batch usable.  Default 2097152 (about a
+ * second); 0: a word must be there when it is first looked for. */
+int hobak_batch_set_wait_limit(hobak_batch b, int polls);
 int hobak_batch_set_tuning(hobak_batch b, const hobak_tuning* t);
 /* Autotuner: times the element kernel per CTA size and the assembly kernel
  * per CTA size (reps launches each, CUDA events), then whole steps for every
