@@ -168,6 +168,7 @@ struct hobak_batch_t {
   cudaEvent_t evTerms = nullptr, evRhs = nullptr;
   int lastStatus = HOBAK_OK;
   std::vector<SolveState> lastSolve;
+  bool waitFailed = false;  // a wait ran out in a step of the last ones collected
   std::vector<int> hostRowptr, hostCols;
   std::vector<SceneParams> sceneParams;   // host copy (active flags)
   SolveState* solvePinned = nullptr;      // pinned landing buffer for per-step stats
@@ -772,6 +773,13 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
 
 int sweeps_of(const hobak_solver_opts& o);
 
+// A scene's solves that a wait ended, by the last steps whose states reached the
+// host (the callers have waited for the stream).
+int wait_failures(const hobak_batch_t* B, size_t scene) {
+  if (B->pending) return B->solvePinned[scene].waitFailures;
+  return B->lastSolve.empty() ? 0 : B->lastSolve[scene].waitFailures;
+}
+
 // No partial of pcg_rows.cu keeps a tag.  On the batch's stream: a memset returns
 // before it has run, and nothing orders one on the default stream before the next
 // step's solve, whose words it could wipe while their readers wait for them.
@@ -782,8 +790,10 @@ int clear_row_words(hobak_batch_t* B) {
 
 int upload_solver_opts(hobak_batch_t* B) {
   std::vector<SolveState> st(B->scenes.size());
-  for (auto& s : st) {
+  for (size_t k = 0; k < st.size(); k++) {
+    SolveState& s = st[k];
     std::memset(&s, 0, sizeof(s));
+    s.waitFailures = wait_failures(B, k);
     s.tol = B->opts.tol;
     s.innerFloor = B->opts.inner_tolerance;
     s.maxit = B->opts.max_iters;
@@ -1844,16 +1854,20 @@ int hobak_batch_wait(hobak_batch b, hobak_step_stats* stats) {
   CUDA_TRY(cudaStreamSynchronize(b->stream));
   const int n = (int)b->scenes.size();
   if (b->pending) {
+    // of all steps enqueued since the last call, and every Newton iteration of
+    // them: a later solve resets `converged`
+    b->waitFailed = false;
+    for (int s = 0; s < n; s++)
+      b->waitFailed |= b->solvePinned[s].waitFailures > (b->lastSolve.empty() ? 0 : b->lastSolve[s].waitFailures);
     b->lastSolve.assign(b->solvePinned, b->solvePinned + n);
     b->pending = false;
     b->clusterOrderStale = true;
   }
   if ((int)b->lastSolve.size() != n) return HOBAK_OK;  // nothing stepped yet
-  int status = HOBAK_OK;
+  int status = b->waitFailed ? HOBAK_ERR_TIMEOUT : HOBAK_OK;
   for (int s = 0; s < n; s++) {
     const SolveState& st = b->lastSolve[s];
-    if (st.converged == kSolveTimedOut) status = HOBAK_ERR_TIMEOUT;
-    else if (st.converged < 0 && status != HOBAK_ERR_TIMEOUT) status = HOBAK_ERR_NAN;
+    if (st.converged < 0 && status != HOBAK_ERR_TIMEOUT) status = HOBAK_ERR_NAN;
     else if (st.converged == 0 && status == HOBAK_OK) status = HOBAK_WARN_NOT_CONVERGED;
     if (stats) {
       stats[s].iterations = st.totalIters;

@@ -87,6 +87,7 @@ struct SolveState {
   float alphaF, betaF;  // FP32 copies for the mixed inner solve (no per-thread conversion)
   int iters, done;
   int epoch;  // inner solves started (tags of pcg_rows.cu)
+  int waitFailures;  // inner solves that a wait ended; never reset
   unsigned ticketA, ticketB;
   // Newmark's Newton loop: iterations done, finished flag, |rhs|^2 of the last one
   int newtonStep, newtonDone;

@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(kRowThreads, 1)
   if (tid == 0 && cta.y == 0) {
     if (failed) {
       ss.converged = kSolveTimedOut;
+      ss.waitFailures += 1;
       ss.outerDone = 1;
     }
     ss.done = 1;

@@ -44,3 +44,32 @@ def test_a_wait_that_runs_out_ends_the_step(N, precision, integrator, use_graph)
     assert b.step(2) == want_stats
     assert all(np.array_equal(g, w) for g, w in zip(b.get_state(0), want))
     b.close()
+
+
+@pytest.mark.parametrize("precision", [hobak.PRECISION_FP64, hobak.PRECISION_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("integrator", [hobak.INTEGRATOR_VELOCITY, hobak.INTEGRATOR_NEWMARK],
+                         ids=["velocity", "newmark"])
+def test_a_wait_that_ran_out_is_not_lost_in_a_later_solve(precision, integrator):
+    """Of several steps, or Newton iterations, enqueued before the host looks."""
+    s = moving(9)
+    b = hobak.BATCH([s], hobak.solver_opts(precision=precision, integrator=integrator))
+    start = b.snapshot()
+    for change_options in (False, True):
+        b.set_wait_limit(0)
+        b.step_async(1)
+        b.set_wait_limit(DEFAULT)
+        b.restore(start)
+        if change_options:
+            b.set_solver(b.opts)
+        b.step_async(1)  # this one succeeds
+        for _ in range(2):  # the same answer until the next step
+            with pytest.raises(HobakError) as e:
+                b.wait()
+            assert e.value.code == HOBAK_ERR_TIMEOUT
+        b.restore(start)
+        b.step(1)
+        b.restore(start)
+        b.set_solver(b.opts)
+        b.step(1)
+        b.restore(start)
+    b.close()
