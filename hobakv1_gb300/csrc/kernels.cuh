@@ -169,9 +169,10 @@ struct DeviceBatch {
   // inner solves
   PcgVecs<double> v64;  // FP64 path (r = r64, d = y)
   PcgVecs<float> v32;   // mixed path
-  double* partial;      // [ntiles][kPartials]
+  double* partial;      // [ntiles][kPartials]; k_spmv in FP32: [3][gridTilesCap]
   // one-launch PCG (pcg_grid.cu): [2][gridTilesCap][3] 16-byte words {partial,
-  // iteration} and a flag per tile
+  // iteration} and a flag per tile.  The FP32 loop of two kernels keeps the sums of
+  // its groups and their tickets there (scene_sums)
   double* gridPartials;
   int* gridFlags;
   int gridTilesCap;

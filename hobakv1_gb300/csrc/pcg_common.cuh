@@ -190,22 +190,70 @@ __device__ __forceinline__ double scene_sum(int n, Group group) {
   return warp_tree(s);
 }
 
-// FP32: the three scene sums from global tile partials, by the last CTA of the
-// scene; sh: 3 doubles.  Result valid in thread 0.
+// FP32: the three scene sums from the tiles' partials, [component][stride], in
+// scene_sum's order.  True in the CTA that ends them, with the sums in thread 0.
+// The iteration waits for them, so the last CTA of a scene adds all groups only up
+// to kOneCta of them.  Past that they lie in segments of 32: the last CTA of a
+// segment forms its groups' sums, a lane each, and the last of the segments adds
+// those (one more ticket: 1.7 us where one CTA is soon done).  Microseconds of
+// k_spmv with one CTA a lane's groups one after the other / this: tiles of 128,
+// 52^3 (291 groups, one CTA) 23.3 / 18.7, 72^3 (760, segments) 65.2 / 54.9; tiles
+// of 64, 45^3 (191, one CTA) 18.6 / 17.5, 52^3 31.0 / 20.8, 72^3 82.6 / 59.2.
+// tickets: one per tile, zero (a segment takes its first tile's).
 template <int NT, int TV>
-__device__ __forceinline__ void scene_sums(const double* partial, int tile0, int n, double* sh, double (&out)[3]) {
-  constexpr int kG = kGroupVerts / TV;
-  for (int c = threadIdx.x / 32; c < 3; c += NT / 32) {
-    const double t = scene_sum((n + kG - 1) / kG, [&](int g) {
-      return group_sum<TV>([&](int i) {
-        return g * kG + i < n ? __ldcg(&partial[(size_t)(tile0 + g * kG + i) * kPartials + c]) : 0.0;
-      });
-    });
-    if (threadIdx.x % 32 == 0) sh[c] = t;
+__device__ __forceinline__ bool scene_sums(const double* partial, double* groupSums, int stride, unsigned* tickets,
+                                           unsigned* sceneTicket, const SceneParams& sp, int tile, int* flag,
+                                           double* sh, double (&out)[3]) {
+  constexpr int kG = kGroupVerts / TV, kWarps = NT / 32, kPer = (3 + kWarps - 1) / kWarps;
+  constexpr int kOneCta = TV == 128 ? 512 : 192;
+  const int tile0 = sp.tile0, n = sp.ntiles, ng = (n + kG - 1) / kG;
+  const bool one = ng <= kOneCta;
+  const int g0 = one ? 0 : (tile - tile0) / (32 * kG) * 32, g1 = one ? ng : min(ng, g0 + 32);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (!last_tile(one ? sceneTicket : &tickets[tile0 + g0 * kG], min(n, g1 * kG) - g0 * kG, flag)) return false;
+  double t[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    const int c = warp + k * kWarps;
+    const double* q = partial + (size_t)c * stride + tile0;
+    auto group = [&](int g) {
+      return group_sum<TV>([&](int i) { return g * kG + i < n ? __ldcg(&q[g * kG + i]) : 0.0; });
+    };
+    t[k] = 0.0;
+    if (c < 3 && one) {
+#pragma unroll 4
+      for (int g = lane; g < ng; g += 32) t[k] += group(g);
+    } else if (c < 3) {
+      t[k] = group(g0 + lane);
+    }
+  }
+  if (!one) {
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+      const int c = warp + k * kWarps;
+      if (c < 3) groupSums[(size_t)c * stride + tile0 + g0 + lane] = t[k];
+    }
+    __syncthreads();  // last_tile's fence by thread 0 covers the writers
+    if (!last_tile(sceneTicket, (ng + 31) / 32, flag)) return false;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+      const int c = warp + k * kWarps;
+      t[k] = 0.0;
+      if (c < 3)
+#pragma unroll 8
+        for (int g = lane; g < ng; g += 32) t[k] += __ldcg(&groupSums[(size_t)c * stride + tile0 + g]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    const int c = warp + k * kWarps;
+    const double total = warp_tree(t[k]);
+    if (c < 3 && lane == 0) sh[c] = total;
   }
   __syncthreads();
 #pragma unroll
   for (int c = 0; c < 3; c++) out[c] = sh[c];
+  return true;
 }
 
 __device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
