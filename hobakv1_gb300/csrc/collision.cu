@@ -710,7 +710,8 @@ __device__ __forceinline__ float line_distance(float3 a, float3 d, float3 b0, fl
   const float ee = e.x * e.x + e.y * e.y + e.z * e.z, pe = p.x * e.x + p.y * e.y + p.z * e.z;
   const float t = ee > 0.f ? fminf(fmaxf(-pe / ee, 0.f), 1.f) : 0.f;
   const float3 m = {p.x + t * e.x, p.y + t * e.y, p.z + t * e.z};
-  return sqrtf(m.x * m.x + m.y * m.y + m.z * m.z);
+  const float mm = m.x * m.x + m.y * m.y + m.z * m.z;
+  return dd < FLT_MAX && ee < FLT_MAX && mm < FLT_MAX ? sqrtf(mm) : 0.f;  // no bound where a square overflows
 }
 
 // Eight lanes per edge, one per cell (at most 2x2x2).  As in k_vf_query a lane
