@@ -84,16 +84,22 @@ struct Built {
   std::string error;
 };
 
-// Device bytes of one scene in a batch, an upper estimate: the common
-// buffers plus those of the precision, at most 16 blocks per vertex row,
-// sliced in 32-vertex slices, plus 1 MB.
+// Device bytes of one scene in a batch, an estimate: the common buffers, those of
+// the precision and of the one-launch PCG, at 16 blocks per vertex row, plus 1 MB
+// for the padding of the 32-vertex slices and what does not grow with the scene.
+// Kuhn cubes of up to 20^3 take less.  Not counted: rows padded further (50^3 and
+// random Delaunay meshes take up to 3% and 11% more), the position integrator's
+// rest Hessian and contact.  An admitted cohort counts by its batch's own bytes.
 long long footprint_bytes(const hobak_scene_desc& s, int precision) {
   const long long nv = s.nv, nt = s.nt, nb = 16 * nv;
   const long long w = precision == HOBAK_PRECISION_MIXED ? 4 : 8;
   const long long perTet = 16 + 72 + 8 + 4 + 96 + 64 + 16 + 8 + 92 * w;  // element Hessians: 92 values per tet
   const long long perBlock = 4 + 4 + 4 + 4 + 9 * w;
   const long long perVertex = 5 * 24 + 8 + 1 + 4 + 4 + 4 + 3 * 24 + 9 * w + (w == 4 ? 6 : 4) * 3 * w;
-  return nt * perTet + nb * perBlock + nv * perVertex + (1LL << 20);
+  // partial words, flags and halo counts per tile of 64 vertices; the halo's lists
+  const long long perVertexPcg = 2 + (w == 4 ? 16 : 0);
+  constexpr long long kBatchPcg = 80 << 10;  // words of the thread-per-row PCG, CTA table
+  return nt * perTet + nb * perBlock + nv * (perVertex + perVertexPcg) + (1LL << 20) + kBatchPcg;
 }
 
 // One builder thread running build tasks in submission order, on the

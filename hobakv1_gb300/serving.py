@@ -53,9 +53,13 @@ from . import hobak
 
 
 def footprint_bytes(scene, precision: int) -> int:
-    """Conservative device bytes of one scene in a batch: the common buffers
-    plus those of its precision (the library allocates only the batch's
-    precision); at most 16 blocks per vertex row, padded in 32-vertex slices."""
+    """Estimated device bytes of one scene in a batch: the common buffers, those
+    of its precision (the library allocates only the batch's precision) and of
+    the one-launch PCG, at 16 blocks per vertex row, plus 1 MB for the padding of
+    the 32-vertex slices and what does not grow with the scene.  Kuhn cubes of up
+    to 20^3 take less.  Not counted: rows padded further (50^3 and random Delaunay
+    meshes take up to 3% and 11% more), the position integrator's rest Hessian
+    and contact.  An admitted cohort counts by its batch's own bytes."""
     nv, nt = scene.nv, scene.nt
     nb = 16 * nv
     w = 4 if precision == hobak.PRECISION_MIXED else 8
@@ -67,7 +71,10 @@ def footprint_bytes(scene, precision: int) -> int:
     # rest, x, v, f_ext, pin target, mass, mask, scene id, rowptr, incidences,
     # rhs, y, r64; block inverse and inner vectors
     per_vertex = 5 * 24 + 8 + 1 + 4 + 4 + 4 + 3 * 24 + 9 * w + (6 if w == 4 else 4) * 3 * w
-    return int(nt * per_tet + nb * per_block + nv * per_vertex + (1 << 20))
+    # partial words, flags and halo counts per tile of 64 vertices; the halo's lists
+    per_vertex_pcg = 2 + (16 if w == 4 else 0)
+    batch_pcg = 80 << 10  # words of the thread-per-row PCG, CTA table
+    return int(nt * per_tet + nb * per_block + nv * (per_vertex + per_vertex_pcg) + (1 << 20) + batch_pcg)
 
 
 @dataclasses.dataclass
