@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/hobak_gpu.h"
+#include "alloc_retry.h"
 #include "element_math.cuh"
 #include "kernels.cuh"
 
@@ -49,7 +50,8 @@ namespace {
 // device, ordered on the default stream these calls run on, where cudaMalloc and
 // cudaFree cost 100 us of a 150 us call.  The pool keeps at most kScratchKept
 // bytes between calls (the rest goes back at the next synchronisation), all of
-// it goes back before a batch allocates, and the driver serialises its users.
+// it goes back before a batch is created and where another allocation of a batch
+// would fail (batch_malloc), and the driver serialises its users.
 constexpr unsigned long long kScratchKept = 64ull << 20;
 
 cudaMemPool_t scratch_pool(bool make) {
@@ -81,6 +83,15 @@ void scratch_trim() {
   if (cudaMemPool_t p = scratch_pool(false)) cudaMemPoolTrimTo(p, 0);
 }
 
+// Device memory of a batch, past its creation too: what the pool keeps makes room.
+cudaError_t batch_malloc(void** p, size_t bytes) {
+  return (cudaError_t)alloc_or_release([&] { return (int)cudaMalloc(p, bytes); },
+                                       [] {
+                                         (void)cudaGetLastError();
+                                         scratch_trim();
+                                       });
+}
+
 struct DeviceScratch {
   void* p = nullptr;
   bool pooled = false;
@@ -92,8 +103,9 @@ struct DeviceScratch {
       }
       (void)cudaGetLastError();
     }
-    return cudaMalloc(&p, bytes);
+    return plain(bytes);
   }
+  cudaError_t plain(size_t bytes) { return batch_malloc(&p, bytes); }
   ~DeviceScratch() {
     if (p) pooled ? cudaFreeAsync(p, 0) : cudaFree(p);
   }
@@ -303,10 +315,10 @@ void set_integrator(SceneParams& p, const hobak_solver_opts& o) {
 int rest_hessian(hobak_batch_t* B) {
   if (B->K0) return HOBAK_OK;
   const size_t kBytes = sizeof(double) * 9 * (size_t)std::max(B->nblocks, 1);
-  CUDA_TRY(cudaMalloc(&B->K0, kBytes));
+  CUDA_TRY(batch_malloc(reinterpret_cast<void**>(&B->K0), kBytes));
   const size_t ehBytes = sizeof(double) * kElemHessStride * (size_t)B->nt, xBytes = sizeof(double) * 3 * (size_t)B->nv;
   void* scratch = nullptr;
-  CUDA_TRY(cudaMalloc(&scratch, ehBytes + 2 * xBytes));
+  CUDA_TRY(batch_malloc(&scratch, ehBytes + 2 * xBytes));
   cudaStream_t s = B->stream;
   DeviceBatch d = B->d;
   d.elemH = static_cast<double*>(scratch);
@@ -357,7 +369,7 @@ int alloc_precision(hobak_batch_t* B) {
   for (int k = 0; k < (mixed ? 6 : 4); k++) oVec[k] = A.reserve(w * 3 * nv);
   const size_t oHalo = mixed ? A.reserve(sizeof(int) * 4 * nv) : 0;  // clusters and the one-launch PCG
   void* base = nullptr;
-  cudaError_t e = cudaMalloc(&base, A.used);
+  cudaError_t e = batch_malloc(&base, A.used);
   if (e != cudaSuccess)
     return fail(e == cudaErrorMemoryAllocation ? HOBAK_ERR_NO_MEMORY : HOBAK_ERR_CUDA,
                 std::string("cudaMalloc of precision buffers: ") + cudaGetErrorString(e));
@@ -648,7 +660,7 @@ int build_batch(hobak_batch_t* B, const hobak_scene_desc* descs, int n) {
   const size_t oGridRw = A.reserve(sizeof(ulonglong2) * grid_row_words());
   const size_t oClHalo = A.reserve(sizeof(int) * (16 * (size_t)n + kClusterClasses));
   void* base = nullptr;
-  cudaError_t e = cudaMalloc(&base, A.used);
+  cudaError_t e = batch_malloc(&base, A.used);
   if (e != cudaSuccess)
     return fail(e == cudaErrorMemoryAllocation ? HOBAK_ERR_NO_MEMORY : HOBAK_ERR_CUDA,
                 std::string("cudaMalloc of batch arena: ") + cudaGetErrorString(e));
@@ -1513,7 +1525,7 @@ int build_collisions(hobak_batch_t* B) {
   const size_t oEeBox = A.reserve(2 * sizeof(float4) * (size_t)nedge), oEeLow = A.reserve(sizeof(int4) * (size_t)nedge);
   const size_t oEeSeg = A.reserve(2 * sizeof(float4) * (size_t)nedge);
   void* base = nullptr;
-  cudaError_t e = cudaMalloc(&base, A.used);
+  cudaError_t e = batch_malloc(&base, A.used);
   if (e != cudaSuccess)
     return fail(e == cudaErrorMemoryAllocation ? HOBAK_ERR_NO_MEMORY : HOBAK_ERR_CUDA,
                 std::string("cudaMalloc of collision buffers: ") + cudaGetErrorString(e));
@@ -2466,7 +2478,7 @@ int hobak_batch_autotune(hobak_batch b, int reps, hobak_tuning* out) {
   const size_t vbytes = 3 * sizeof(double) * (size_t)b->nv;
   CUDA_TRY(cudaStreamSynchronize(s));
   DeviceScratch saved;
-  CUDA_TRY(cudaMalloc(&saved.p, 3 * vbytes));
+  CUDA_TRY(saved.plain(3 * vbytes));
   double* x0 = static_cast<double*>(saved.p);
   double* v0 = x0 + 3 * (size_t)b->nv;
   double* a0 = v0 + 3 * (size_t)b->nv;  // Newmark's acceleration
@@ -2739,7 +2751,7 @@ int hobak_batch_assemble(hobak_batch b, int scene, int* nblocks, int* rowptr, in
   // order, scratch) and R (into the per-step rhs buffer)
   DeviceScratch scratch;
   const size_t ehBytes = sizeof(double) * kElemHessStride * (size_t)b->nt;
-  CUDA_TRY(cudaMalloc(&scratch.p, ehBytes + sizeof(double) * 9 * (size_t)std::max(b->nblocks, 1)));
+  CUDA_TRY(scratch.plain(ehBytes + sizeof(double) * 9 * (size_t)std::max(b->nblocks, 1)));
   DeviceBatch d = b->d;
   d.elemH = static_cast<double*>(scratch.p);
   double* Kd = reinterpret_cast<double*>(static_cast<char*>(scratch.p) + ehBytes);

@@ -8,11 +8,24 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "hobakv1_gb300", "csrc")
 
 
+def runs(name, tmp_path):
+    exe = str(tmp_path / name)
+    subprocess.run(["g++", "-std=c++17", "-I" + CSRC, os.path.join(ROOT, "tests", "cpp", name + ".cpp"), "-o", exe],
+                   check=True)
+    return subprocess.run([exe], capture_output=True, text=True).stdout
+
+
 def test_set_up_runs_once_on_each_device(tmp_path):
-    exe = str(tmp_path / "once_per_device")
-    subprocess.run(["g++", "-std=c++17", "-I" + CSRC, os.path.join(ROOT, "tests", "cpp", "once_per_device.cpp"),
-                    "-o", exe], check=True)
-    assert subprocess.run([exe], capture_output=True, text=True).stdout == "ok\n"
+    assert runs("once_per_device", tmp_path) == "ok\n"
+
+
+def test_kept_scratch_makes_room_for_a_batch(tmp_path):
+    """The evaluation calls' pool keeps memory between calls; no allocation of a
+    batch (precision, contact, rest Hessian, autotuner, inspection) fails for it."""
+    assert runs("alloc_retry", tmp_path) == "ok\n"
+    with open(os.path.join(CSRC, "api.cu")) as fh:
+        text = fh.read()
+    assert len(re.findall(r"[^a-z_]cudaMalloc\(", text)) == 1  # in batch_malloc
 
 
 def test_every_opt_in_is_per_device():
