@@ -815,9 +815,15 @@ void launch_cluster_gather(const DeviceBatch& b, cudaStream_t s) {
   k_cluster_gather<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b, b.clusterGather);
 }
 size_t cluster_fixed_bytes() { return kSlotBytes; }
+// Halo vertices of a CTA that leave the SM's L1 cache as large as without them: past
+// 196 KB an SM gives all of its 228 KB to shared memory and keeps 28 KB, and the
+// matrix comes slower than the halo's copy saves.  Steps of 120 iterations, four
+// scenes of 35,937 vertices (171 KB of vectors, 36 KB of halo): gathers 4.36 ms,
+// halo 5.89 ms; of 32,768 (156 and 33 KB): 3.53 and 3.22 ms.
 size_t cluster_halo_room(int vpcMax) {
+  constexpr size_t kRoom = 194 * 1024;  // and 1 KB the system's, and the static variables
   const size_t used = kSlotBytes + cluster_vertex_bytes(true) * vpcMax;
-  return used < kClusterSmemAll ? (kClusterSmemAll - used) / sizeof(float4) : 0;
+  return used < kRoom ? (kRoom - used) / sizeof(float4) : 0;
 }
 void launch_cluster_halo(const DeviceBatch& b, int* largest, cudaStream_t s) {
   k_cluster_halo<<<dim3((unsigned)b.nscenes, 16), 256, 0, s>>>(b, b.clusterGather, largest);
