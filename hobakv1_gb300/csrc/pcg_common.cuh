@@ -195,64 +195,61 @@ __device__ __forceinline__ double scene_sum(int n, Group group) {
 // The iteration waits for them, so the last CTA of a scene adds all groups only up
 // to kOneCta of them.  Past that they lie in segments of 32: the last CTA of a
 // segment forms its groups' sums, a lane each, and the last of the segments adds
-// those (one more ticket: 1.7 us where one CTA is soon done).  Microseconds of
-// k_spmv with one CTA a lane's groups one after the other / this: tiles of 128,
-// 52^3 (291 groups, one CTA) 23.3 / 18.7, 72^3 (760, segments) 65.2 / 54.9; tiles
-// of 64, 45^3 (191, one CTA) 18.6 / 17.5, 52^3 31.0 / 20.8, 72^3 82.6 / 59.2.
+// those (one more ticket: 1.7 us where one CTA is soon done).  Steps of 400
+// iterations, one CTA with a lane's groups one after the other / one CTA as here /
+// segments: tiles of 128 (three warps), 59,319 vertices (116 groups) 7.42 / 6.85 /
+// 7.44 ms; tiles of 64 (two warps), 59,319 vertices 9.1 / 8.8 / 7.7 ms, 17,576 (35)
+// 5.3 / 5.1 / 5.7 ms.  k_spmv of 72^3 (760 groups): 65 us with one CTA, 55 (tiles of
+// 64: 83 and 59) with segments.
 // tickets: one per tile, zero (a segment takes its first tile's).
 template <int NT, int TV>
 __device__ __forceinline__ bool scene_sums(const double* partial, double* groupSums, int stride, unsigned* tickets,
                                            unsigned* sceneTicket, const SceneParams& sp, int tile, int* flag,
                                            double* sh, double (&out)[3]) {
-  constexpr int kG = kGroupVerts / TV, kWarps = NT / 32, kPer = (3 + kWarps - 1) / kWarps;
-  constexpr int kOneCta = TV == 128 ? 512 : 192;
+  constexpr int kG = kGroupVerts / TV, kWarps = NT / 32;
+  constexpr int kOneCta = TV == 128 ? 512 : 64;
   const int tile0 = sp.tile0, n = sp.ntiles, ng = (n + kG - 1) / kG;
   const bool one = ng <= kOneCta;
   const int g0 = one ? 0 : (tile - tile0) / (32 * kG) * 32, g1 = one ? ng : min(ng, g0 + 32);
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  // a warp's component, and with two warps the first one's second: both in flight
+  const int c = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const bool mine = c < 3, two = kWarps < 3 && c + kWarps < 3;
   if (!last_tile(one ? sceneTicket : &tickets[tile0 + g0 * kG], min(n, g1 * kG) - g0 * kG, flag)) return false;
-  double t[kPer];
-#pragma unroll
-  for (int k = 0; k < kPer; k++) {
-    const int c = warp + k * kWarps;
-    const double* q = partial + (size_t)c * stride + tile0;
-    auto group = [&](int g) {
-      return group_sum<TV>([&](int i) { return g * kG + i < n ? __ldcg(&q[g * kG + i]) : 0.0; });
-    };
-    t[k] = 0.0;
-    if (c < 3 && one) {
+  auto group = [&](int comp, int g) {
+    const double* q = partial + (size_t)comp * stride + tile0;
+    return group_sum<TV>([&](int i) { return g * kG + i < n ? __ldcg(&q[g * kG + i]) : 0.0; });
+  };
+  double a = 0.0, b = 0.0;
+  if (one) {
+    if (mine)
 #pragma unroll 4
-      for (int g = lane; g < ng; g += 32) t[k] += group(g);
-    } else if (c < 3) {
-      t[k] = group(g0 + lane);
-    }
-  }
-  if (!one) {
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-      const int c = warp + k * kWarps;
-      if (c < 3) groupSums[(size_t)c * stride + tile0 + g0 + lane] = t[k];
-    }
+      for (int g = lane; g < ng; g += 32) {
+        a += group(c, g);
+        if (two) b += group(c + kWarps, g);
+      }
+  } else {
+    double* sums = groupSums + (size_t)c * stride + tile0;
+    if (mine) a = group(c, g0 + lane);
+    if (two) b = group(c + kWarps, g0 + lane);
+    if (mine) sums[g0 + lane] = a;
+    if (two) sums[(size_t)kWarps * stride + g0 + lane] = b;
     __syncthreads();  // last_tile's fence by thread 0 covers the writers
     if (!last_tile(sceneTicket, (ng + 31) / 32, flag)) return false;
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-      const int c = warp + k * kWarps;
-      t[k] = 0.0;
-      if (c < 3)
+    a = b = 0.0;
+    if (mine)
 #pragma unroll 8
-        for (int g = lane; g < ng; g += 32) t[k] += __ldcg(&groupSums[(size_t)c * stride + tile0 + g]);
-    }
+      for (int g = lane; g < ng; g += 32) {
+        a += __ldcg(&sums[g]);
+        if (two) b += __ldcg(&sums[(size_t)kWarps * stride + g]);
+      }
   }
-#pragma unroll
-  for (int k = 0; k < kPer; k++) {
-    const int c = warp + k * kWarps;
-    const double total = warp_tree(t[k]);
-    if (c < 3 && lane == 0) sh[c] = total;
-  }
+  a = warp_tree(a);
+  if (kWarps < 3) b = warp_tree(b);
+  if (mine && lane == 0) sh[c] = a;
+  if (two && lane == 0) sh[c + kWarps] = b;
   __syncthreads();
 #pragma unroll
-  for (int c = 0; c < 3; c++) out[c] = sh[c];
+  for (int k = 0; k < 3; k++) out[k] = sh[k];
   return true;
 }
 

@@ -1,4 +1,4 @@
-"""The loop of two kernels on scenes too large for one launch, in FP32: past 192
+"""The loop of two kernels on scenes too large for one launch, in FP32: past 64
 groups of 512 vertices (tiles of 64) or 512 (tiles of 128) a scene's sums are
 formed by several CTAs, below that by one."""
 import numpy as np
@@ -9,8 +9,8 @@ from hobakv1_gb300 import hobak, scenes
 pytestmark = pytest.mark.gpu
 
 
-# 97,336 vertices: 191 groups; 117,649: 230; 274,625: 537 (the last of their
-# segments with 6 and 25 groups)
+# 97,336 vertices: 191 groups; 117,649: 230; 274,625: 537 (the last
+# segments with 31, 6 and 25 groups; one CTA for 48^3 with tiles of 128)
 @pytest.mark.parametrize("N,tile", [(45, 64), (48, 64), (48, 128), (64, 128)])
 def test_large_scenes_match_fp64(N, tile):
     s = scenes.config2_scene(N, "arap")
