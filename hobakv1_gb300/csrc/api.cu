@@ -1041,7 +1041,8 @@ int prepare_grid_plan(hobak_batch_t* B) {
     for (int s = 0; s < n; s++) nv[s] = B->sceneParams[s].pcgCluster ? 0 : B->sceneParams[s].nv;
     g = plan_rows_pcg(nv.data(), n, B->longestRow, sms);
   }
-  if (!g.ctas) g = plan_grid_pcg(tiles.data(), n, B->d.tileV, mixed, sms);
+  const bool uneven = B->longestRow > 20 && 4ll * kSlice * B->d.nslotRows > 5ll * B->nblocks;
+  if (!g.ctas) g = plan_grid_pcg(tiles.data(), n, B->d.tileV, mixed, uneven, sms);
   if (g.ctas) {
     std::vector<int2> list;
     for (int s = 0; s < n; s++)

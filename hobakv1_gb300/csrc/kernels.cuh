@@ -295,7 +295,7 @@ void launch_element_eval(int nt, const int4* tets, const double* rest, const dou
 template <typename T>
 int launch_cluster_pcg(const DeviceBatch& b, const PcgVecs<T>& v, const ClusterClass* classes, int k,
                        cudaStream_t s);
-GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, bool mixed, int sms);
+GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, bool mixed, bool uneven, int sms);
 void plan_grid_smem(GridPlan& g, int tileV, int longestRow, bool mixed);
 // FP32: the halo lists of a plan's CTAs (largest: a device word)
 void launch_grid_halo(const DeviceBatch& b, const GridPlan& g, int* largest, cudaStream_t s);

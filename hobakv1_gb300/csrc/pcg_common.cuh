@@ -196,11 +196,10 @@ __device__ __forceinline__ double scene_sum(int n, Group group) {
 // to kOneCta of them.  Past that they lie in segments of 32: the last CTA of a
 // segment forms its groups' sums, a lane each, and the last of the segments adds
 // those (one more ticket: 1.7 us where one CTA is soon done).  Steps of 400
-// iterations, one CTA with a lane's groups one after the other / one CTA as here /
-// segments: tiles of 128 (three warps), 59,319 vertices (116 groups) 7.42 / 6.85 /
-// 7.44 ms; tiles of 64 (two warps), 59,319 vertices 9.1 / 8.8 / 7.7 ms, 17,576 (35)
-// 5.3 / 5.1 / 5.7 ms.  k_spmv of 72^3 (760 groups): 65 us with one CTA, 55 (tiles of
-// 64: 83 and 59) with segments.
+// iterations, one CTA / segments: tiles of 128 (three warps), 59,319 vertices (116
+// groups) 6.85 / 7.44 ms; tiles of 64 (two warps) 9.1 / 7.7 ms, 17,576 (35 groups)
+// 5.1 / 5.7 ms.  With one CTA and a lane's groups one after the other k_spmv of 52^3
+// took 23.3 us (18.7 as here), of 72^3 (760 groups) 65 (55; tiles of 64 83 and 59).
 // tickets: one per tile, zero (a segment takes its first tile's).
 template <int NT, int TV>
 __device__ __forceinline__ bool scene_sums(const double* partial, double* groupSums, int stride, unsigned* tickets,

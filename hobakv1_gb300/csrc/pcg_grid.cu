@@ -566,13 +566,24 @@ cudaError_t launch_tv(const DeviceBatch& b, const PcgVecs<T>& v, const GridPlan&
 
 // The line between the one launch and the loop: whether the tiles are resident
 // at once, one CTA of at most 512 threads (128 registers each) per SM; below it
-// the launch was the faster at every size measured (343 to 68,921 vertices,
+// the launch was the faster at every size of cube measured (343 to 68,921 vertices,
 // 1.3 to 2.1 times an iteration).
+// Not so in FP64 where rows are uneven: a warp's 32 rows take the longest one's
+// time on the FP64 pipe, in the loop (a thread per scalar row) only 11 do, and the
+// loop spreads any scene over all SMs.  Random Delaunay meshes, rows of 16 blocks
+// and the longest of 32 on average 25, 5,500 to 77,000 vertices: the launch is the
+// faster with 192 to 384 vertices a CTA on at least 70% of the SMs, 128 on 80% (us an
+// iteration of launch / loop: 18,000 vertices 30.6 / 32.5, 32,000 38.6 / 45.7, 50,000
+// 49.4 / 60.8) and the slower outside (5,500 26.6 / 20.6; 7,500 with 64 vertices a
+// CTA 25.5 / 20.2; 15,000 with 128 on 78%, tiles of 64, 29.6 / 27.1; 20,000 on 52%
+// 37.1 / 33.4; 70,000 with 512 69.5 / 59.8).  uneven: rows
+// past those of a cube (15) and a quarter of the slices' places empty (cubes 2-6%,
+// these meshes 55%).
 // Tiles per CTA so that the tiles of the given scenes (their tile counts) take
 // at most one CTA per SM, the fewest that does (an SM's FP64 pipe and L2 port
 // are what an iteration runs at); none: they do not fit, and solver.cu's loop
 // runs them.
-GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, bool mixed, int sms) {
+GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, bool mixed, bool uneven, int sms) {
   GridPlan g{};
   int most = 0;
   for (int s = 0; s < n; s++) most = std::max(most, tiles[s]);
@@ -581,12 +592,14 @@ GridPlan plan_grid_pcg(const int* tiles, int n, int tileV, bool mixed, int sms) 
     long long ctas = 0;
     for (int s = 0; s < n; s++) ctas += (tiles[s] + tpc - 1) / tpc;
     if (ctas > std::min(sms, kMaxCtas)) continue;
+    const int verts = tpc * tileV;
+    if (!mixed && uneven && (verts < 128 || verts > 384 || 10 * ctas < (verts == 128 ? 8 : 7) * sms))
+      return g;
     g.ctas = (int)ctas;
     g.tpc = tpc;
     // the partials of a scene (in FP64 beside its tree's lanes); in FP64 the row
     // products, nine a thread
-    const int threads = tpc * tileV;
-    g.scratch = mixed ? 3 * std::max(most, threads) : std::max(9 * threads, 3 * most + 9 * tileV);
+    g.scratch = mixed ? 3 * std::max(most, verts) : std::max(9 * verts, 3 * most + 9 * tileV);
     g.scratch += g.scratch % 2;
     return g;
   }

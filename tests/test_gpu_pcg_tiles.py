@@ -70,9 +70,10 @@ def test_tiles_of_64(N, precision):
     alone_and_in_the_loop(s, hobak.solver_opts(precision=precision, max_iters=40), tile_vertices=64)
 
 
-# rows of 51 blocks (thread per row in FP64), 99 (too long for its shared memory: a
-# thread per vertex) and 51 again past its vertices
-@pytest.mark.parametrize("layers,sides", [(40, 24), (40, 48), (240, 24)])
+# rows of 51 blocks: a thread per row in FP64, and a thread per vertex where 80% of
+# the SMs have a CTA of 128 of them (16,000 vertices); of 99, too long for the first
+# one's shared memory
+@pytest.mark.parametrize("layers,sides", [(40, 24), (640, 24), (330, 48)])
 @pytest.mark.parametrize("precision", [hobak.PRECISION_FP64, hobak.PRECISION_MIXED], ids=["fp64", "mixed"])
 @pytest.mark.parametrize("tile", [64, 128])
 def test_long_rows(layers, sides, precision, tile):
@@ -117,3 +118,28 @@ def test_clusters_beside_the_one_launch(sizes, clusters, precision):
             assert all(np.array_equal(g, w) for g, w in zip(b.get_state(k), alone.get_state(0)))
             alone.close()
     b.close()
+
+
+def launches(s, precision, tile, steps=1):
+    b = hobak.BATCH([s], hobak.solver_opts(precision=precision))
+    b.set_tuning(tile_vertices=tile)
+    before = b.launch_count()
+    st = b.step(steps)[0]
+    n = b.launch_count() - before
+    b.close()
+    return n, st[0]
+
+
+@pytest.mark.parametrize("layers,sides,tile,one", [
+    (200, 48, 64, False),   # 9,800 vertices: CTAs of 64
+    (200, 48, 128, False),  # on half of the SMs
+    (330, 48, 128, True),   # 16,170 on 127 of them
+    (330, 48, 64, True),    # CTAs of 128 all the same
+    (1400, 48, 128, False),  # 68,600: CTAs of 512
+])
+def test_uneven_rows_choose_the_faster_path_in_fp64(layers, sides, tile, one):
+    """Meshes whose rows differ much in length take the one launch in FP64 only
+    where it is the faster of the two."""
+    s = tower(layers, sides)
+    n, iterations = launches(s, hobak.PRECISION_FP64, tile)
+    assert (n < 30) == one and (n >= 2 * iterations) == (not one) and iterations > 40
