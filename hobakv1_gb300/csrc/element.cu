@@ -276,10 +276,12 @@ template <typename HT, int KC>
 // FP32 is bound by latency (the FP64 pipe is 59% busy with F, the stress and
 // the force, 16 warps an SM): six CTAs per SM at 80 registers, though they
 // spill ~500 bytes, take 177 us for 384,000 SNH tets where four at 128 took
-// 204 and five at 96 took 184; 96 scenes 1,224 -> 1,203 us.  FP64 is bound by its
+// 204 and five at 96 took 184; 96 scenes 1,224 -> 1,203 us.  ARAP's, with the FP64
+// rotation beside the FP32 factors, stays at four and 128 (384,000 tets 251.3 us, 254
+// with six; 48,000 SNH and 55,566 ARAP tets 97.7, 100.4).  FP64 is bound by its
 // pipe (88% busy at 8 warps an SM): 168 registers and 12 warps gain nothing
 // over the 216 it takes when left alone.
-__global__ void __launch_bounds__(128, sizeof(HT) == 4 ? 6 : 1)
+__global__ void __launch_bounds__(128, sizeof(HT) != 4 ? 1 : KC == kElemArap ? 4 : 6)
     k_element(DeviceBatch b, int rawForces, HT* __restrict__ outH) {
   // The CTA's tets read their corners from shared memory: the distinct
   // vertices of its one or two staging blocks (host-built, ascending ids)
