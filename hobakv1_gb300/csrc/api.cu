@@ -1502,7 +1502,7 @@ int build_collisions(hobak_batch_t* B) {
   const size_t oTriArea = A.reserve(sizeof(double) * ntri), oTriNbr = A.reserve(sizeof(int) * 3 * (size_t)ntri);
   const size_t oSv = A.reserve(sizeof(int) * nsv), oSvScene = A.reserve(sizeof(int) * nsv);
   const size_t oSvArea = A.reserve(sizeof(double) * nsv);
-  const size_t oCell = A.reserve(sizeof(unsigned) * n), oInv = A.reserve(nv), oSkip = A.reserve(ntri);
+  const size_t oCell = A.reserve(sizeof(unsigned) * n), oInv = A.reserve(nv);
   const size_t oBucket = A.reserve(sizeof(int) * (hash + 1)), oCursor = A.reserve(sizeof(int) * hash);
   const size_t oEntry = A.reserve(sizeof(int) * 8 * (size_t)ntri);
   const size_t oTriBox = A.reserve(2 * sizeof(float4) * (size_t)ntri);
@@ -1550,7 +1550,6 @@ int build_collisions(hobak_batch_t* B) {
   c.svArea = carve<double>(base, oSvArea);
   c.cellBits = carve<unsigned>(base, oCell);
   c.vInverted = carve<unsigned char>(base, oInv);
-  c.triSkip = carve<unsigned char>(base, oSkip);
   c.bucketCount = carve<int>(base, oBucket);
   c.bucketCursor = carve<int>(base, oCursor);
   c.entryTri = carve<int>(base, oEntry);

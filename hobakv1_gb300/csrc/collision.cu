@@ -172,7 +172,6 @@ __global__ void k_tri_prepare(DeviceBatch b, DeviceCollisions c) {
   const double area = 0.5 * norm(cross(bb - a, cc - a));
   const bool degenerate = area / c.triArea[f] < 1e-4;
   const bool allInv = c.vInverted[v0] && c.vInverted[v1] && c.vInverted[v2];
-  c.triSkip[f] = (degenerate || allInv) ? 1 : 0;
   const double ext = fmax(fmax(fmax(fmax(a.x, bb.x), cc.x) - fmin(fmin(a.x, bb.x), cc.x),
                                fmax(fmax(a.y, bb.y), cc.y) - fmin(fmin(a.y, bb.y), cc.y)),
                           fmax(fmax(a.z, bb.z), cc.z) - fmin(fmin(a.z, bb.z), cc.z)) +

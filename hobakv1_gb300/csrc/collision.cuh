@@ -42,7 +42,6 @@ struct DeviceCollisions {
   // per step
   unsigned* cellBits;      // [nscenes] largest triangle extent (float bits) -> cell size
   unsigned char* vInverted;  // [nv]
-  unsigned char* triSkip;    // [ntri] degenerate or all-inverted
   // FP32 boxes for the queries, rounded outward: lo.xyz and the scene id, hi.xyz
   // and the skip flag (triangles) or the cell of the box's lower corner (edges,
   // eeCell); a triangle's box inflated by eps and a margin, an edge's by eps
