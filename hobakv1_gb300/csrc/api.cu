@@ -367,7 +367,8 @@ int alloc_precision(hobak_batch_t* B) {
   const size_t oMinv = A.reserve(w * kSlotVals * ((nv + kSlice - 1) / kSlice));
   size_t oVec[6];
   for (int k = 0; k < (mixed ? 6 : 4); k++) oVec[k] = A.reserve(w * 3 * nv);
-  const size_t oHalo = mixed ? A.reserve(sizeof(int) * 4 * nv) : 0;  // clusters and the one-launch PCG
+  // clusters and the one-launch PCG (halo_list)
+  const size_t oHalo = mixed ? A.reserve(sizeof(int) * (4 * nv + kHaloSpare * B->scenes.size())) : 0;
   void* base = nullptr;
   cudaError_t e = batch_malloc(&base, A.used);
   if (e != cudaSuccess)

@@ -406,7 +406,7 @@ __global__ void k_cluster_gather(DeviceBatch b, int* __restrict__ gather) {
 // A cluster CTA's halo and its slots' columns as indices into the CTA's u (own
 // vertices, then the halo in ascending order): a bit per vertex of the scene,
 // then ranks.  CTA (scene, rank).  largest[class]: the largest halo of the
-// class, INT_MAX where one exceeds its list (four times the CTA's vertices).
+// class, INT_MAX where one exceeds its list (halo_list).
 constexpr int kHaloWords = 2048;  // 65,536 vertices: more than 16 CTAs hold
 __global__ void __launch_bounds__(256) k_cluster_halo(DeviceBatch b, int* __restrict__ gather, int* largest) {
   __shared__ unsigned bits[kHaloWords];
@@ -448,8 +448,8 @@ __global__ void __launch_bounds__(256) k_cluster_halo(DeviceBatch b, int* __rest
   __syncthreads();
   int at = x - mine;
   for (int i = 0; i < tid / 32; i++) at += warpTot[i];
-  const int cap = 4 * (z - a);
-  int* list = b.gridHalo + 4 * (size_t)a;
+  const int cap = 4 * vpc;
+  int* list = halo_list(b, sc, a);
   for (int i = i0; i < i1; i++) {
     rank[i] = at;
     for (unsigned m = bits[i]; m; m &= m - 1, at++) {
@@ -499,7 +499,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kClusterThreads, 1)
   // contact on this scene: its rows add w H_coll u (collision_lhs_scale)
   const bool contact = b.collOn && (b.coll.scenes[sc].vfOn || b.coll.scenes[sc].eeOn);
   constexpr int kUShift = sizeof(T) == 4 ? 4 : 5;  // bytes of one u entry: 16 (float4) or 32
-  const int* halo = HALO ? b.gridHalo + 4 * (size_t)(v0 + my0) : nullptr;
+  const int* halo = HALO ? halo_list(b, sc, v0 + my0) : nullptr;
   const int nHalo = HALO ? b.clusterHaloCount[16 * sc + rank] : 0;
   if (threadIdx.x < CL) m.ubase[threadIdx.x] = map_cluster(m.u, threadIdx.x);
 

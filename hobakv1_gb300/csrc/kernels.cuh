@@ -180,10 +180,10 @@ struct DeviceBatch {
   ulonglong2* gridRowWords;  // [2][CTAs][9] partials of pcg_rows.cu
   int waitPolls;  // polls after which a wait of these launches gives up
   // FP32 (pcg_grid.cu and clusters): per CTA the vertices of other CTAs that its
-  // rows' columns name (at 4 x its first vertex), their number (per tile: a
+  // rows' columns name, their number (per tile: a
   // CTA's is its first tile's), and every column as the CTA's own index of it
   // (k_grid_halo, k_cluster_halo; the slots of clusterGather)
-  int* gridHalo;
+  int* gridHalo;  // halo_list
   int* gridHaloCount;
   int* clusterHaloCount;  // cluster scenes' halos (lists in gridHalo): [scene][16]
   double* psi;          // [T] energy density scratch
@@ -207,6 +207,14 @@ __device__ __forceinline__ size_t col_slot(const DeviceBatch& b, int u, int j) {
 // Offset of entry 0 of vertex u's preconditioner block (entry e at + kSlice * e).
 __device__ __forceinline__ size_t minv_slot(int u) {
   return (size_t)(u >> 5) * kSlotVals + (u & (kSlice - 1));
+}
+
+// Halo list of the CTA of `scene` whose first vertex is `first`: room for four times
+// the vertices of a full CTA, for a scene's last and shorter one too, whose one
+// vertex may have a dozen neighbours: kHaloSpare more a scene.
+constexpr int kHaloSpare = 4 * 512;
+__device__ __forceinline__ int* halo_list(const DeviceBatch& b, int scene, int first) {
+  return b.gridHalo + 4 * (size_t)first + (size_t)kHaloSpare * scene;
 }
 
 // Weight of the collision Hessian H_coll in the step's matrix A, with

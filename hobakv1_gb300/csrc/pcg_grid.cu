@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   const int lenMax = __reduce_max_sync(0xffffffffu, len);
   __syncthreads();
   int* flags = b.gridFlags + sp.tile0;  // a CTA's flag: that of its first tile
-  const int* haloList = b.gridHalo + 4 * (size_t)b.tileV0[sp.tile0 + cta.y];
+  const int* haloList = halo_list(b, s, b.tileV0[sp.tile0 + cta.y]);
   const int nHalo = kF32 ? b.gridHaloCount[sp.tile0 + cta.y] : 0;
   if constexpr (kF32) us[tid] = make_float4(un[0], un[1], un[2], 0.f);
   const bool whole = kF32 && tpc == kG;  // partials: one per group, else one per tile
@@ -625,7 +625,7 @@ void plan_grid_smem(GridPlan& g, int tileV, int longestRow, bool mixed) {
 // A CTA's halo: the vertices of other CTAs in its rows' columns, ascending (a
 // bit per vertex of the scene, then ranks), and every column's index in the
 // shared u: the thread of an own vertex, or past the threads the halo's rank.
-// A list longer than its room (four times the CTA's vertices, kHaloMax) leaves
+// A list longer than its room (four times the threads, kHaloMax) leaves
 // the batch to solver.cu's loop.
 constexpr int kHaloWords = 152 * kGridThreads / 32 + 8 * kMaxCtas;
 __global__ void __launch_bounds__(kGridThreads) k_grid_halo(DeviceBatch b, const int2* __restrict__ ctas, int tpc,
@@ -663,8 +663,8 @@ __global__ void __launch_bounds__(kGridThreads) k_grid_halo(DeviceBatch b, const
   __syncthreads();
   int at = x - mine;
   for (int i = 0; i < tid / 32; i++) at += warpTot[i];
-  const int cap = min(kHaloMax, 4 * (z - a));
-  int* list = b.gridHalo + 4 * (size_t)a;
+  const int cap = min(kHaloMax, 4 * NT);
+  int* list = halo_list(b, cta.x, a);
   for (int i = i0; i < i1; i++) {
     rank[i] = at;
     for (unsigned m = bits[i]; m; m &= m - 1, at++)

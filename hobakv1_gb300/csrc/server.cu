@@ -98,7 +98,7 @@ long long footprint_bytes(const hobak_scene_desc& s, int precision) {
   const long long perVertex = 5 * 24 + 8 + 1 + 4 + 4 + 4 + 3 * 24 + 9 * w + (w == 4 ? 6 : 4) * 3 * w;
   // partial words, flags and halo counts per tile of 64 vertices; the halo's lists
   const long long perVertexPcg = 2 + (w == 4 ? 16 : 0);
-  constexpr long long kBatchPcg = 80 << 10;  // words of the thread-per-row PCG, CTA table
+  constexpr long long kBatchPcg = 88 << 10;  // words of the thread-per-row PCG, CTA table, spare of a halo list
   return nt * perTet + nb * perBlock + nv * (perVertex + perVertexPcg) + (1LL << 20) + kBatchPcg;
 }
 

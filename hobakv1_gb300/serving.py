@@ -73,7 +73,7 @@ def footprint_bytes(scene, precision: int) -> int:
     per_vertex = 5 * 24 + 8 + 1 + 4 + 4 + 4 + 3 * 24 + 9 * w + (6 if w == 4 else 4) * 3 * w
     # partial words, flags and halo counts per tile of 64 vertices; the halo's lists
     per_vertex_pcg = 2 + (16 if w == 4 else 0)
-    batch_pcg = 80 << 10  # words of the thread-per-row PCG, CTA table
+    batch_pcg = 88 << 10  # words of the thread-per-row PCG, CTA table, spare of a halo list
     return int(nt * per_tet + nb * per_block + nv * (per_vertex + per_vertex_pcg) + (1 << 20) + batch_pcg)
 
 

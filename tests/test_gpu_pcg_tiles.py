@@ -143,3 +143,29 @@ def test_uneven_rows_choose_the_faster_path_in_fp64(layers, sides, tile, one):
     s = tower(layers, sides)
     n, iterations = launches(s, hobak.PRECISION_FP64, tile)
     assert (n < 30) == one and (n >= 2 * iterations) == (not one) and iterations > 40
+
+
+@pytest.mark.parametrize("layers,sides", [(77, 4), (43, 8), (49, 12)])  # 385, 387 and 637 vertices
+@pytest.mark.parametrize("tile", [64, 128])
+def test_last_cta_of_few_vertices(layers, sides, tile):
+    """In FP32 a CTA lists its halo.  The last CTA of a scene may hold one vertex (385
+    = 3 x 128 + 1 = 6 x 64 + 1), which has more than four neighbours in other CTAs."""
+    s = tower(layers, sides)
+    alone_and_in_the_loop(s, hobak.solver_opts(precision=hobak.PRECISION_MIXED), tile_vertices=tile)
+
+
+def test_cluster_with_a_cta_of_one_vertex():
+    """121 vertices in a cluster of 16: eight a CTA and one in the last.  Beside a
+    scene whose halo has no room the class gathers from the other CTAs: same bits."""
+    s = tower(11, 10)
+    out = []
+    for group in ([s], [s, scenes.config2_scene(34, "arap")]):
+        b = hobak.BATCH(group, hobak.solver_opts(precision=hobak.PRECISION_MIXED))
+        b.set_tuning(cluster_pcg=1)
+        b.set_scene_cluster(0, 16)
+        assert (b.pcg_path() == 16).all()
+        st = b.step(2)[0]
+        out.append((st, *b.get_state(0)))
+        b.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
